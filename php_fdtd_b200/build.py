@@ -65,7 +65,7 @@ def build_host(verbose: bool = False) -> Path:
 def build_device(verbose: bool = False) -> Path:
     out = PKG / "libphpfdtd.so"
     sources = [CSRC / "php_fdtd.cu", CSRC / "php_noalloc.cu", CSRC / "php_serve.cu"]
-    deps = sources + [INC / "php_fdtd.h", INC / "php_serve.h"] + [p for p in CSRC.glob("*.cuh")]
+    deps = sources + [INC / "php_fdtd.h", INC / "php_serve.h", CSRC / "php_internal.h"] + [p for p in CSRC.glob("*.cuh")]
     if _stale(out, deps):
         _run([_nvcc(), *NVCC_ARCH, "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC,-ffp-contract=off",
               "-shared", f"-I{INC}", *sources, "-o", out], verbose)

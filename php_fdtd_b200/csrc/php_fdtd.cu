@@ -11,6 +11,7 @@
  * contraction off), so the device sees the same doubles fdtd.c computes.
  */
 #include "php_fdtd.h"
+#include "php_internal.h"
 #include "php_kernels.cuh"
 
 #include <cuda_runtime.h>
@@ -36,6 +37,11 @@ using namespace phpdev;
 namespace {
 
 constexpr int kMaxChunk = 256;      /* steps per recorded graph */
+/* steps per graph where a step has branches: recording and instantiating one
+ * takes some 60 us per step then, 10 us without; every php_step call of more
+ * steps replays it (its input rows come through page-locked slots of this
+ * many steps, so that the same 512 steps are enqueued ahead) */
+constexpr int kBranchChunk = 16;
 constexpr int kProfKinds = PHP_PROFILE_KINDS; /* H sweep, E sweep, probe, DFT, ion pass, one-launch step */
 constexpr int kProbeCap = 8192;     /* probe rows held on the device */
 constexpr double kEpsInf = 20.0;    /* EPS_INF, fdtd.c:202 */
@@ -50,6 +56,17 @@ constexpr double kEpsInf = 20.0;    /* EPS_INF, fdtd.c:202 */
 constexpr double kIonScale32 = 281474976710656.0; /* 2^48 */
 
 thread_local std::string g_create_error; /* errors of php_create, per calling thread */
+
+/* Streams and events that fork a step's launches into branches while its
+ * graph is recorded (only then: the recorded graph holds the branches).  Taken
+ * from a pool, since creating streams takes milliseconds; the pool keeps at
+ * most kSidePool of them, one per thread recording at a time. */
+struct SideStreams {
+    int device = 0;
+    cudaStream_t s[2] = {};
+    cudaEvent_t fork = nullptr, join[2] = {};
+};
+constexpr size_t kSidePool = 8;
 
 struct DftPlane {
     int comp, z, first, interval, nfreq, cast_f32;
@@ -87,6 +104,9 @@ struct php_ctx {
      * device busy does not queue behind their sweeps; `stream` (default
      * priority) takes over at the end of php_create */
     cudaStream_t setup = nullptr;
+    /* split: the H sweep of the rest runs beside the interior launch, and the
+     * E sweep's launches of the three kinds of blocks beside each other */
+    SideStreams* side = nullptr; /* while a graph is recorded */
     /* page-locked staging of host -> device uploads (upload()) */
     void* up_buf[2] = {};
     cudaEvent_t up_ev[2] = {};
@@ -107,10 +127,21 @@ struct php_ctx {
      * launch writes the new level to; swap_levels exchanges them with f and
      * psi after it.  level: how many swaps since php_create, mod 2 */
     bool fused = false;
+    /* the interior of the domain in one launch (interior_sweep_tma), the rest
+     * in the two sweeps: E and H double buffered like the one-launch step's,
+     * the H CPML state in place (the interior has none).  Block lists
+     * (StepArgs::list): interior, H sweep, E sweep */
+    bool split = false;
+    /* the E sweep's blocks in a launch per kind (lists[2..4]), in place */
+    bool by_class = false;
+    bool allow_split = true;     /* php_create_buffers */
+    int4* lists[5] = {};         /* interior, H sweep, E sweep: plain, atom, general blocks */
+    int nlist[5] = {};
     void* fo[9] = {};
     void* psio[6] = {};
     int level = 0;
-    uint8_t* plain_hf = nullptr;  /* StepArgs::plain_hf */
+    uint16_t* pcls = nullptr;    /* StepArgs::pcls */
+    int zstep = 0;               /* planes per block of he_sweep_tma */
     uint8_t* mat = nullptr;
     uint8_t* plain_blk = nullptr; /* plain blocks of the fused sweep (StepArgs::plain_blk) */
     double kdp[3] = {};
@@ -121,18 +152,24 @@ struct php_ctx {
     uint8_t* slot_mat = nullptr;
     int32_t* slot_n3 = nullptr;
     void *P = nullptr, *Po = nullptr, *r = nullptr, *v = nullptr;
+    void* Dp = nullptr;          /* D of the cells with a slot (fast modes; the strict mode keeps D in f[3..5]) */
+    uint32_t* Dc = nullptr;      /* StepArgs::Dc */
+    double* dmat = nullptr;      /* M^-1 per material, for D of the cells that keep E alone */
     void* mc = nullptr;          /* MatCoef<R>[nmat] */
     void* ion_coef = nullptr;
     void* axis_tab[3][7] = {};   /* kappa b c kh kd ch cd per axis */
-    int32_t* axis_slot[3] = {};
     /* per-step inputs (source values, DFT flags and phasors), double
      * buffered so that the host fills one while the GPU runs the other */
     double* step_in = nullptr;   /* buffer the graph being recorded reads */
     double* step_in_dev[2] = {};  /* [kMaxChunk][row] each */
     double* step_in_host[2] = {}; /* pinned */
-    cudaEvent_t staged[2] = {};   /* copy out of step_in_host[b] finished */
+    int max_chunk = kMaxChunk;    /* steps per graph: kMaxChunk or kBranchChunk */
+    /* copy out of a page-locked slot (max_chunk rows; 2 kMaxChunk rows in all) finished */
+    cudaEvent_t staged[2 * kMaxChunk / kBranchChunk] = {};
     int chunk_no = 0;
     int step_row = 0;
+    int probe_off = 0;           /* offset of the monitor row's index in a step-input row */
+    double* src_acc = nullptr;   /* StepArgs::src_acc */
     void* scratch = nullptr;     /* plane gathers, diagnostics */
     size_t scratch_bytes = 0;
     void* host_stage = nullptr;  /* pinned */
@@ -158,6 +195,7 @@ struct php_ctx {
     /* probe */
     bool probe = false;
     int64_t probe_cf = 0, probe_slot = -1;
+    DCell probe_d{};             /* where D of the field cell is */
     int probe_ka = 0;            /* plane of the atom cell */
     int probe_n3 = 0;
     double* probe_rows = nullptr;
@@ -196,15 +234,18 @@ struct php_ctx {
     int ion_k_off = -1;
     std::vector<double> ion_k;
     std::vector<double> iso_scale;   /* StepArgs::iso, per material */
-    /* per material: eps_inv, eps_im, cs, sn of the packed record; the
-     * chosen one rides in StepArgs::tns_* */
-    std::vector<std::array<double, 20>> mat_tns;
+    /* per material: em and eps_im of the packed record; the chosen one rides
+     * in StepArgs::tns_* */
+    std::vector<std::array<double, 18>> mat_tns;
     int tns_id = -1;
-    /* the few-atom material of ion_k and its packed record (MatCoef<R>
-     * bytes), for StepArgs::amc; atom_blocks: kPlainAtoms blocks exist */
+    /* the few-atom material of ion_k (with the ion pass apart: the atom
+     * material with the most cells) and its packed record (MatCoef<R> bytes),
+     * for StepArgs::amc; atom_blocks: kPlainAtoms blocks exist */
     int atom_id = -1;
     std::vector<unsigned char> atom_mc;
     bool atom_blocks = false;
+    int ade_id = -1;             /* StepArgs::dmc */
+    std::vector<unsigned char> ade_mc;
 
     /* output frames (php_frame_begin): page-locked slots taken in ticket
      * order; state 0 free, 1 taken (begun and not released) */
@@ -330,7 +371,52 @@ struct MatD {
     double eps_inv[9] = {}, eps_im[9] = {};
     double lf = 1.0, lt = 0.0, cs = 1.0, sn = 0.0;
     double gp_inv[9] = {}, gm[9] = {}, wp2[9] = {};
+    /* fast modes, materials without ADE and atoms: E = em D in the lab frame
+     * and D = dm E; e_only: both well conditioned, the cells keep E alone */
+    double em[9] = {}, dm[9] = {};
+    bool e_only = false;
+    /* whether a cell of the material has a pool slot */
+    bool slotted(bool strict) const { return (flags & (kAde | kAtoms)) || (!strict && !e_only); }
 };
+
+/* em = R^T eps^-1 R lf (1 - lt) / eps0, the map from D to E that the fast
+ * modes apply (fdtd.c:3429-3503), and its inverse.  Where eps^-1 is close to
+ * singular (its real part can be, for complex eps) the increment form would
+ * lose digits, and D has no read-out from E: those materials keep D. */
+static void derive_e_only(const php_desc& d, MatD& o)
+{
+    double rot[3][3] = {{1, 0, 0}, {0, 1, 0}, {0, 0, 1}}, m[3][3], inv[3][3];
+    if (o.flags & kRotZ) {
+        rot[0][0] = rot[1][1] = o.cs;
+        rot[0][1] = -o.sn;
+        rot[1][0] = o.sn;
+    } else if (o.flags & kRotX) {
+        rot[1][1] = rot[2][2] = o.cs;
+        rot[1][2] = -o.sn;
+        rot[2][1] = o.sn;
+    }
+    double big = 0.0, big_inv = 0.0;
+    for (int a = 0; a < 3; a++)
+        for (int b = 0; b < 3; b++) {
+            double v = 0.0;
+            for (int p = 0; p < 3; p++)
+                for (int q = 0; q < 3; q++) v += rot[p][a] * (o.eps_inv[p * 3 + q] * (o.lf * (1.0 - o.lt))) * rot[q][b];
+            m[a][b] = v;
+            big = std::max(big, fabs(v));
+        }
+    if (!(big > 0.0) || !std::isfinite(big)) return;
+    double s[3][3]; /* scaled to order one, for inverse3's absolute bound on the determinant */
+    for (int a = 0; a < 3; a++)
+        for (int b = 0; b < 3; b++) s[a][b] = m[a][b] / big;
+    if (inverse3(s, inv)) return;
+    for (int a = 0; a < 9; a++) big_inv = std::max(big_inv, fabs(inv[a / 3][a % 3]));
+    if (!(big_inv < 256.0)) return;
+    for (int a = 0; a < 9; a++) {
+        o.em[a] = m[a / 3][a % 3] / d.epsilon0;
+        o.dm[a] = inv[a / 3][a % 3] / big * d.epsilon0;
+    }
+    o.e_only = true;
+}
 
 static int derive_material(php_ctx* ctx, int id, const php_material_desc& m, MatD& o)
 {
@@ -401,8 +487,11 @@ static int derive_material(php_ctx* ctx, int id, const php_material_desc& m, Mat
         o.flags |= kAtoms;
         o.natom = m.natom;
     }
+    if (!(o.flags & (kAde | kAtoms))) derive_e_only(d, o);
     return PHP_OK;
 }
+
+static bool is_iso(const MatD& s);
 
 template <typename R>
 static MatCoef<R> pack_material(const php_ctx* ctx, const MatD& s, int ion_off)
@@ -450,12 +539,11 @@ static MatCoef<R> pack_material(const php_ctx* ctx, const MatD& s, int ion_off)
     o.cs = (R)s.cs;
     o.sn = (R)s.sn;
     o.ade_scale = (R)((1.0 - s.lt) / (d.epsilon0 * kEpsInf));
-    if (!strict && !(s.flags & (kLossy | kAde | kRotZ | kRotX | kAtoms))) {
-        const double* e = s.eps_inv;
-        if (e[1] == 0.0 && e[2] == 0.0 && e[3] == 0.0 && e[5] == 0.0 && e[6] == 0.0 && e[7] == 0.0 && e[0] == e[4] &&
-            e[0] == e[8])
-            o.flags |= kIso;
+    if (!strict && s.e_only) {
+        o.flags |= kEOnly;
+        for (int q = 0; q < 9; q++) o.em[q] = (R)s.em[q];
     }
+    if (!strict && is_iso(s)) o.flags |= kIso;
     return o;
 }
 
@@ -556,15 +644,16 @@ static bool dft_folded(const php_ctx* ctx, size_t q)
     return before < kDftFold;
 }
 
-/* Whether the E sweep records the monitor row itself (StepArgs::probe_*):
- * the field cell is a plane of the grid (not a halo plane) in the z chunk
- * of the atom cell, whose r and v that sweep updates (no ion pass apart). */
+/* Whether the sweeps record the monitor row themselves (StepArgs::probe_*):
+ * the field cell is a plane of the grid (not a halo plane) and a sweep
+ * updates the atom cell's r and v (no ion pass apart).  Where the caller set
+ * the z chunks, only for field and atom cells of one chunk. */
 static bool probe_folded(const php_ctx* ctx)
 {
     if (!ctx->probe || !ctx->probe_fold || ctx->ion_split) return false;
     const int kf = (int)(ctx->probe_cf / ctx->plane);
     if (ctx->probe_cf < 0 || kf >= ctx->nz) return false;
-    return ctx->probe_n3 == 0 || kf / ctx->zchunk == ctx->probe_ka / ctx->zchunk;
+    return ctx->probe_n3 == 0 || ctx->d.z_chunk <= 0 || kf / ctx->zchunk == ctx->probe_ka / ctx->zchunk;
 }
 
 /* dft_sample launches per step */
@@ -576,18 +665,32 @@ static int dft_launched(const php_ctx* ctx)
 }
 
 template <typename R>
+static Fields<R> make_fields(const php_ctx* ctx)
+{
+    R* const* fp = reinterpret_cast<R* const*>(ctx->f);
+    return Fields<R>{fp[0], fp[1], fp[2], fp[3], fp[4], fp[5], fp[6], fp[7], fp[8]};
+}
+
+template <typename R>
+static DView<R> make_dview(const php_ctx* ctx)
+{
+    return DView<R>{(const R*)ctx->Dp, ctx->mat, ctx->slot, ctx->dmat, ctx->nslot, ctx->ncell_dev};
+}
+
+template <typename R>
 static StepArgs<R> make_args(php_ctx* ctx, int s_local)
 {
     StepArgs<R> a;
     memset(&a, 0, sizeof(a));
-    R* const* fp = reinterpret_cast<R* const*>(ctx->f);
-    a.f = Fields<R>{fp[0], fp[1], fp[2], fp[3], fp[4], fp[5], fp[6], fp[7], fp[8]};
+    a.f = make_fields<R>(ctx);
+    a.Dp = (R*)ctx->Dp;
+    a.Dc = ctx->Dc;
+    a.dv = make_dview<R>(ctx);
     R* const* pp = reinterpret_cast<R* const*>(ctx->psi);
     a.psi = Psi<R>{pp[0], pp[1], pp[2], pp[3], pp[4], pp[5], pp[6], pp[7], pp[8], pp[9], pp[10], pp[11]};
     AxisTab<R>* tabs[3] = {&a.tx, &a.ty, &a.tz};
     for (int ax = 0; ax < 3; ax++) {
         AxisTab<R>& t = *tabs[ax];
-        t.slot = ctx->axis_slot[ax];
         t.kappa = (const R*)ctx->axis_tab[ax][0];
         t.b = (const R*)ctx->axis_tab[ax][1];
         t.c = (const R*)ctx->axis_tab[ax][2];
@@ -613,31 +716,30 @@ static StepArgs<R> make_args(php_ctx* ctx, int s_local)
     a.plain_h = ctx->plain_h;
     for (int q = 0; q < 3; q++) a.khp[q] = (R)ctx->khp[q];
     a.tns_flags = 0;
-    a.tns_cs = a.tns_sn = R(0);
-    for (int q = 0; q < 9; q++) a.tns_inv[q] = a.tns_im[q] = R(0);
     if (ctx->tns_id >= 0) {
-        const std::array<double, 20>& t = ctx->mat_tns[ctx->tns_id];
+        const std::array<double, 18>& t = ctx->mat_tns[ctx->tns_id];
         a.tns_flags = ctx->mat_flags[ctx->tns_id];
         for (int q = 0; q < 9; q++) {
-            a.tns_inv[q] = (R)t[q];
+            a.tns_em[q] = (R)t[q];
             a.tns_im[q] = (R)t[9 + q];
         }
-        a.tns_cs = (R)t[18];
-        a.tns_sn = (R)t[19];
     }
     memset(&a.amc, 0, sizeof(a.amc));
     if (ctx->atom_blocks && ctx->atom_mc.size() == sizeof(MatCoef<R>)) memcpy(&a.amc, ctx->atom_mc.data(), sizeof(MatCoef<R>));
+    a.dmc_id = -1;
+    if (ctx->ade_id >= 0 && ctx->ade_mc.size() == sizeof(MatCoef<R>)) {
+        a.dmc_id = ctx->ade_id;
+        memcpy(&a.dmc, ctx->ade_mc.data(), sizeof(MatCoef<R>));
+    }
     a.nslot = ctx->nslot;
-#ifndef PHP_SMEM_MATS
-#define PHP_SMEM_MATS 0
-#endif
-    a.nmat = PHP_SMEM_MATS ? std::min(ctx->d.num_materials, kSmemMats) : 0;
     a.nx = ctx->nx;
     a.ny = ctx->ny;
     a.nz = ctx->nz;
     a.nxp = ctx->nxp;
     a.L = ctx->L;
     a.zchunk = ctx->zchunk;
+    a.z_off = ctx->z_off;
+    a.nzg = ctx->nz_glob;
     a.plane = ctx->plane;
     const php_desc& d = ctx->d;
     a.dt = d.dt;
@@ -654,6 +756,7 @@ static StepArgs<R> make_args(php_ctx* ctx, int s_local)
         a.src_comp[s] = ctx->src_comp[s];
     }
     a.src_val = ctx->step_in + (size_t)s_local * ctx->step_row;
+    a.src_acc = ctx->src_acc;
     a.err = ctx->err_flag;
     a.stall_test = ctx->stall_test;
     a.ndft = 0;
@@ -674,6 +777,8 @@ static StepArgs<R> make_args(php_ctx* ctx, int s_local)
         a.probe_rows = ctx->probe_rows;
         a.probe_count = ctx->probe_count;
         a.probe_kf = (int32_t)(cf / ctx->plane);
+        a.probe_ka = ctx->probe_ka;
+        a.probe_off = ctx->probe_off;
         a.probe_j = (int32_t)((cf % ctx->plane) / ctx->nxp);
         a.probe_i = (int32_t)(cf % ctx->nxp);
         a.probe_n3 = ctx->probe_n3;
@@ -681,18 +786,18 @@ static StepArgs<R> make_args(php_ctx* ctx, int s_local)
         a.probe_cap = kProbeCap;
     }
     a.rv_unit = ctx->rv_unit;
-    if (ctx->fused) {
-        for (int q = 0; q < 3; q++) {
-            a.enew[q] = (R*)ctx->fo[PHP_EX + q];
-            a.hnew[q] = (R*)ctx->fo[PHP_HX + q];
-        }
-        for (int q = 0; q < 6; q++) a.psin_h[q] = (R*)ctx->psio[q];
-        a.plain_hf = ctx->plain_hf;
+    const bool dbl = ctx->fused || ctx->split;
+    for (int q = 0; q < 3; q++) {
+        a.enew[q] = (R*)(dbl ? ctx->fo : ctx->f)[PHP_EX + q];
+        a.hnew[q] = (R*)(dbl ? ctx->fo : ctx->f)[PHP_HX + q];
     }
+    for (int q = 0; q < 6; q++) a.psin_h[q] = (R*)(ctx->fused ? ctx->psio : ctx->psi)[q];
+    a.pcls = ctx->pcls;
+    a.zstep = ctx->zstep;
     return a;
 }
 
-/* After a one-launch step: the buffers it wrote hold the current E, H and H
+/* After a double-buffered step: the buffers it wrote hold the current E, H and H
  * CPML state (on the host side, for every later launch and read). */
 static void swap_levels(php_ctx* ctx)
 {
@@ -700,15 +805,24 @@ static void swap_levels(php_ctx* ctx)
         std::swap(ctx->f[PHP_EX + q], ctx->fo[PHP_EX + q]);
         std::swap(ctx->f[PHP_HX + q], ctx->fo[PHP_HX + q]);
     }
-    for (int q = 0; q < 6; q++) std::swap(ctx->psi[q], ctx->psio[q]);
+    if (ctx->fused)
+        for (int q = 0; q < 6; q++) std::swap(ctx->psi[q], ctx->psio[q]);
     std::swap(ctx->maps, ctx->maps_o);
     ctx->level ^= 1;
 }
 
-static inline void prof_mark(php_ctx* ctx, int s_local, int kind, int end)
+/* sweep launches of a step with the interior apart */
+static int split_launches(const php_ctx* ctx)
+{
+    int n = 0;
+    for (int c : ctx->nlist) n += c > 0;
+    return n;
+}
+
+static inline void prof_mark(php_ctx* ctx, int s_local, int kind, int end, cudaStream_t st = nullptr)
 {
     if (ctx->profile)
-        cudaEventRecordWithFlags(ctx->prof_ev[((size_t)s_local * kProfKinds + kind) * 2 + end], ctx->stream,
+        cudaEventRecordWithFlags(ctx->prof_ev[((size_t)s_local * kProfKinds + kind) * 2 + end], st ? st : ctx->stream,
                                  cudaEventRecordExternal);
 }
 
@@ -766,6 +880,41 @@ static void launch_ions(php_ctx* ctx)
     ion_update_cc<R, 64><<<grid, kIonTile, 0, st>>>(a);
 }
 
+/* The E sweep's launches over the block lists of its three kinds, beside each
+ * other; a.f and maps as for one launch. */
+template <typename R, int NA>
+static void launch_e_lists(php_ctx* ctx, int s_local, StepArgs<R>& a, const TmaMaps& maps)
+{
+    const dim3 block(kBlockX, kBlockY, 1);
+    const uint32_t smem = TmaGeom<R>::E_SMEM;
+    SideStreams& sd = *ctx->side;
+    auto fork = [&](int q) { cudaStreamWaitEvent(sd.s[q], sd.fork, 0); };
+    auto join = [&](int q) {
+        cudaEventRecord(sd.join[q], sd.s[q]);
+        cudaStreamWaitEvent(ctx->stream, sd.join[q], 0);
+    };
+    prof_mark(ctx, s_local, 1, 0);
+    cudaEventRecord(sd.fork, ctx->stream);
+    if (ctx->nlist[4]) { /* few blocks with long chains: first */
+        fork(0);
+        a.list = ctx->lists[4];
+        e_sweep_tma<R, false, NA, kEGeneral><<<ctx->nlist[4], block, smem, sd.s[0]>>>(a, maps);
+    }
+    if (ctx->nlist[3]) {
+        fork(1);
+        a.list = ctx->lists[3];
+        e_sweep_tma<R, false, NA, kEAtoms><<<ctx->nlist[3], block, smem, sd.s[1]>>>(a, maps);
+    }
+    if (ctx->nlist[2]) {
+        a.list = ctx->lists[2];
+        e_sweep_tma<R, false, 0, kEPlain><<<ctx->nlist[2], block, smem, ctx->stream>>>(a, maps);
+    }
+    if (ctx->nlist[4]) join(0);
+    if (ctx->nlist[3]) join(1);
+    prof_mark(ctx, s_local, 1, 1);
+    a.list = nullptr;
+}
+
 template <typename R, bool STRICT, int NA>
 static void launch_step_t(php_ctx* ctx, int s_local, int& launches)
 {
@@ -778,10 +927,37 @@ static void launch_step_t(php_ctx* ctx, int s_local, int& launches)
     bool do_h = ctx->step_part & 1, do_e = ctx->step_part & 2;
     const bool do_rest = ctx->step_part & 4;
     if constexpr (!STRICT) {
+        if (ctx->split && ctx->side && do_h && do_e && grid.z > 0) {
+            /* the interior and the H sweep of the rest read this level and
+             * write the other; then the E sweep of the rest, whose H is the new
+             * one */
+            StepArgs<R> in = a;
+            in.list = ctx->lists[0];
+            SideStreams& sd = *ctx->side;
+            cudaEventRecord(sd.fork, ctx->stream);
+            cudaStreamWaitEvent(sd.s[0], sd.fork, 0);
+            prof_mark(ctx, s_local, 5, 0);
+            interior_sweep_tma<R><<<ctx->nlist[0], block, FusedGeom<R, true>::SMEM, ctx->stream>>>(in, ctx->maps);
+            prof_mark(ctx, s_local, 5, 1);
+            a.list = ctx->lists[1];
+            prof_mark(ctx, s_local, 0, 0, sd.s[0]);
+            h_sweep_tma<R, STRICT><<<ctx->nlist[1], block, TmaGeom<R>::H_SMEM, sd.s[0]>>>(a, ctx->maps);
+            prof_mark(ctx, s_local, 0, 1, sd.s[0]);
+            cudaEventRecord(sd.join[0], sd.s[0]);
+            cudaStreamWaitEvent(ctx->stream, sd.join[0], 0);
+            TmaMaps me = ctx->maps;
+            me.h_halo = ctx->maps_o.h_halo;
+            launch_e_lists<R, NA>(ctx, s_local, a, me);
+            launches += split_launches(ctx);
+            swap_levels(ctx);
+            do_h = do_e = false;
+        }
         if (ctx->fused && do_h && do_e && grid.z > 0) {
             /* the one-launch step: reads this level, writes the other */
             prof_mark(ctx, s_local, 5, 0);
-            he_sweep_tma<R, NA><<<grid, block, FusedGeom<R>::SMEM, ctx->stream>>>(a, ctx->maps);
+            const dim3 fgrid((ctx->nx + FusedGeom<R, false>::TX - 1) / FusedGeom<R, false>::TX, (ctx->ny + FusedGeom<R, false>::TY - 1) / FusedGeom<R, false>::TY,
+                             (ctx->nz + ctx->zstep - 1) / ctx->zstep);
+            he_sweep_tma<R, NA><<<fgrid, block, FusedGeom<R, false>::SMEM, ctx->stream>>>(a, ctx->maps);
             prof_mark(ctx, s_local, 5, 1);
             launches++;
             swap_levels(ctx);
@@ -795,9 +971,16 @@ static void launch_step_t(php_ctx* ctx, int s_local, int& launches)
         prof_mark(ctx, s_local, 0, 1);
         launches++;
     }
+    if constexpr (!STRICT) {
+        if (ctx->by_class && ctx->side && do_e && ctx->zc_count < 0) {
+            launch_e_lists<R, NA>(ctx, s_local, a, ctx->maps);
+            launches += split_launches(ctx);
+            do_e = false;
+        }
+    }
     if (do_e && grid.z > 0) {
         prof_mark(ctx, s_local, 1, 0);
-        e_sweep_tma<R, STRICT, NA><<<grid, block, TmaGeom<R>::E_SMEM + a.nmat * sizeof(MatCoef<R>), ctx->stream>>>(a, ctx->maps);
+        e_sweep_tma<R, STRICT, NA, kEAll><<<grid, block, TmaGeom<R>::E_SMEM, ctx->stream>>>(a, ctx->maps);
         prof_mark(ctx, s_local, 1, 1);
         launches++;
     }
@@ -812,11 +995,9 @@ static void launch_step_t(php_ctx* ctx, int s_local, int& launches)
     }
     if (ctx->probe && !probe_folded(ctx)) {
         prof_mark(ctx, s_local, 2, 0);
-        R* const* fp = reinterpret_cast<R* const*>(ctx->f);
-        Fields<R> f{fp[0], fp[1], fp[2], fp[3], fp[4], fp[5], fp[6], fp[7], fp[8]};
         const int threads = (9 + 2 * ctx->probe_n3 + 31) / 32 * 32;
         probe_record_counted<R><<<1, threads, 0, ctx->stream>>>(
-            f, ctx->probe_cf, (const R*)ctx->r, (const R*)ctx->v, ctx->rv_unit, ctx->nslot, ctx->probe_slot,
+            make_fields<R>(ctx), (const R*)ctx->Dp, ctx->probe_d, ctx->probe_cf, (const R*)ctx->r, (const R*)ctx->v, ctx->rv_unit, ctx->nslot, ctx->probe_slot,
             ctx->probe_n3, ctx->probe_rows, ctx->probe_count, kProbeCap, 9 + 2 * ctx->probe_n3);
         prof_mark(ctx, s_local, 2, 1);
         launches++;
@@ -826,10 +1007,9 @@ static void launch_step_t(php_ctx* ctx, int s_local, int& launches)
     for (size_t q = 0; q < ctx->dft.size(); q++) {
         if (dft_folded(ctx, q)) continue; /* sampled by the E sweep */
         const DftPlane& p = ctx->dft[q];
-        R* const* fp = reinterpret_cast<R* const*>(ctx->f);
         const int64_t n = (int64_t)ctx->nx * ctx->ny;
         int blocks = (int)std::min<int64_t>((n + 255) / 256, 148 * 8);
-        dft_sample<R><<<blocks, 256, 0, ctx->stream>>>(fp[p.comp], (int64_t)p.z * ctx->plane, ctx->nx, ctx->ny, ctx->nxp,
+        dft_sample<R><<<blocks, 256, 0, ctx->stream>>>(make_fields<R>(ctx), make_dview<R>(ctx), p.comp, (int64_t)p.z * ctx->plane, ctx->nx, ctx->ny, ctx->nxp,
                                                        p.nfreq, p.cast_f32, ctx->step_in + (size_t)s_local * ctx->step_row,
                                                        p.in_off, p.in_off + 1, p.acc);
         launches++;
@@ -840,6 +1020,26 @@ static void launch_step_t(php_ctx* ctx, int s_local, int& launches)
 typedef void (*step_fn)(php_ctx*, int, int&);
 typedef int (*prep_fn)(php_ctx*);
 
+/* Planes per block of he_sweep_tma: a block pays about two planes more than
+ * its range (the H of the plane below it, the E above, the first loads), and
+ * blocks run in waves of `slots`, the last one partly empty: the range with
+ * the shortest waves x (planes + 2). */
+static int fused_zstep(int tiles, int nz, int slots)
+{
+    int best = std::max(1, nz);
+    double cost = 1e300;
+    for (int n = 1; n <= nz; n++) {
+        const int64_t blocks = (int64_t)tiles * ((nz + n - 1) / n);
+        const double waves = std::max(1.0, blocks <= 4 * (int64_t)slots ? std::ceil((double)blocks / slots) : (double)blocks / slots + 0.5);
+        const double t = waves * (n + 2.0);
+        if (t < cost) {
+            cost = t;
+            best = n;
+        }
+    }
+    return best;
+}
+
 /* the TMA sweeps need more than the default 48 KB of dynamic shared memory */
 template <typename R, bool STRICT, int NA>
 static int prepare_t(php_ctx* ctx)
@@ -847,12 +1047,32 @@ static int prepare_t(php_ctx* ctx)
     cudaError_t e = cudaFuncSetAttribute(h_sweep_tma<R, STRICT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)TmaGeom<R>::H_SMEM);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(e_sweep_tma<R, STRICT, NA>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(TmaGeom<R>::E_SMEM + kSmemMats * sizeof(MatCoef<R>)));
+        e = cudaFuncSetAttribute(e_sweep_tma<R, STRICT, NA, kEAll>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)TmaGeom<R>::E_SMEM);
+    if constexpr (!STRICT)
+        if (e == cudaSuccess && (ctx->split || ctx->by_class)) {
+            const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
+            e = cudaFuncSetAttribute(e_sweep_tma<R, STRICT, 0, kEPlain>, at, (int)TmaGeom<R>::E_SMEM);
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(e_sweep_tma<R, STRICT, NA, kEAtoms>, at, (int)TmaGeom<R>::E_SMEM);
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(e_sweep_tma<R, STRICT, NA, kEGeneral>, at, (int)TmaGeom<R>::E_SMEM);
+        }
+    if constexpr (!STRICT)
+        if (e == cudaSuccess && ctx->split)
+            e = cudaFuncSetAttribute(interior_sweep_tma<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)FusedGeom<R, true>::SMEM);
     if constexpr (!STRICT)
         if (e == cudaSuccess && ctx->fused)
             e = cudaFuncSetAttribute(he_sweep_tma<R, NA>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)FusedGeom<R>::SMEM);
+                                     (int)FusedGeom<R, false>::SMEM);
+    if constexpr (!STRICT) {
+        if (e == cudaSuccess && ctx->fused) { /* planes per block */
+            int nb = 0;
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, he_sweep_tma<R, NA>, kBlockX * kBlockY, FusedGeom<R, false>::SMEM);
+            const int tiles = ((ctx->nx + FusedGeom<R, false>::TX - 1) / FusedGeom<R, false>::TX) *
+                              ((ctx->ny + FusedGeom<R, false>::TY - 1) / FusedGeom<R, false>::TY);
+            ctx->zstep = ctx->d.z_chunk > 0 ? ctx->d.z_chunk : fused_zstep(tiles, ctx->nz, std::max(1, nb) * ctx->num_sms);
+        }
+    }
     if (e != cudaSuccess) return fail(ctx, PHP_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     return PHP_OK;
 }
@@ -886,8 +1106,10 @@ static StepKernels pick_step(const php_ctx* ctx)
 
 /* ------------------------------------------------------------ tensor maps */
 
+/* d3, s3: size and byte stride of a fourth dimension, all of it in the box
+ * (0: three dimensions) */
 static int encode_map(php_ctx* ctx, CUtensorMap* m, void* base, CUtensorMapDataType dt, size_t esize, uint64_t d0,
-                      uint64_t d1, uint64_t d2, uint32_t b0, uint32_t b1)
+                      uint64_t d1, uint64_t d2, uint32_t b0, uint32_t b1, uint32_t d3 = 0, uint64_t s3 = 0)
 {
     static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
     if (!encode) {
@@ -898,39 +1120,42 @@ static int encode_map(php_ctx* ctx, CUtensorMap* m, void* base, CUtensorMapDataT
             return fail(ctx, PHP_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
         encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
     }
-    const cuuint64_t dims[3] = {d0, d1, d2};
-    const cuuint64_t strides[2] = {d0 * esize, d0 * d1 * esize};
-    const cuuint32_t box[3] = {b0, b1, 1};
-    const cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = encode(m, dt, 3, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    const cuuint64_t dims[4] = {d0, d1, d2, d3};
+    const cuuint64_t strides[3] = {d0 * esize, d0 * d1 * esize, s3};
+    const cuuint32_t box[4] = {b0, b1, 1, d3};
+    const cuuint32_t estr[4] = {1, 1, 1, 1};
+    CUresult r = encode(m, dt, d3 ? 4 : 3, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                         CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(ctx, PHP_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
     return PHP_OK;
 }
 
-/* Maps of the field arrays (planes -1..nz) and the material ids (planes
- * 0..nz-1) with the boxes of php_sweeps_tma.cuh. */
+/* Maps of the field arrays (planes -1..nz) with the boxes of
+ * php_sweeps_tma.cuh and php_sweep_fused.cuh. */
 template <typename R>
 static int make_maps(php_ctx* ctx)
 {
     using G = TmaGeom<R>;
+    using F = FusedGeom<R, false>;
+    using I = FusedGeom<R, true>;
     const CUtensorMapDataType dt = sizeof(R) == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
     const uint64_t nxp = ctx->nxp, ny = ctx->ny, nzh = ctx->nz + 2;
+    const uint64_t comp = (uint64_t)ctx->plane * nzh * sizeof(R); /* bytes from one component to the next */
     int rc = PHP_OK;
-    using F = FusedGeom<R>;
-    /* maps of the current buffers, then (one-launch step) of the second ones */
-    for (int set = 0; set < (ctx->fused ? 2 : 1) && !rc; ++set) {
+    /* maps of the current buffers, then of the second ones */
+    for (int set = 0; set < (ctx->fused || ctx->split ? 2 : 1) && !rc; ++set) {
         TmaMaps& m = set ? ctx->maps_o : ctx->maps;
         void* const* fb = set ? ctx->fo : ctx->f;
-        auto base = [&](int q) { return (void*)((char*)fb[q] - (size_t)ctx->plane * sizeof(R)); };
-        for (int q = 0; q < 3 && !rc; ++q) {
-            rc = encode_map(ctx, &m.e_halo[q], base(PHP_EX + q), dt, sizeof(R), nxp, ny, nzh, G::BX, G::BY);
-            if (!rc) rc = encode_map(ctx, &m.h_own[q], base(PHP_HX + q), dt, sizeof(R), nxp, ny, nzh, G::TX, G::TY);
-            if (!rc) rc = encode_map(ctx, &m.h_halo[q], base(PHP_HX + q), dt, sizeof(R), nxp, ny, nzh, G::BX, G::BY);
-            if (!rc) rc = encode_map(ctx, &m.d_own[q], base(PHP_DX + q), dt, sizeof(R), nxp, ny, nzh, G::TX, G::TY);
-            if (!rc) rc = encode_map(ctx, &m.e_wide[q], base(PHP_EX + q), dt, sizeof(R), nxp, ny, nzh, F::EX, F::EY);
-        }
-        if (!rc) rc = encode_map(ctx, &m.mat, ctx->mat, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, nxp, ny, ctx->nz, G::TX, G::TY);
+        auto map = [&](CUtensorMap& t, int field, uint32_t bx, uint32_t by) {
+            if (!rc)
+                rc = encode_map(ctx, &t, (char*)fb[field] - (size_t)ctx->plane * sizeof(R), dt, sizeof(R), nxp, ny, nzh, bx, by, 3, comp);
+        };
+        map(m.e_halo, PHP_EX, G::BX, G::BY);
+        map(m.h_own, PHP_HX, G::TX, G::TY);
+        map(m.h_halo, PHP_HX, G::BX, G::BY);
+        map(m.own, ctx->prec == PHP_PREC_FP64_STRICT ? PHP_DX : PHP_EX, G::TX, G::TY);
+        map(m.e_wide, PHP_EX, ctx->split ? I::EX : F::EX, ctx->split ? I::EY : F::EY);
+        map(m.h_wide, PHP_HX, ctx->split ? I::HX : F::HX, ctx->split ? I::HY : F::HY);
     }
     return rc;
 }
@@ -948,14 +1173,16 @@ static int upload_tables(php_ctx* ctx, const std::vector<MatD>& mats, const std:
         mc[i] = pack_material<R>(ctx, mats[i], ion_off[i]);
         if (mc[i].flags & kIso) ctx->iso_scale[i] = (double)mc[i].eps_inv[0];
         for (int q = 0; q < 9; q++) {
-            ctx->mat_tns[i][q] = (double)mc[i].eps_inv[q];
+            ctx->mat_tns[i][q] = (double)mc[i].em[q];
             ctx->mat_tns[i][9 + q] = (double)mc[i].eps_im[q];
         }
-        ctx->mat_tns[i][18] = (double)mc[i].cs;
-        ctx->mat_tns[i][19] = (double)mc[i].sn;
         if ((int)i == ctx->atom_id) {
             const unsigned char* p = reinterpret_cast<const unsigned char*>(&mc[i]);
             ctx->atom_mc.assign(p, p + sizeof(MatCoef<R>));
+        }
+        if ((int)i == ctx->ade_id) {
+            const unsigned char* p = reinterpret_cast<const unsigned char*>(&mc[i]);
+            ctx->ade_mc.assign(p, p + sizeof(MatCoef<R>));
         }
     }
     int rc = dalloc(ctx, &ctx->mc, mc.size() * sizeof(MatCoef<R>));
@@ -976,9 +1203,6 @@ static int upload_tables(php_ctx* ctx, const std::vector<MatD>& mats, const std:
             if (rc) return rc;
             if ((rc = upload(ctx, ctx->axis_tab[ax][q], h.data(), h.size() * sizeof(R)))) return rc;
         }
-        rc = dalloc(ctx, (void**)&ctx->axis_slot[ax], A.slot.size() * sizeof(int32_t));
-        if (rc) return rc;
-        if ((rc = upload(ctx, ctx->axis_slot[ax], A.slot.data(), A.slot.size() * sizeof(int32_t)))) return rc;
     }
     /* host tables must stay alive until the copies finish */
     CK(cudaStreamSynchronize(ctx->stream));
@@ -1063,6 +1287,55 @@ static void upload_release(php_ctx* ctx)
     }
 }
 
+static std::mutex g_side_mu;
+static std::vector<SideStreams*> g_side_free;
+
+static void side_destroy(SideStreams* s)
+{
+    for (int q = 0; q < 2; q++) {
+        if (s->join[q]) cudaEventDestroy(s->join[q]);
+        if (s->s[q]) cudaStreamDestroy(s->s[q]);
+    }
+    if (s->fork) cudaEventDestroy(s->fork);
+    delete s;
+}
+
+static SideStreams* side_get(int device)
+{
+    {
+        std::lock_guard<std::mutex> g(g_side_mu);
+        for (size_t q = 0; q < g_side_free.size(); q++)
+            if (g_side_free[q]->device == device) {
+                SideStreams* s = g_side_free[q];
+                g_side_free.erase(g_side_free.begin() + q);
+                return s;
+            }
+    }
+    SideStreams* s = new SideStreams();
+    s->device = device;
+    bool ok = cudaEventCreateWithFlags(&s->fork, cudaEventDisableTiming) == cudaSuccess;
+    for (int q = 0; q < 2 && ok; q++)
+        ok = cudaStreamCreateWithFlags(&s->s[q], cudaStreamNonBlocking) == cudaSuccess &&
+             cudaEventCreateWithFlags(&s->join[q], cudaEventDisableTiming) == cudaSuccess;
+    if (ok) return s;
+    cudaGetLastError();
+    side_destroy(s);
+    return nullptr;
+}
+
+static void side_put(SideStreams* s)
+{
+    if (!s) return;
+    {
+        std::lock_guard<std::mutex> g(g_side_mu);
+        if (g_side_free.size() < kSidePool) {
+            g_side_free.push_back(s);
+            return;
+        }
+    }
+    side_destroy(s);
+}
+
 static void ctx_free(php_ctx* ctx)
 {
     if (!ctx) return;
@@ -1076,8 +1349,9 @@ static void ctx_free(php_ctx* ctx)
     pinned_put(ctx->host_stage);
     for (int b = 0; b < 2; ++b) {
         pinned_put(ctx->step_in_host[b]);
-        if (ctx->staged[b]) cudaEventDestroy(ctx->staged[b]);
     }
+    for (cudaEvent_t e : ctx->staged)
+        if (e) cudaEventDestroy(e);
     upload_release(ctx);
     for (int b = 0; b < 2; ++b)
         if (ctx->up_ev[b]) cudaEventDestroy(ctx->up_ev[b]);
@@ -1107,8 +1381,9 @@ static int alloc_step_inputs(php_ctx* ctx, int row)
         pinned_put(ctx->step_in_host[b]);
         ctx->step_in_host[b] = (double*)pinned_get((size_t)kMaxChunk * row * sizeof(double));
         if (!ctx->step_in_host[b]) return fail(ctx, PHP_ERR_OOM, "page-locked host allocation failed");
-        if (!ctx->staged[b]) CK(cudaEventCreateWithFlags(&ctx->staged[b], cudaEventDisableTiming));
     }
+    for (int q = 0; q < 2 * kMaxChunk / ctx->max_chunk; q++)
+        if (!ctx->staged[q]) CK(cudaEventCreateWithFlags(&ctx->staged[q], cudaEventDisableTiming));
     ctx->step_in = ctx->step_in_dev[0];
     return PHP_OK;
 }
@@ -1237,6 +1512,186 @@ static int setup_ion_pass(php_ctx* ctx, const std::vector<MatD>& mats, const std
     return PHP_OK;
 }
 
+/* E = em D with em a multiple of the identity and no loss (kIso) */
+static bool is_iso(const MatD& s)
+{
+    const double* e = s.eps_inv;
+    return s.e_only && !(s.flags & (kLossy | kRotZ | kRotX)) && e[1] == 0.0 && e[2] == 0.0 && e[3] == 0.0 && e[5] == 0.0 &&
+           e[6] == 0.0 && e[7] == 0.0 && e[0] == e[4] && e[0] == e[8];
+}
+
+/* Sizes from which the interior runs in a launch of its own, and the share
+ * of the cells it has to hold: below, its blocks do not fill the GPU, or the
+ * third launch costs what the interior saves. */
+constexpr int64_t kSplitCells = 8 << 20;
+constexpr double kSplitShare = 0.4;
+static bool split_size(const php_desc& d) { return (int64_t)d.nx * d.ny * d.nz >= kSplitCells; }
+
+/* Whether the E sweep in place takes a launch per kind of block, where atom
+ * blocks want other registers than the rest: from about 74^3 cells (two-atom
+ * slab: step of 64^3 21.4 -> 19.7 us FP64, 17.4 -> 17.5 us FP32; 80^3 34.8 ->
+ * 32.1, 28.5 -> 25.9; 128^3 112.9 -> 104.5, 78.1 -> 72.0; 192^3 319 -> 296,
+ * 215 -> 192). */
+constexpr int64_t kByClassCells = 400000;
+static bool by_class_size(const php_ctx* ctx)
+{
+    return (int64_t)ctx->nx * ctx->ny * ctx->nz >= kByClassCells;
+}
+
+/* Block classes of a domain in the fast modes, from the one material id (or
+ * -1) of each plane and 32 x 8 tile. */
+struct BlockPlan {
+    int nx = 0, ny = 0, nz = 0, gx = 0, gy = 0;
+    const AxisD* axes = nullptr;
+    std::vector<int> pml_before[3]; /* CPML cells of the axis below each index */
+    const int16_t* uni = nullptr;
+    bool on = false;
+    int atom_id = -1, tns_id = -1;
+    std::vector<std::array<int, 3>> src;
+    std::vector<char> iso;
+    /* the interior launch's blocks (tiles of inner_ty rows), and the planes and
+     * 32 x 8 tiles they cover */
+    std::vector<int4> inner;
+    std::vector<uint8_t> inner_cell;
+    int64_t inner_cells = 0;
+
+    /* no CPML cell in [lo, hi) of the axis */
+    bool no_pml(int ax, int lo, int hi) const
+    {
+        const std::vector<int>& n = pml_before[ax];
+        const int last = (int)n.size() - 1;
+        return n[std::min(hi, last)] == n[std::min(std::max(lo, 0), last)];
+    }
+    void set_axes(const AxisD* a)
+    {
+        axes = a;
+        for (int ax = 0; ax < 3; ax++) {
+            pml_before[ax].assign(1, 0);
+            for (int32_t s : a[ax].slot) pml_before[ax].push_back(pml_before[ax].back() + (s >= 0));
+        }
+    }
+    bool source_in(int i0, int j0, int ty, int k0, int k1) const
+    {
+        for (const auto& q : src)
+            if (q[0] >= i0 && q[0] < i0 + kBlockX && q[1] >= j0 && q[1] < j0 + ty && q[2] >= k0 && q[2] < k1) return true;
+        return false;
+    }
+    /* the one material of plane k over the tile's rows j0 .. j0+ty-1, or -1 */
+    int tile_id(int bx, int j0, int ty, int k) const
+    {
+        int id = uni[((size_t)k * gy + j0 / kBlockY) * gx + bx];
+        for (int q = j0 / kBlockY + 1; q < std::min(gy, (j0 + ty) / kBlockY) && id >= 0; q++)
+            if (uni[((size_t)k * gy + q) * gx + bx] != id) id = -1;
+        return id;
+    }
+    /* class of a block of one material id; inner: no CPML cell and no domain
+     * edge cell */
+    uint8_t code(int id, bool inner_blk) const
+    {
+        if (id < 0) return 255;
+        if (id < kIsoMats && iso[id]) return (uint8_t)(inner_blk ? id : kPlainCpml + id);
+        if (id == atom_id) return (uint8_t)kPlainAtoms;
+        return (uint8_t)(id == tns_id ? kPlainTensor : 255);
+    }
+    bool full(int i0, int j0, int ty) const { return i0 + kBlockX <= nx - 1 && j0 + ty <= ny - 1; } /* all i < nx-1, j < ny-1 */
+    /* H sweep: no CPML cell, every cell updated */
+    bool h_plain(int bx, int by, int k0, int k1) const
+    {
+        const int i0 = bx * kBlockX, j0 = by * kBlockY;
+        return full(i0, j0, kBlockY) && no_pml(0, i0, i0 + kBlockX) && no_pml(1, j0, j0 + kBlockY) && no_pml(2, k0, k1);
+    }
+    uint8_t e_class(int bx, int by, int k0, int k1) const
+    {
+        const int i0 = bx * kBlockX, j0 = by * kBlockY;
+        if (source_in(i0, j0, kBlockY, k0, k1)) return 255;
+        int id = tile_id(bx, j0, kBlockY, k0);
+        for (int k = k0 + 1; k < k1 && id >= 0; k++)
+            if (tile_id(bx, j0, kBlockY, k) != id) id = -1;
+        return code(id, i0 >= 1 && j0 >= 1 && h_plain(bx, by, k0, k1));
+    }
+    /* The interior: tiles of ty rows whose cells, and those one below in x and
+     * y, lie outside the CPML and off the domain edge; of them, runs of at
+     * least min_run planes of one plain or tensor material without a source,
+     * outside the z CPML with the plane below (the march starts with that
+     * plane's H).  Runs are cut into ranges: a range costs about two planes
+     * more than it holds, and the blocks run in waves of `slots`. */
+    void find_interior(int ty, int slots, int min_run)
+    {
+        struct Run { int bx, j0, k0, k1, cls; };
+        std::vector<Run> runs;
+        inner_cell.assign((size_t)nz * gy * gx, 0);
+        std::vector<char> ztop(nz + 1, 0); /* plane k and the one below it outside the CPML */
+        for (int k = 0; k < nz; k++) ztop[k] = axes[2].slot[k] < 0 && (k == 0 || axes[2].slot[k - 1] < 0);
+        for (int j0 = 0; j0 + ty <= ny - 1; j0 += ty)
+            for (int bx = 0; bx < gx; bx++) {
+                const int i0 = bx * kBlockX;
+                if (i0 < 1 || j0 < 1 || !full(i0, j0, ty) || !no_pml(0, i0 - 1, i0 + kBlockX) || !no_pml(1, j0 - 1, j0 + ty)) continue;
+                const bool s = source_in(i0, j0, ty, 0, nz);
+                int start = 0, cur = 255;
+                for (int k = 0; k <= nz; k++) {
+                    int c = 255;
+                    if (ztop[k] && !(s && source_in(i0, j0, ty, k, k + 1)))
+                        c = code(tile_id(bx, j0, ty, k), true);
+                    if (c == kPlainAtoms) c = 255;
+                    if (c == cur) continue;
+                    if (cur != 255 && k - start >= min_run) runs.push_back({bx, j0, start, k, cur});
+                    start = k;
+                    cur = c;
+                }
+            }
+        int best = 8;
+        double cost = 1e300;
+        for (int n = 8; n <= 64; n++) {
+            int64_t blocks = 0;
+            for (const Run& r : runs) blocks += (r.k1 - r.k0 + n - 1) / n;
+            const double w = (double)blocks / slots, waves = w <= 4.0 ? std::ceil(w) : w + 0.5;
+            if (waves * (n + 2.0) < cost) {
+                cost = waves * (n + 2.0);
+                best = n;
+            }
+        }
+        for (const Run& r : runs) {
+            const int m = (r.k1 - r.k0 + best - 1) / best;
+            for (int q = 0; q < m; q++) {
+                const int a = r.k0 + (int)((int64_t)(r.k1 - r.k0) * q / m), b = r.k0 + (int)((int64_t)(r.k1 - r.k0) * (q + 1) / m);
+                inner.push_back(make_int4(r.bx | (r.j0 / ty) << 16, a, b, r.cls));
+            }
+            inner_cells += (int64_t)kBlockX * ty * (r.k1 - r.k0);
+            for (int k = r.k0; k < r.k1; k++)
+                for (int by = r.j0 / kBlockY; by < (r.j0 + ty) / kBlockY; by++) inner_cell[((size_t)k * gy + by) * gx + r.bx] = 1;
+        }
+        /* neighbouring tiles of one range run together: their halos meet in L2 */
+        std::stable_sort(inner.begin(), inner.end(), [](const int4& a, const int4& b) { return a.y < b.y; });
+    }
+    /* The blocks of the two sweeps over the rest: planes outside the interior
+     * in chunks of at most zc, cut where the class changes once half a chunk
+     * is full. */
+    void rest(int zc, std::vector<int4>& hj, std::vector<int4>& ej) const
+    {
+        for (int by = 0; by < gy; by++)
+            for (int bx = 0; bx < gx; bx++)
+                for (int sweep = 0; sweep < 2; sweep++) {
+                    auto cls = [&](int k0, int k1) { return sweep ? (int)e_class(bx, by, k0, k1) : (int)h_plain(bx, by, k0, k1); };
+                    for (int k = 0; k < nz;) {
+                        if (inner_cell[((size_t)k * gy + by) * gx + bx]) {
+                            k++;
+                            continue;
+                        }
+                        int e = k + 1;
+                        const int c = cls(k, k + 1);
+                        while (e < nz && e - k < zc && !inner_cell[((size_t)e * gy + by) * gx + bx] &&
+                               !(2 * (e - k) >= zc && cls(e, e + 1) != c))
+                            e++;
+                        (sweep ? ej : hj).push_back(make_int4(bx | by << 16, k, e, cls(k, e)));
+                        k = e;
+                    }
+                }
+        auto order = [](const int4& a, const int4& b) { return a.y < b.y; };
+        std::stable_sort(hj.begin(), hj.end(), order);
+        std::stable_sort(ej.begin(), ej.end(), order);
+    }
+};
+
 static int create_impl(const php_desc* desc, php_ctx* ctx)
 {
     const php_desc& d = *desc;
@@ -1304,6 +1759,10 @@ static int create_impl(const php_desc* desc, php_ctx* ctx)
     std::vector<int32_t> slot_n3;
     int n3max = 0;
     std::vector<int64_t> mat_cells(d.num_materials, 0);
+    /* per plane and 32 x 8 tile: the one material id of its cells, or -1 */
+    const int gx = (nx + kBlockX - 1) / kBlockX, gy = (ny + kBlockY - 1) / kBlockY;
+    std::vector<int16_t> uni((size_t)gx * gy * nz, -1);
+    const bool strict = ctx->prec == PHP_PREC_FP64_STRICT;
     {
         /* the medium from file order (z fastest) into the device layout (x
          * fastest), with the pool slots of ADE and atom cells in device cell
@@ -1324,7 +1783,7 @@ static int create_impl(const php_desc* desc, php_ctx* ctx)
             Part& P = parts[t];
             P.count.assign(d.num_materials, 0);
             const int k0 = (int)((int64_t)nz * t / nt), k1 = (int)((int64_t)nz * (t + 1) / nt);
-            for (int k = k0; k < k1; k++)
+            for (int k = k0; k < k1; k++) {
                 for (int j = 0; j < ny; j++)
                     for (int i = 0; i < nx; i++) {
                         const int32_t id = d.medium[((size_t)i * ny + j) * nz + k];
@@ -1337,7 +1796,7 @@ static int create_impl(const php_desc* desc, php_ctx* ctx)
                         const int64_t c = ((int64_t)k * ny + j) * nxp + i;
                         mat_dev[c] = (uint8_t)id;
                         P.count[id]++;
-                        if (mats[id].flags & (kAde | kAtoms)) {
+                        if (mats[id].slotted(strict)) {
                             P.cell.push_back(c);
                             P.n3.push_back(3 * mats[id].natom);
                             P.n3max = std::max(P.n3max, 3 * mats[id].natom);
@@ -1345,6 +1804,15 @@ static int create_impl(const php_desc* desc, php_ctx* ctx)
                             if (mats[id].flags & kAtoms) P.atoms = true;
                         }
                     }
+                for (int by = 0; by < gy && !strict; by++)
+                    for (int bx = 0; bx < gx; bx++) {
+                        const int i0 = bx * kBlockX, w = std::min(kBlockX, nx - i0), j1 = std::min((by + 1) * kBlockY, ny);
+                        const uint8_t* first = &mat_dev[((int64_t)k * ny + by * kBlockY) * nxp + i0];
+                        bool same = w < 2 || !memcmp(first, first + 1, w - 1);
+                        for (int j = by * kBlockY + 1; j < j1 && same; j++) same = !memcmp(first, first + (int64_t)(j - by * kBlockY) * nxp, w);
+                        if (same) uni[((size_t)k * gy + by) * gx + bx] = *first;
+                    }
+            }
         };
         std::vector<std::thread> th;
         for (int t = 1; t < nt; t++) th.emplace_back(work, t);
@@ -1395,6 +1863,9 @@ static int create_impl(const php_desc* desc, php_ctx* ctx)
             ctx->atom_id = best;
         }
     }
+    for (int i = 0; i < d.num_materials; i++)
+        if ((mats[i].flags & (kAde | kAtoms)) == kAde && mat_cells[i] > 0 && (ctx->ade_id < 0 || mat_cells[i] > mat_cells[ctx->ade_id]))
+            ctx->ade_id = i;
     const int namax = n3max / 3;
     ctx->namax_tpl = namax == 0 ? 0 : namax <= 2 ? 2 : namax <= 4 ? 4 : namax <= 8 ? 8 : namax <= 16 ? 16 : 64;
     if (namax > 64) return fail(ctx, PHP_ERR_UNSUPPORTED, "natom %d above the supported 64", namax);
@@ -1420,17 +1891,70 @@ static int create_impl(const php_desc* desc, php_ctx* ctx)
         ctx->nsrc_active++;
     }
 
-    /* z chunking: short marches while keeping at least ~4 waves of blocks on
+    /* z chunking: short marches while keeping at least ~2 waves of blocks on
      * 148 SMs.  Measured on 256^3 (the tip workload): FP64 fastest with 4
      * planes per block (E sweep 0.331 ms, H 0.210 ms; 8 planes 0.339 and
      * 0.214; 16 planes 0.364 and 0.225), FP32 with 8 (E 0.204 ms; 4 planes
-     * 0.210, 16 planes 0.219) */
+     * 0.210, 16 planes 0.219); on the 96^3 two-atom slab with 2 (1728 blocks;
+     * FP64 step 56.3 us, 1 plane 61.0, 4 planes 62.5; FP32 36.6, 39.1, 39.7),
+     * on 101 x 67 x 53 with 1 (1908 blocks; strict step 51 us, 2 planes 56) */
     {
         const int tiles = ((nx + kBlockX - 1) / kBlockX) * ((ny + kBlockY - 1) / kBlockY);
         int zc = std::min(ctx->prec == PHP_PREC_FP32 ? 8 : 4, nz);
-        while (zc > 1 && (int64_t)tiles * ((nz + zc - 1) / zc) < 148 * 4 * 4) zc /= 2;
+        while (zc > 1 && (int64_t)tiles * ((nz + zc - 1) / zc) < 148 * 4 * 2) zc /= 2;
         ctx->zchunk = d.z_chunk > 0 ? d.z_chunk : zc;
     }
+    AxisD axes[3];
+    derive_axis(d, nx, d.dx, false, axes[0]);
+    derive_axis(d, ny, d.dy, false, axes[1]);
+    derive_axis(d, ctx->nz_glob, d.dz, true, axes[2]);
+    if (ctx->nz_glob != nz) { /* a z slab: its planes of the global profile */
+        AxisD& z = axes[2];
+        auto cut = [&](auto& v) { v = std::vector<typename std::decay_t<decltype(v)>::value_type>(
+                                      v.begin() + ctx->z_off, v.begin() + ctx->z_off + nz); };
+        cut(z.slot); cut(z.kappa); cut(z.b); cut(z.c); cut(z.kh); cut(z.kd); cut(z.ch); cut(z.cd);
+    }
+    /* block classes of the fast modes (see plan_split and the plain blocks
+     * below) */
+    BlockPlan plan;
+    plan.nx = nx, plan.ny = ny, plan.nz = nz, plan.gx = gx, plan.gy = gy;
+    plan.set_axes(axes);
+    plan.uni = uni.data();
+    {
+        const char* pv = getenv("PHP_PLAIN");
+        const char* tv = getenv("PHP_PLAIN_TENSOR");
+        plan.on = !strict && !(pv && !strcmp(pv, "0"));
+        for (int s = 0; s < ctx->nsrc_active; s++) {
+            const int64_t sc = ctx->src_cell[s];
+            plan.src.push_back({(int)(sc % nxp), (int)((sc % ctx->plane) / nxp), (int)(sc / ctx->plane)});
+        }
+        for (const MatD& m : mats) plan.iso.push_back(!strict && is_iso(m));
+        /* the lossy or anisotropic material filling the most tiles */
+        std::vector<size_t> count(mats.size(), 0);
+        if (plan.on && !(tv && !strcmp(tv, "0")))
+            for (int16_t id : uni)
+                if (id >= 0 && mats[id].e_only && !plan.iso[id]) count[id]++;
+        for (size_t id = 0; id < count.size(); id++)
+            if (count[id] && (ctx->tns_id < 0 || count[id] > count[ctx->tns_id])) ctx->tns_id = (int)id;
+        plan.tns_id = ctx->tns_id;
+    }
+    /* the interior in a launch of its own (interior_sweep_tma) */
+    {
+        const char* fv = getenv("PHP_FUSED");
+        const bool whole = !strict && ctx->z_off == 0 && ctx->nz_glob == nz && ctx->allow_split && plan.on;
+        const bool forced = fv && !strcmp(fv, "2");
+        if (whole && (forced || (!fv && split_size(d)))) {
+            const int rows = ctx->prec == PHP_PREC_FP32 ? FusedGeom<float, true>::ROWS : FusedGeom<double, true>::ROWS;
+            plan.find_interior(kBlockY * rows, ctx->num_sms * (ctx->prec == PHP_PREC_FP32 ? PHP_INNER_MINB32 : PHP_INNER_MINB64),
+                               forced ? 2 : 8);
+            size_t free_b = 0, total_b = 0;
+            CK(cudaMemGetInfo(&free_b, &total_b));
+            const uint64_t need = 12 * (uint64_t)ctx->plane * (nz + 2) * rsize(ctx->prec);
+            ctx->split = !plan.inner.empty() &&
+                         (forced || (plan.inner_cells >= kSplitShare * (double)nx * ny * nz && need + total_b / 2 <= free_b));
+        }
+    }
+
     /* 32-bit cell offsets inside the sweeps */
     if ((int64_t)ctx->plane * (nz + 2) >= ((int64_t)1 << 31))
         return fail(ctx, PHP_ERR_UNSUPPORTED, "grid of %lld padded cells exceeds the 2^31 cell limit of one domain",
@@ -1439,11 +1963,18 @@ static int create_impl(const php_desc* desc, php_ctx* ctx)
     /* allocations */
     const size_t rs = rsize(ctx->prec);
     const size_t field_bytes = (size_t)ctx->plane * (nz + 2) * rs;
-    for (int q = 0; q < 9; q++) {
+    /* the three components of a field in one allocation (TmaMaps); in the fast
+     * modes Dp and E hold D */
+    auto alloc_field = [&](void** f3) -> int {
         void* p;
-        int rc = dalloc(ctx, &p, field_bytes);
+        int rc = dalloc(ctx, &p, 3 * field_bytes);
+        for (int q = 0; q < 3 && !rc; q++) f3[q] = (char*)p + q * field_bytes + (size_t)ctx->plane * rs; /* plane 0; plane -1 is the low halo */
+        return rc;
+    };
+    for (int f : {PHP_EX, PHP_DX, PHP_HX}) {
+        if (!strict && f == PHP_DX) continue;
+        int rc = alloc_field(&ctx->f[f]);
         if (rc) return rc;
-        ctx->f[q] = (char*)p + (size_t)ctx->plane * rs; /* plane 0; plane -1 is the low halo */
     }
     const int L = ctx->L;
     const size_t xs = (size_t)nz * ny * 2 * L, ys = (size_t)nz * 2 * L * nxp, zs = (size_t)2 * L * ny * nxp;
@@ -1460,19 +1991,14 @@ static int create_impl(const php_desc* desc, php_ctx* ctx)
     {
         const char* fv = getenv("PHP_FUSED");
         ctx->fused = ctx->prec != PHP_PREC_FP64_STRICT && ctx->z_off == 0 && ctx->nz_glob == nz && fv && !strcmp(fv, "1");
+        if (ctx->fused) ctx->split = false;
     }
-    if (ctx->fused) {
-        for (int q = 0; q < 9; q++) {
-            if (q >= PHP_DX && q < PHP_DX + 3) {
-                ctx->fo[q] = ctx->f[q];
-                continue;
-            }
-            void* p;
-            int rc = dalloc(ctx, &p, field_bytes);
+    if (ctx->split || ctx->fused) {
+        for (int f : {PHP_EX, PHP_HX}) {
+            int rc = alloc_field(&ctx->fo[f]);
             if (rc) return rc;
-            ctx->fo[q] = (char*)p + (size_t)ctx->plane * rs;
         }
-        for (int q = 0; q < 6; q++) {
+        for (int q = 0; q < 6 && ctx->fused; q++) {
             int rc = dalloc(ctx, &ctx->psio[q], psz[q] * rs);
             if (rc) return rc;
         }
@@ -1499,6 +2025,14 @@ static int create_impl(const php_desc* desc, php_ctx* ctx)
         if ((rc = upload(ctx, ctx->slot_mat, slot_mat.data(), slot_mat.size()))) return rc;
         CK(cudaStreamSynchronize(ctx->stream)); /* the host vectors go out of scope */
     }
+    if (!strict) {
+        if (ctx->nslot > 0 && (rc = dalloc(ctx, &ctx->Dp, 3 * (size_t)ctx->nslot * rs))) return rc;
+        if (ctx->prec == PHP_PREC_FP32 && ctx->any_atoms && (rc = dalloc(ctx, (void**)&ctx->Dc, (size_t)ctx->nslot * 4))) return rc;
+        std::vector<double> dm(9 * mats.size());
+        for (size_t i = 0; i < mats.size(); i++) memcpy(&dm[9 * i], mats[i].dm, sizeof(mats[i].dm));
+        if ((rc = dalloc(ctx, (void**)&ctx->dmat, dm.size() * sizeof(double)))) return rc;
+        if ((rc = upload(ctx, ctx->dmat, dm.data(), dm.size() * sizeof(double)))) return rc;
+    }
     if (ctx->any_ade) {
         if ((rc = dalloc(ctx, &ctx->P, 3 * (size_t)ctx->nslot * rs))) return rc;
         if ((rc = dalloc(ctx, &ctx->Po, 3 * (size_t)ctx->nslot * rs))) return rc;
@@ -1508,17 +2042,12 @@ static int create_impl(const php_desc* desc, php_ctx* ctx)
         if ((rc = dalloc(ctx, &ctx->v, (size_t)n3max * ctx->nslot * rs))) return rc;
     }
     if ((rc = setup_ion_pass(ctx, mats, ion_off, d))) return rc;
-
-    AxisD axes[3];
-    derive_axis(d, nx, d.dx, false, axes[0]);
-    derive_axis(d, ny, d.dy, false, axes[1]);
-    derive_axis(d, ctx->nz_glob, d.dz, true, axes[2]);
-    if (ctx->nz_glob != nz) { /* a z slab: its planes of the global profile */
-        AxisD& z = axes[2];
-        auto cut = [&](auto& v) { v = std::vector<typename std::decay_t<decltype(v)>::value_type>(
-                                      v.begin() + ctx->z_off, v.begin() + ctx->z_off + nz); };
-        cut(z.slot); cut(z.kappa); cut(z.b); cut(z.c); cut(z.kh); cut(z.kd); cut(z.ch); cut(z.cd);
+    if (ctx->ion_split) { /* the atom material whose blocks read their record from the kernel parameters */
+        ctx->atom_id = -1;
+        for (int i = 0; i < d.num_materials; i++)
+            if ((mats[i].flags & kAtoms) && (ctx->atom_id < 0 || mat_cells[i] > mat_cells[ctx->atom_id])) ctx->atom_id = i;
     }
+
     if (ctx->prec == PHP_PREC_FP32) rc = upload_tables<float>(ctx, mats, ion_off, ion_coef, axes);
     else rc = upload_tables<double>(ctx, mats, ion_off, ion_coef, axes);
     if (rc) return rc;
@@ -1534,85 +2063,71 @@ static int create_impl(const php_desc* desc, php_ctx* ctx)
      * few-atom material whose ions the sweep updates (kPlainAtoms;
      * PHP_PLAIN_ATOMS=0). */
     {
-        const char* pv = getenv("PHP_PLAIN");
-        const int gx = (nx + kBlockX - 1) / kBlockX, gy = (ny + kBlockY - 1) / kBlockY;
         const int gz = (nz + ctx->zchunk - 1) / ctx->zchunk;
-        std::vector<uint8_t> pm((size_t)gx * gy * gz, 255), ph(pm.size(), 0), phf(pm.size(), 0);
-        std::vector<char> src_tile(pm.size(), 0);
-        for (int s = 0; s < ctx->nsrc_active; s++) {
-            const int64_t sc = ctx->src_cell[s];
-            const int sk = (int)(sc / ctx->plane), sj = (int)((sc % ctx->plane) / nxp), si = (int)(sc % nxp);
-            src_tile[((size_t)(sk / ctx->zchunk) * gy + sj / kBlockY) * gx + si / kBlockX] = 1;
-        }
-        size_t nplain = 0, nplain_h = 0, nplain_hf = 0;
-        const char* tv = getenv("PHP_PLAIN_TENSOR");
-        const bool tns_off = tv && !strcmp(tv, "0");
-        /* blocks of the few-atom material when the fused sweep updates its
-         * ions (two or four atoms, no ion pass apart) */
+        std::vector<uint8_t> pm((size_t)gx * gy * gz, 255), ph(pm.size(), 0);
+        size_t nplain = 0, nplain_h = 0;
+        /* blocks of one atom material: the fused sweep updates its ions (two
+         * or four atoms), or the ion pass runs apart */
         const char* av = getenv("PHP_PLAIN_ATOMS");
-        const bool atoms_on = !(av && !strcmp(av, "0")) && ctx->atom_id >= 0 && !ctx->ion_split &&
-                              (ctx->namax_tpl == 2 || ctx->namax_tpl == 4) &&
-                              !(ctx->mat_flags[ctx->atom_id] & kAde) && ctx->atom_mc.size() > 0;
-        std::vector<int16_t> uni(pm.size(), -1);
-        std::vector<size_t> tns_count(ctx->mat_flags.size(), 0);
-        for (int bz = 0; bz < gz && !(pv && !strcmp(pv, "0")) && ctx->prec != PHP_PREC_FP64_STRICT; bz++)
+        if (!(av && !strcmp(av, "0")) && ctx->atom_id >= 0 && (ctx->ion_split || ctx->namax_tpl == 2 || ctx->namax_tpl == 4) &&
+            !(ctx->mat_flags[ctx->atom_id] & kAde) && ctx->atom_mc.size() > 0)
+            plan.atom_id = ctx->atom_id;
+        for (int bz = 0; bz < gz && plan.on; bz++)
             for (int by = 0; by < gy; by++)
                 for (int bx = 0; bx < gx; bx++) {
-                    const int i0 = bx * kBlockX, j0 = by * kBlockY, k0 = bz * ctx->zchunk;
-                    const int k1 = std::min(k0 + ctx->zchunk, nz);
+                    const int k0 = bz * ctx->zchunk, k1 = std::min(k0 + ctx->zchunk, nz);
                     const size_t b = ((size_t)bz * gy + by) * gx + bx;
-                    const int i1 = std::min(i0 + kBlockX, nx), j1 = std::min(j0 + kBlockY, ny);
-                    bool pml_free = true;
-                    for (int i = i0; i < i1 && pml_free; i++) pml_free = axes[0].slot[i] < 0;
-                    for (int j = j0; j < j1 && pml_free; j++) pml_free = axes[1].slot[j] < 0;
-                    for (int k = k0; k < k1 && pml_free; k++) pml_free = axes[2].slot[k] < 0;
-                    const bool full = i0 + kBlockX <= nx - 1 && j0 + kBlockY <= ny - 1; /* every cell has i < nx-1, j < ny-1 */
-                    if (full && pml_free) { /* the H sweep needs no more */
-                        ph[b] = 1;
-                        nplain_h++;
-                    }
-                    /* the one-launch step computes H one cell further down in
-                     * x, y and z: those cells must be outside the CPML too */
-                    bool ring_free = pml_free;
-                    if (ring_free && i0 >= 1) ring_free = axes[0].slot[i0 - 1] < 0;
-                    if (ring_free && j0 >= 1) ring_free = axes[1].slot[j0 - 1] < 0;
-                    if (ring_free && k0 >= 1) ring_free = axes[2].slot[k0 - 1] < 0;
-                    if (full && ring_free) {
-                        phf[b] = 1;
-                        nplain_hf++;
-                    }
-                    if (src_tile[b]) continue;
-                    const int id = mat_dev[((size_t)k0 * ny + j0) * nxp + i0];
-                    bool ok = id < (int)ctx->mat_flags.size() && id < (int)ctx->iso_scale.size();
-                    for (int k = k0; k < k1 && ok; k++)
-                        for (int j = j0; j < j1 && ok; j++) {
-                            const uint8_t* row = &mat_dev[((size_t)k * ny + j) * nxp];
-                            for (int i = i0; i < i1 && ok; i++) ok = row[i] == id;
-                        }
-                    if (!ok) continue;
-                    if (id < kIsoMats && ctx->iso_scale[id] != 0.0) {
-                        /* one plain material: the stencil-only path, or with CPML or
-                         * domain-edge cells the path that adds their CPML terms */
-                        pm[b] = (uint8_t)((full && i0 >= 1 && j0 >= 1 && pml_free) ? id : kPlainCpml + id);
-                        nplain++;
-                    } else if (atoms_on && id == ctx->atom_id) {
-                        pm[b] = (uint8_t)kPlainAtoms;
-                        nplain++;
-                        ctx->atom_blocks = true;
-                    } else if (!(ctx->mat_flags[id] & (kAde | kAtoms)) && ctx->iso_scale[id] == 0.0 && !tns_off) {
-                        uni[b] = (int16_t)id; /* a tensor block if id is the material chosen below */
-                        tns_count[id]++;
+                    ph[b] = plan.h_plain(bx, by, k0, k1);
+                    nplain_h += ph[b];
+                    pm[b] = plan.e_class(bx, by, k0, k1);
+                    nplain += pm[b] != 255;
+                }
+        ctx->atom_blocks = plan.atom_id >= 0;
+        if (ctx->fused) {
+            /* the one-launch step's classes, per plane and tile of its height;
+             * its H part also computes the cells one below the tile in x and y */
+            const int ty = kBlockY * (ctx->prec == PHP_PREC_FP32 ? FusedGeom<float, false>::ROWS : FusedGeom<double, false>::ROWS);
+            const int fy = (ny + ty - 1) / ty;
+            std::vector<uint16_t> pc((size_t)gx * fy * nz, 255);
+            for (int by = 0; by < fy && plan.on; by++)
+                for (int bx = 0; bx < gx; bx++) {
+                    const int i0 = bx * kBlockX, j0 = by * ty;
+                    const bool full = i0 + kBlockX <= nx - 1 && j0 + ty <= ny - 1;
+                    const bool inner = full && i0 >= 1 && j0 >= 1 && plan.no_pml(0, i0, i0 + kBlockX) && plan.no_pml(1, j0, j0 + ty);
+                    const bool ring = full && plan.no_pml(0, i0 - 1, i0 + kBlockX) && plan.no_pml(1, j0 - 1, j0 + ty);
+                    const bool src = plan.source_in(i0, j0, ty, 0, nz);
+                    for (int k = 0; k < nz; k++) {
+                        const bool zfree = axes[2].slot[k] < 0;
+                        const int id = src && plan.source_in(i0, j0, ty, k, k + 1) ? -1 : plan.tile_id(bx, j0, ty, k);
+                        pc[((size_t)k * fy + by) * gx + bx] = (uint16_t)(plan.code(id, inner && zfree) | (ring && zfree ? kHPlain : 0u));
                     }
                 }
-        /* the lossy or anisotropic material filling the most blocks */
-        for (size_t id = 0; id < tns_count.size(); id++)
-            if (tns_count[id] && (ctx->tns_id < 0 || tns_count[id] > tns_count[ctx->tns_id])) ctx->tns_id = (int)id;
-        if (ctx->tns_id >= 0)
-            for (size_t b = 0; b < pm.size(); b++)
-                if (uni[b] == ctx->tns_id) {
-                    pm[b] = (uint8_t)kPlainTensor;
-                    nplain++;
-                }
+            if ((rc = dalloc(ctx, (void**)&ctx->pcls, pc.size() * sizeof(uint16_t)))) return rc;
+            if ((rc = upload(ctx, ctx->pcls, pc.data(), pc.size() * sizeof(uint16_t)))) return rc;
+        }
+        ctx->by_class = !ctx->split && !ctx->fused && plan.on && plan.atom_id >= 0 && by_class_size(ctx);
+        if (ctx->split || ctx->by_class) {
+            ctx->max_chunk = kBranchChunk;
+            std::vector<int4> hj, ej_all;
+            if (ctx->split) {
+                plan.rest(ctx->prec == PHP_PREC_FP32 ? 8 : 4, hj, ej_all);
+            } else {
+                for (int bz = 0; bz < gz; bz++)
+                    for (int by = 0; by < gy; by++)
+                        for (int bx = 0; bx < gx; bx++)
+                            ej_all.push_back(make_int4(bx | by << 16, bz * ctx->zchunk, std::min((bz + 1) * ctx->zchunk, nz),
+                                                       pm[((size_t)bz * gy + by) * gx + bx]));
+            }
+            std::vector<int4> ej[3];
+            for (const int4& e : ej_all) ej[e.w == 255 ? 2 : e.w == kPlainAtoms ? 1 : 0].push_back(e);
+            const std::vector<int4>* jobs[5] = {&plan.inner, &hj, &ej[0], &ej[1], &ej[2]};
+            for (int q = 0; q < 5; q++) {
+                ctx->nlist[q] = (int)jobs[q]->size();
+                if (jobs[q]->empty()) continue;
+                if ((rc = dalloc(ctx, (void**)&ctx->lists[q], jobs[q]->size() * sizeof(int4)))) return rc;
+                if ((rc = upload(ctx, ctx->lists[q], jobs[q]->data(), jobs[q]->size() * sizeof(int4)))) return rc;
+            }
+        }
         for (size_t b = 0; b < pm.size(); b++) {
             const int c = pm[b] == 255 ? 4 : pm[b] == kPlainAtoms ? 3 : pm[b] == kPlainTensor ? 2
                         : pm[b] >= kPlainCpml ? 1 : 0;
@@ -1627,10 +2142,6 @@ static int create_impl(const php_desc* desc, php_ctx* ctx)
         if (nplain_h) {
             if ((rc = dalloc(ctx, (void**)&ctx->plain_h, ph.size()))) return rc;
             if ((rc = upload(ctx, ctx->plain_h, ph.data(), ph.size()))) return rc;
-        }
-        if (nplain_hf && ctx->fused) {
-            if ((rc = dalloc(ctx, (void**)&ctx->plain_hf, phf.size()))) return rc;
-            if ((rc = upload(ctx, ctx->plain_hf, phf.data(), phf.size()))) return rc;
         }
         ctx->khp[0] = d.dt / (d.mu0 * d.dx * 1.0);
         ctx->khp[1] = d.dt / (d.mu0 * d.dy * 1.0);
@@ -1650,7 +2161,9 @@ static int create_impl(const php_desc* desc, php_ctx* ctx)
     if (rc) return rc;
 
     /* per-step inputs, scratch, staging */
-    if ((rc = alloc_step_inputs(ctx, std::max(1, ctx->nsrc_active)))) return rc;
+    ctx->probe_off = ctx->nsrc_active;
+    if ((rc = alloc_step_inputs(ctx, ctx->probe_off + 1))) return rc;
+    if ((rc = dalloc(ctx, (void**)&ctx->src_acc, 3 * kMaxSources * sizeof(double)))) return rc;
     const size_t maxplane = std::max({(size_t)nx * ny, (size_t)ny * nz, (size_t)nx * nz});
     ctx->scratch_bytes = std::max(maxplane * sizeof(double), (size_t)4096 * sizeof(DiagPartial));
     if ((rc = dalloc(ctx, &ctx->scratch, ctx->scratch_bytes))) return rc;
@@ -1670,12 +2183,13 @@ static int create_impl(const php_desc* desc, php_ctx* ctx)
 
 /* Device bytes php_create will allocate for a description (the buffers of
  * create_impl, without DFT planes or the probe ring); no device needed. */
-static int estimate_bytes(const php_desc& d, uint64_t* out)
+static int estimate_bytes(const php_desc& d, uint64_t* out, uint64_t* more)
 {
     if (d.nx < 2 || d.ny < 2 || d.nz < 1 || d.num_materials < 1 || !d.materials || !d.medium || d.pml_thickness < 0 ||
         d.precision < 0 || d.precision > 2)
         return PHP_ERR_INPUT;
     const uint64_t rs = d.precision == PHP_PREC_FP32 ? 4 : 8;
+    const bool strict = d.precision == PHP_PREC_FP64_STRICT;
     const uint64_t nxp = (uint64_t)(d.nx + 31) / 32 * 32, plane = nxp * d.ny, ncell = plane * d.nz;
     std::vector<int> n3(d.num_materials, 0);
     std::vector<char> slotted(d.num_materials, 0);
@@ -1683,6 +2197,12 @@ static int estimate_bytes(const php_desc& d, uint64_t* out)
     for (int m = 0; m < d.num_materials; m++) {
         n3[m] = 3 * std::max(0, (int)d.materials[m].natom);
         slotted[m] = d.materials[m].use_ade == 1 || d.materials[m].natom > 0;
+        if (!slotted[m] && !strict) { /* a material that keeps D although it has no ADE and no atoms */
+            php_ctx probe;
+            MatD o;
+            probe.d = d;
+            slotted[m] = derive_material(&probe, m, d.materials[m], o) == PHP_OK && o.slotted(false);
+        }
     }
     uint64_t nslot = 0;
     int n3max = 0;
@@ -1698,7 +2218,9 @@ static int estimate_bytes(const php_desc& d, uint64_t* out)
         }
     }
     const uint64_t L = d.pml_thickness;
-    uint64_t b = 9 * plane * (d.nz + 2) * rs;
+    uint64_t b = (strict ? 9 : 6) * plane * (d.nz + 2) * rs;
+    /* second E and H buffers and block lists of the interior launch */
+    *more = !strict && split_size(d) ? 6 * plane * (d.nz + 2) * rs + 48 * ((uint64_t)d.nz * (d.nx / 32 + 1) * (d.ny / 8 + 1) / 2) : 0;
     b += 4 * ((uint64_t)d.nz * d.ny * 2 * L + (uint64_t)d.nz * 2 * L * nxp + 2 * L * d.ny * nxp) * rs;
     const char* fv = getenv("PHP_FUSED");
     if (d.precision != PHP_PREC_FP64_STRICT && fv && !strcmp(fv, "1")) { /* second E, H and H CPML buffers */
@@ -1706,7 +2228,8 @@ static int estimate_bytes(const php_desc& d, uint64_t* out)
         b += 2 * ((uint64_t)d.nz * d.ny * 2 * L + (uint64_t)d.nz * 2 * L * nxp + 2 * L * d.ny * nxp) * rs;
     }
     b += ncell; /* material ids */
-    if (nslot) b += ncell * 4 + nslot * 12;
+    if (nslot) b += ncell * 4 + nslot * 13;
+    if (nslot && !strict) b += 3 * nslot * rs + (any_atoms && rs == 4 ? 4 * nslot : 0);
     if (any_ade) b += 6 * nslot * rs;
     if (any_atoms) b += 2 * (uint64_t)n3max * nslot * rs;
     if (n3max >= 24 && d.precision != PHP_PREC_FP64_STRICT) b += 3 * nslot * rs + 64 * 64 * 8; /* ion pass */
@@ -1751,12 +2274,22 @@ static int record_graph(php_ctx* ctx, int n, int b, cudaGraphExec_t* out)
     ctx->step_in = ctx->step_in_dev[b];
     step_fn fn = pick_step(ctx).launch;
     cudaGraph_t g = nullptr;
-    CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
+    if (ctx->split || ctx->by_class) {
+        ctx->side = side_get(ctx->d.device);
+        if (!ctx->side) return fail(ctx, PHP_ERR_CUDA, "stream creation for a step's branches failed");
+    }
+    if (cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
+        side_put(ctx->side);
+        ctx->side = nullptr;
+        return fail(ctx, PHP_ERR_CUDA, "cudaStreamBeginCapture failed: %s", cudaGetErrorString(cudaGetLastError()));
+    }
     int launches = 0;
     for (int s = 0; s < n; s++) fn(ctx, s, launches);
     if (ctx->level != level) swap_levels(ctx);
     cudaError_t le = cudaGetLastError();
     cudaError_t ce = cudaStreamEndCapture(ctx->stream, &g);
+    side_put(ctx->side);
+    ctx->side = nullptr;
     if (le != cudaSuccess) {
         if (g) cudaGraphDestroy(g);
         return fail(ctx, PHP_ERR_CUDA, "kernel launch during capture failed: %s", cudaGetErrorString(le));
@@ -1778,9 +2311,19 @@ static void drop_graphs(php_ctx* ctx)
     ctx->graphs.clear();
 }
 
+/* The caller holds the addresses of planes, or orders the sweeps itself: the
+ * context's E and H stay where they are from now on (the buffers current at
+ * this point), stepped by the two sweeps. */
+static void step_in_place(php_ctx* ctx)
+{
+    if (!ctx->split) return;
+    drop_graphs(ctx);
+    ctx->split = false;
+}
+
 static int relayout_step_inputs(php_ctx* ctx)
 {
-    int row = std::max(1, ctx->nsrc_active);
+    int row = ctx->probe_off + 1;
     for (auto& p : ctx->dft) {
         p.in_off = row;
         row += 1 + 2 * p.nfreq;
@@ -1793,10 +2336,10 @@ static int relayout_step_inputs(php_ctx* ctx)
 template <typename R>
 static void launch_gather_plane(php_ctx* ctx, int comp, int axis, int pos, bool f32)
 {
-    R* const* fp = reinterpret_cast<R* const*>(ctx->f);
-    Fields<R> f{fp[0], fp[1], fp[2], fp[3], fp[4], fp[5], fp[6], fp[7], fp[8]};
-    if (f32) gather_plane<R, float><<<296, 256, 0, ctx->stream>>>(f, comp, axis, pos, ctx->nx, ctx->ny, ctx->nz, ctx->nxp, (float*)ctx->scratch);
-    else gather_plane<R, double><<<296, 256, 0, ctx->stream>>>(f, comp, axis, pos, ctx->nx, ctx->ny, ctx->nz, ctx->nxp, (double*)ctx->scratch);
+    const Fields<R> f = make_fields<R>(ctx);
+    const DView<R> dv = make_dview<R>(ctx);
+    if (f32) gather_plane<R, float><<<296, 256, 0, ctx->stream>>>(f, dv, comp, axis, pos, ctx->nx, ctx->ny, ctx->nz, ctx->nxp, (float*)ctx->scratch);
+    else gather_plane<R, double><<<296, 256, 0, ctx->stream>>>(f, dv, comp, axis, pos, ctx->nx, ctx->ny, ctx->nz, ctx->nxp, (double*)ctx->scratch);
 }
 
 /* Fills pinned buffer b with the per-step inputs (source values, DFT
@@ -1805,16 +2348,18 @@ static void launch_gather_plane(php_ctx* ctx, int comp, int axis, int pos, bool 
 static int stage_step_inputs(php_ctx* ctx, int n, int b)
 {
     const double dt = ctx->d.dt;
-    /* the copy out of this pinned buffer two chunks ago must be done; the
-     * chunk in between keeps the GPU busy meanwhile */
-    CK(cudaEventSynchronize(ctx->staged[b]));
-    double* h = ctx->step_in_host[b];
+    /* the last copy out of this page-locked slot must be done; the chunks in
+     * between keep the GPU busy meanwhile */
+    const int slots = 2 * kMaxChunk / ctx->max_chunk, slot = ctx->chunk_no % slots;
+    CK(cudaEventSynchronize(ctx->staged[slot]));
+    double* h = ctx->step_in_host[slot * 2 / slots] + (size_t)(slot % (slots / 2)) * ctx->max_chunk * ctx->step_row;
     for (int s = 0; s < n; s++) {
         const int t = ctx->t + s;
         double* row = h + (size_t)s * ctx->step_row;
         const double current_time = t * dt; /* fdtd.c:3117 */
         for (int q = 0; q < ctx->nsrc_active; q++)
             row[q] = source_value(&ctx->src[ctx->src_active_index[q]], current_time);
+        row[ctx->probe_off] = t - ctx->probe_t0;
         for (auto& p : ctx->dft) {
             const bool take = t >= p.first && ((t - p.first) % p.interval) == 0;
             row[p.in_off] = take ? 1.0 : 0.0;
@@ -1830,7 +2375,7 @@ static int stage_step_inputs(php_ctx* ctx, int n, int b)
      * which precedes this copy on the stream */
     CK(cudaMemcpyAsync(ctx->step_in_dev[b], h, (size_t)n * ctx->step_row * sizeof(double), cudaMemcpyHostToDevice,
                        ctx->stream));
-    CK(cudaEventRecord(ctx->staged[b], ctx->stream));
+    CK(cudaEventRecord(ctx->staged[slot], ctx->stream));
     return PHP_OK;
 }
 
@@ -1846,9 +2391,7 @@ static int64_t point_index(const php_ctx* ctx, const int32_t* p)
 template <typename R>
 static void launch_frame_gather(php_ctx* ctx, const DiagPartial* fin, int has_point, int64_t pc, int64_t cc)
 {
-    R* const* fp = reinterpret_cast<R* const*>(ctx->f);
-    Fields<R> f{fp[0], fp[1], fp[2], fp[3], fp[4], fp[5], fp[6], fp[7], fp[8]};
-    frame_gather<R><<<1, 256, 0, ctx->stream>>>(f, ctx->mat, ctx->slot, (const MatCoef<R>*)ctx->mc, (const R*)ctx->r,
+    frame_gather<R><<<1, 256, 0, ctx->stream>>>(make_fields<R>(ctx), make_dview<R>(ctx), ctx->mat, ctx->slot, (const MatCoef<R>*)ctx->mc, (const R*)ctx->r,
                                                  (const R*)ctx->v, ctx->rv_unit, ctx->nslot, ctx->nx, ctx->ny, ctx->nz, ctx->nxp,
                                                  ctx->n3max, fin, has_point, pc, cc,
                                                  ctx->probe ? ctx->probe_count : nullptr, ctx->err_flag,
@@ -1859,10 +2402,16 @@ extern "C" {
 
 int php_create(const php_desc* desc, php_ctx** out)
 {
+    return php_create_buffers(desc, true, out);
+}
+
+int php_create_buffers(const php_desc* desc, bool split, php_ctx** out)
+{
     if (!desc || !out) return fail(nullptr, PHP_ERR_INPUT, "null argument");
     *out = nullptr;
     php_ctx* ctx = new (std::nothrow) php_ctx();
     if (!ctx) return fail(nullptr, PHP_ERR_OOM, "host allocation failed");
+    ctx->allow_split = split;
     int rc = create_impl(desc, ctx);
     if (rc) {
         g_create_error = ctx->err;
@@ -1912,6 +2461,7 @@ int php_create_slab(const php_desc* desc, int32_t z0, int32_t nz_local, php_ctx*
 int php_halo_planes(php_ctx* ctx, int32_t which, void** ptrs, uint64_t* plane_bytes)
 {
     if (!ctx || !ptrs || which < 0 || which > 3) return PHP_ERR_INPUT;
+    step_in_place(ctx);
     /* E plane 0 | E halo above | H top plane | H halo below */
     const int64_t plane_idx[4] = {0, ctx->nz, ctx->nz - 1, -1};
     const int first[4] = {PHP_EX, PHP_EX, PHP_HX, PHP_HX};
@@ -1925,6 +2475,7 @@ int php_halo_planes(php_ctx* ctx, int32_t which, void** ptrs, uint64_t* plane_by
 int php_step_half(php_ctx* ctx, int32_t half)
 {
     if (!ctx || (half != 0 && half != 1)) return PHP_ERR_INPUT;
+    step_in_place(ctx);
     ctx->last_launches = 0;
     int launches = 0;
     const int b = ctx->chunk_no & 1;
@@ -1948,6 +2499,7 @@ int php_step_half(php_ctx* ctx, int32_t half)
 int php_step_part(php_ctx* ctx, int32_t part, void* stream)
 {
     if (!ctx || part < 0 || part > 4) return PHP_ERR_INPUT;
+    step_in_place(ctx);
     ctx->last_launches = 0;
     int launches = 0;
     const int b = ctx->chunk_no & 1;
@@ -2004,17 +2556,15 @@ int php_step(php_ctx* ctx, int32_t nsteps)
     if (nsteps < 0) return fail(ctx, PHP_ERR_INPUT, "negative step count");
     ctx->last_launches = 0;
     while (nsteps > 0) {
-        const int n = std::min(nsteps, kMaxChunk);
+        const int n = std::min(nsteps, ctx->max_chunk);
         const int b = ctx->chunk_no & 1;
-        /* the copy out of this pinned buffer two chunks ago must be done;
-         * the chunk in between keeps the GPU busy meanwhile */
         int rc = stage_step_inputs(ctx, n, b);
         if (rc) return rc;
         cudaGraphExec_t g;
         rc = ensure_graph(ctx, n, b, &g);
         if (rc) return rc;
         CK(cudaGraphLaunch(g, ctx->stream));
-        if (ctx->fused && (n & 1)) swap_levels(ctx); /* the level the graph leaves current */
+        if ((ctx->fused || ctx->split) && (n & 1)) swap_levels(ctx); /* the level the graph leaves current */
         ctx->chunk_no++;
         if (ctx->profile) {
             CK(cudaStreamSynchronize(ctx->stream));
@@ -2022,7 +2572,7 @@ int php_step(php_ctx* ctx, int32_t nsteps)
                 for (int kind = 0; kind < kProfKinds; kind++) {
                     if ((kind == 2 && (!ctx->probe || probe_folded(ctx))) || (kind == 3 && dft_launched(ctx) == 0) ||
                         (kind == 4 && !ctx->ion_split) ||
-                        (kind <= 1 && ctx->fused) || (kind == 5 && !ctx->fused))
+                        (kind <= 1 && ctx->fused) || (kind == 5 && !ctx->fused && !ctx->split))
                         continue;
                     float ms = 0.f;
                     CK(cudaEventElapsedTime(&ms, ctx->prof_ev[((size_t)s * kProfKinds + kind) * 2],
@@ -2031,7 +2581,7 @@ int php_step(php_ctx* ctx, int32_t nsteps)
                     ctx->prof_n[kind] += kind == 3 ? (int64_t)dft_launched(ctx) : 1;
                 }
         }
-        ctx->last_launches += n * ((ctx->fused ? 1 : 2) + (ctx->ion_split ? 1 : 0) + (ctx->probe && !probe_folded(ctx) ? 1 : 0) +
+        ctx->last_launches += n * ((ctx->fused ? 1 : ctx->split ? split_launches(ctx) : ctx->by_class ? 1 + split_launches(ctx) : 2) + (ctx->ion_split ? 1 : 0) + (ctx->probe && !probe_folded(ctx) ? 1 : 0) +
                                    dft_launched(ctx));
         ctx->t += n;
         nsteps -= n;
@@ -2044,13 +2594,13 @@ int php_prepare(php_ctx* ctx, int32_t nsteps)
     if (!ctx) return PHP_ERR_INPUT;
     if (nsteps < 0) return fail(ctx, PHP_ERR_INPUT, "negative step count");
     cudaGraphExec_t g;
-    /* with the one-launch step, a chunk of odd length leaves the other level
-     * current: the graphs of both levels */
+    /* double buffered, a chunk of odd length leaves the other level current:
+     * the graphs of both levels */
     int rc = PHP_OK;
-    for (int lv = 0; lv < (ctx->fused ? 2 : 1) && rc == PHP_OK; lv++) {
+    for (int lv = 0; lv < (ctx->fused || ctx->split ? 2 : 1) && rc == PHP_OK; lv++) {
         if (lv) swap_levels(ctx);
-        if (nsteps >= kMaxChunk) rc = ensure_graph(ctx, kMaxChunk, 0, &g);
-        if (rc == PHP_OK && nsteps % kMaxChunk) rc = ensure_graph(ctx, nsteps % kMaxChunk, 0, &g);
+        if (nsteps >= ctx->max_chunk) rc = ensure_graph(ctx, ctx->max_chunk, 0, &g);
+        if (rc == PHP_OK && nsteps % ctx->max_chunk) rc = ensure_graph(ctx, nsteps % ctx->max_chunk, 0, &g);
         if (lv) swap_levels(ctx);
     }
     return rc;
@@ -2136,9 +2686,9 @@ int php_read_volume(php_ctx* ctx, int32_t comp, double* out)
     void* dbuf = nullptr;
     CK(cudaMallocAsync(&dbuf, n * sizeof(double), ctx->stream));
     if (ctx->prec == PHP_PREC_FP32)
-        gather_volume<float><<<592, 256, 0, ctx->stream>>>((const float*)ctx->f[comp], ctx->nx, ctx->ny, ctx->nz, ctx->nxp, (double*)dbuf);
+        gather_volume<float><<<592, 256, 0, ctx->stream>>>(make_fields<float>(ctx), make_dview<float>(ctx), comp, ctx->nx, ctx->ny, ctx->nz, ctx->nxp, (double*)dbuf);
     else
-        gather_volume<double><<<592, 256, 0, ctx->stream>>>((const double*)ctx->f[comp], ctx->nx, ctx->ny, ctx->nz, ctx->nxp, (double*)dbuf);
+        gather_volume<double><<<592, 256, 0, ctx->stream>>>(make_fields<double>(ctx), make_dview<double>(ctx), comp, ctx->nx, ctx->ny, ctx->nz, ctx->nxp, (double*)dbuf);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(out, dbuf, n * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaFreeAsync(dbuf, ctx->stream));
@@ -2152,13 +2702,13 @@ int php_read_point(php_ctx* ctx, int32_t i, int32_t j, int32_t k, double* out9)
     if (i < 0 || i >= ctx->nx || j < 0 || j >= ctx->ny || k < -1 || k > ctx->nz)
         return fail(ctx, PHP_ERR_INPUT, "point (%d,%d,%d) outside the grid", i, j, k);
     const int64_t c = ((int64_t)k * ctx->ny + j) * ctx->nxp + i;
-    const size_t rs = rsize(ctx->prec);
-    char* stage = (char*)ctx->host_stage;
+    double* pt = (double*)ctx->scratch;
+    if (ctx->prec == PHP_PREC_FP32) point_gather<float><<<1, 32, 0, ctx->stream>>>(make_fields<float>(ctx), make_dview<float>(ctx), c, pt);
+    else point_gather<double><<<1, 32, 0, ctx->stream>>>(make_fields<double>(ctx), make_dview<double>(ctx), c, pt);
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(ctx->host_stage, pt, 9 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
-    for (int q = 0; q < 9; q++)
-        CK(cudaMemcpyAsync(stage + q * rs, (const char*)ctx->f[q] + c * (int64_t)rs, rs, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    for (int q = 0; q < 9; q++) out9[q] = rs == 4 ? (double)((float*)stage)[q] : ((double*)stage)[q];
+    memcpy(out9, ctx->host_stage, 9 * sizeof(double));
     return PHP_OK;
 }
 
@@ -2203,9 +2753,10 @@ int php_read_cell_state(php_ctx* ctx, int32_t i, int32_t j, int32_t k, int32_t* 
              * J = P - P_old (crystal frame) in the P_old pool */
             double dl[3];
             for (int q = 0; q < 3; q++) {
-                float dv = 0.f;
-                CK(cudaMemcpy(&dv, (const float*)ctx->f[3 + q] + c, sizeof(float), cudaMemcpyDeviceToHost));
-                dl[q] = (double)dv - pq[q];
+                double dv = 0.0;
+                int rc = fetch(ctx->Dp, q, &dv);
+                if (rc) return rc;
+                dl[q] = dv - pq[q];
             }
             const int fl = ctx->mat_flags[mid];
             const double cs = ctx->mat_cs[mid], sn = ctx->mat_sn[mid];
@@ -2242,15 +2793,11 @@ static int enqueue_diag(php_ctx* ctx, DiagPartial** fin_out)
     DiagPartial* fin = part + blocks;
     *fin_out = fin;
     if (ctx->prec == PHP_PREC_FP32) {
-        float* const* fp = reinterpret_cast<float* const*>(ctx->f);
-        Fields<float> f{fp[0], fp[1], fp[2], fp[3], fp[4], fp[5], fp[6], fp[7], fp[8]};
-        diag_pass1<float><<<blocks, 256, 0, ctx->stream>>>(f, ctx->nx, ctx->ny, ctx->nz, ctx->nxp, (const float*)ctx->r,
+        diag_pass1<float><<<blocks, 256, 0, ctx->stream>>>(make_fields<float>(ctx), ctx->nx, ctx->ny, ctx->nz, ctx->nxp, (const float*)ctx->r,
                                                            ctx->rv_unit, ctx->any_atoms ? ctx->nslot : 0, ctx->slot_cell, ctx->slot_n3,
                                                            std::max(ctx->n3max, 1), part);
     } else {
-        double* const* fp = reinterpret_cast<double* const*>(ctx->f);
-        Fields<double> f{fp[0], fp[1], fp[2], fp[3], fp[4], fp[5], fp[6], fp[7], fp[8]};
-        diag_pass1<double><<<blocks, 256, 0, ctx->stream>>>(f, ctx->nx, ctx->ny, ctx->nz, ctx->nxp, (const double*)ctx->r,
+        diag_pass1<double><<<blocks, 256, 0, ctx->stream>>>(make_fields<double>(ctx), ctx->nx, ctx->ny, ctx->nz, ctx->nxp, (const double*)ctx->r,
                                                             ctx->rv_unit, ctx->any_atoms ? ctx->nslot : 0, ctx->slot_cell, ctx->slot_n3,
                                                             std::max(ctx->n3max, 1), part);
     }
@@ -2309,6 +2856,17 @@ int php_probe_set(php_ctx* ctx, int32_t i, int32_t j, int32_t k_field, int32_t k
     int32_t s = -1;
     if (ctx->slot) CK(cudaMemcpy(&s, ctx->slot + ca, sizeof(int32_t), cudaMemcpyDeviceToHost));
     ctx->probe_slot = s;
+    DCell& pd = ctx->probe_d;
+    pd.slot = -1;
+    for (double& m : pd.dm) m = 0.0;
+    if (k_field >= 0 && k_field < ctx->nz) {
+        if (ctx->slot) CK(cudaMemcpy(&pd.slot, ctx->slot + ctx->probe_cf, sizeof(int32_t), cudaMemcpyDeviceToHost));
+        if (ctx->dmat) {
+            uint8_t fm = 0;
+            CK(cudaMemcpy(&fm, ctx->mat + ctx->probe_cf, 1, cudaMemcpyDeviceToHost));
+            CK(cudaMemcpy(pd.dm, ctx->dmat + 9 * (int)fm, sizeof(pd.dm), cudaMemcpyDeviceToHost));
+        }
+    }
     if (ctx->probe_n3 == 0) ctx->probe_slot = 0;
     if (!ctx->probe_rows) {
         int rc = dalloc(ctx, (void**)&ctx->probe_rows, (size_t)kProbeCap * (9 + 2 * std::max(ctx->n3max, 1)) * sizeof(double));
@@ -2530,10 +3088,18 @@ int php_memory_bytes(const php_ctx* ctx, uint64_t* bytes)
     return PHP_OK;
 }
 
+int php_estimate_buffers(const php_desc* desc, uint64_t* bytes, uint64_t* more)
+{
+    return estimate_bytes(*desc, bytes, more);
+}
+
 int php_estimate_bytes(const php_desc* desc, uint64_t* bytes)
 {
     if (!desc || !bytes) return PHP_ERR_INPUT;
-    return estimate_bytes(*desc, bytes);
+    uint64_t more = 0;
+    const int rc = estimate_bytes(*desc, bytes, &more);
+    if (rc == PHP_OK) *bytes += more;
+    return rc;
 }
 
 int php_last_launch_count(const php_ctx* ctx, int32_t* launches)

@@ -15,6 +15,15 @@
  *   psi y-slab    [nz][2L][nxp]
  *   psi z-slab    [2L][ny][nxp]
  *   pools         SoA: P[3][nslot], Po[3][nslot], r[3*natom_max][nslot], v[...]
+ *   D             strict mode: field arrays like E and H.  Fast modes: only
+ *                 where E is not a fixed linear map of D (ADE and atom
+ *                 cells): Dp[3][nslot] beside the other state of those
+ *                 cells.  Every other cell keeps E alone and advances it by
+ *                 M (D^{n+1} - D^n), M the material's 3 x 3 map from D to E
+ *                 (e_only_add): a step then neither reads nor writes D
+ *                 there, 6 of the 21 field words per cell of the two sweeps
+ *                 (256^3 tip workload: see php_sweeps_tma.cuh).  Read-outs
+ *                 of D form M^-1 E (d_at).
  *
  * Arithmetic modes:
  *   Strict (double): every operation of the reference in its order, with
@@ -42,7 +51,7 @@ constexpr int kBlockY = 8;
  * fields not used by a mode are zero. */
 template <typename R>
 struct MatCoef {
-    int32_t flags;     /* kLossy | kAde | kRotZ | kRotX | kAtoms */
+    int32_t flags;     /* kLossy | kAde | kRotZ | kRotX | kAtoms | kIso | kEOnly */
     int32_t natom;
     int32_t ion_off;   /* offset of QeZV (9N), QeZM (9N), DMM (9N^2) in ion_coef */
     int32_t pad;
@@ -55,22 +64,21 @@ struct MatCoef {
     R wp2[9];          /* strict: wp2; fast: eps0 dt^2 wp2 */
     R ade_scale;       /* fast: (1-lt)/(eps0*EPS_INF) */
     R pad2;
+    R em[9];           /* fast: E = em D in the lab frame (rotations folded in) */
 };
 
 /* kIso (fast modes only): no rotation, loss, ADE or atoms and eps^-1 a
- * multiple of the identity, so E = eps_inv[0] * D. */
-enum : int32_t { kLossy = 1, kAde = 2, kRotZ = 4, kRotX = 8, kAtoms = 16, kIso = 32 };
-
-/* materials the fused sweep keeps in shared memory (ids above read global) */
-constexpr int kSmemMats = 16;
+ * multiple of the identity, so E = eps_inv[0] * D.
+ * kEOnly (fast modes only): no ADE or atoms, and em is well conditioned, so
+ * the cell keeps E alone (kIso implies it); the other cells have a pool slot. */
+enum : int32_t { kLossy = 1, kAde = 2, kRotZ = 4, kRotX = 8, kAtoms = 16, kIso = 32, kEOnly = 64 };
 
 /* Per-axis CPML tables, indexed by the cell index along the axis.  slot < 0
- * outside the PML.  Strict uses kappa, b, c (fdtd.c:3146-3151 evaluated on
+ * outside the PML (pml_slot).  Strict uses kappa, b, c (fdtd.c:3146-3151 evaluated on
  * the host); fast uses kh = dt/(mu0 d kappa), kd = dt/(d kappa),
  * ch = dt c/(mu0 d), cd = dt c/d. */
 template <typename R>
 struct AxisTab {
-    const int32_t* slot;
     const R* kappa;
     const R* b;
     const R* c;
@@ -83,6 +91,17 @@ struct AxisTab {
 template <typename R>
 struct Fields {
     R *ex, *ey, *ez, *dx, *dy, *dz, *hx, *hy, *hz;
+};
+
+/* Where D is in the fast modes (Fields::dx is null): the pool of the cells
+ * with a slot, M^-1 E (dm, 9 doubles per material) in the others. */
+template <typename R>
+struct DView {
+    const R* dp;
+    const uint8_t* mat;
+    const int32_t* slot;       /* null: no cell has one */
+    const double* dm;
+    int64_t nslot, ncell;
 };
 
 template <typename R>
@@ -119,10 +138,13 @@ struct StepArgs {
     const MatCoef<R>* mc;
     const R* ion_coef;
     R *P, *Po, *r, *v;         /* pools */
+    R* Dp;                     /* D of the cells with a slot [3][nslot] (fast modes) */
+    uint32_t* Dc;              /* FP32 without ADE: what Dp's sums rounded off (pool_add) [nslot], else null */
+    DView<R> dv;
     const R* pr;               /* QeZV . r [3][nslot] when the ion pass runs apart (php_ions.cuh), else null */
     int32_t ion_k_off;         /* ion_coef offset of the material copied in ion_k, -1 for none */
     R ion_k[kIonK];
-    /* E = iso[id] * D for the plain isotropic materials (kIso) among the
+    /* dE = iso[id] * dD for the plain isotropic materials (kIso) among the
      * first kIsoMats ids, 0 for the others: the fused sweep's common case
      * without a load of the material record */
     R iso[kIsoMats];
@@ -139,14 +161,19 @@ struct StepArgs {
     /* the material record of one lossy or anisotropic material without ADE
      * or ions (the one filling most blocks): blocks of that material alone
      * (kPlainTensor) read it as constant-bank operands */
-    R tns_inv[9], tns_im[9], tns_cs, tns_sn;
+    R tns_em[9], tns_im[9];
     int32_t tns_flags;
     /* the material record of the few-atom material whose ion coefficients
      * are in ion_k, for blocks of that material alone (kPlainAtoms) */
     MatCoef<R> amc;
+    /* the record of the ADE material (without atoms) filling the most cells,
+     * -1 for none: the general path reads some 30 of its values per cell as
+     * constant-bank operands instead of loads */
+    MatCoef<R> dmc;
+    int32_t dmc_id;
     int64_t nslot;
-    int32_t nmat;
     int32_t nx, ny, nz, nxp, L, zchunk;
+    int32_t z_off, nzg;        /* global index of plane 0 and plane count (z slabs) */
     int32_t zc0;                /* first z chunk of the launch (blockIdx.z + zc0 is the chunk) */
     int64_t plane;             /* nxp * ny */
     /* strict scalars */
@@ -156,18 +183,29 @@ struct StepArgs {
     int64_t src_cell[kMaxSources];
     int32_t src_comp[kMaxSources];
     const double* src_val;     /* nsrc values of this step */
+    /* FP32: E of the source cells that keep E alone, summed in double [nsrc][3].
+     * A point source's own cell holds some 1e4 times the field of the
+     * radiation zone, so the rounding of its sum is the largest error there. */
+    double* src_acc;
     int32_t* err;              /* set to 1 by a block whose bounded wait gave up */
     int32_t stall_test;        /* failure-path test: the first H sweep block's wait gives up */
-    /* the one-launch step (he_sweep_tma): f's E and H and psi's H arrays hold
-     * the old time level, read only during the launch; the new E, H and H
-     * CPML state go to these buffers (D, the D CPML state and the pools are
-     * updated in place) */
+    /* where the sweeps write the new E, H and H CPML state.  The two sweeps of
+     * a domain in place: the arrays of f and psi.  Double buffered (the
+     * one-launch step, and the interior / rest split): f's E and H hold the
+     * old time level, read only during the step (the one-launch step's H CPML
+     * state likewise).  The D CPML state and the pools are updated in place. */
     R *enew[3], *hnew[3];
     R* psin_h[6];              /* hxy hxz hyx hyz hzx hzy */
-    /* per block of he_sweep_tma: 1 when the H part needs no CPML term and
-     * updates every cell, over the tile, the cells one below it in x and y
-     * and the plane below the z chunk */
-    const uint8_t* plain_hf;
+    /* blocks of a launch over part of the domain (blockIdx.x indexes it):
+     * x = tile x | tile y << 16, y .. z the planes [k0, k1), w the class (H
+     * sweep: 1 for a plain block; fused sweep: its plain-block code);
+     * nullptr: the whole grid in z chunks */
+    const int4* list;
+    /* he_sweep_tma: planes per block, and per plane and tile (of its own
+     * height) the class of the fused sweep's plain blocks, plus kHPlain
+     * [nz][tiles y][tiles x] */
+    int32_t zstep;
+    const uint16_t* pcls;
     /* running DFT planes of E or D components that the E sweep samples
      * after its z march (dft_fold), instead of a dft_sample launch: plane,
      * component (0-5), frequencies, the float32 cast flag, the offset of the
@@ -176,18 +214,28 @@ struct StepArgs {
     int32_t ndft;
     int32_t dft_z[kDftFold], dft_comp[kDftFold], dft_nfreq[kDftFold], dft_cast[kDftFold], dft_off[kDftFold];
     double* dft_acc[kDftFold];
-    /* the monitor row the E sweep records after its z march (probe_fold),
-     * instead of a probe_record_counted launch, when the field cell (i, j,
-     * kf) and the atom cell of slot (its r and v updated by the sweep) lie in
-     * one z chunk; probe_rows null: no such row */
+    /* the monitor row the sweeps record after their z march (probe_fold),
+     * instead of a probe_record_counted launch: its index is the value at
+     * probe_off of the step's input row (src_val), the fields are those of
+     * (i, j, kf), r and v those of slot, the cell (i, j, ka); probe_rows null:
+     * no such row */
     double* probe_rows;
     int32_t* probe_count;      /* [rows written, overflow flag] */
-    int32_t probe_i, probe_j, probe_kf, probe_n3, probe_cap;
+    int32_t probe_i, probe_j, probe_kf, probe_ka, probe_n3, probe_cap, probe_off;
     int64_t probe_slot;
     double rv_unit;            /* physical r, v per stored unit */
 };
 
 /* ------------------------------------------------------------ arithmetic */
+
+/* The fast modes' updates are written with explicit fused multiply-adds, so
+ * that every kernel and block path that contains them rounds alike (slabs,
+ * the one-launch step and the two sweeps give the same fields, bit for bit). */
+__device__ __forceinline__ double fma_(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float fma_(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+/* ka a - kb b: one component of a scaled curl */
+template <typename R>
+__device__ __forceinline__ R curl2(R ka, R a, R kb, R b) { return fma_(ka, a, -(kb * b)); }
 
 struct SOp {
     static __device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, b); }
@@ -222,13 +270,53 @@ __device__ __forceinline__ int32_t ldg_nh(const int32_t* p)
     return v;
 }
 
+/* CPML slot of cell i of an axis of n cells: i at the low side, L + n - 1 - i
+ * at the high one, -1 between */
+__host__ __device__ __forceinline__ int pml_slot(int i, int n, int L)
+{
+    return i < L ? i : i >= n - L ? L + n - 1 - i : -1;
+}
+
 /* ========================================================== small kernels */
+
+/* one row of M^-1 E, rounded as a stored D would be */
+template <typename R>
+__device__ __forceinline__ double d_of_e(const double* m, R ex, R ey, R ez)
+{
+    return (double)(R)__fma_rn(m[0], (double)ex, __fma_rn(m[1], (double)ey, m[2] * (double)ez));
+}
+
+/* D component q of device cell c, halo planes included (zero) */
+template <typename R>
+__device__ __forceinline__ double d_at(const Fields<R>& f, const DView<R>& v, int q, int64_t c)
+{
+    if (f.dx) return (double)(q == 0 ? f.dx : q == 1 ? f.dy : f.dz)[c];
+    if (c < 0 || c >= v.ncell) return 0.0;
+    const int32_t s = v.slot ? v.slot[c] : -1;
+    if (s >= 0) return (double)v.dp[(int64_t)q * v.nslot + s];
+    return d_of_e<R>(v.dm + 9 * (int)v.mat[c] + 3 * q, f.ex[c], f.ey[c], f.ez[c]);
+}
+
+/* field component comp (0-8) of device cell c */
+template <typename R>
+__device__ __forceinline__ double field_at(const Fields<R>& f, const DView<R>& v, int comp, int64_t c)
+{
+    switch (comp) {
+    case 0: return (double)f.ex[c];
+    case 1: return (double)f.ey[c];
+    case 2: return (double)f.ez[c];
+    case 6: return (double)f.hx[c];
+    case 7: return (double)f.hy[c];
+    case 8: return (double)f.hz[c];
+    default: return d_at(f, v, comp - 3, c);
+    }
+}
 
 /* Gathers one plane of a component into out (float or double).
  * axis 0: z plane kk -> [i][j]; axis 1: x plane -> [j][k]; axis 2: y plane
  * -> [i][k].  comp 9 is |E|. */
 template <typename R, typename O>
-__global__ void gather_plane(const Fields<R> f, int comp, int axis, int pos, int nx, int ny, int nz,
+__global__ void gather_plane(const Fields<R> f, const DView<R> dv, int comp, int axis, int pos, int nx, int ny, int nz,
                              int nxp, O* out)
 {
     int A, B;
@@ -244,43 +332,47 @@ __global__ void gather_plane(const Fields<R> f, int comp, int axis, int pos, int
         else { i = u; j = pos; k = w; }
         const int64_t c = ((int64_t)k * ny + j) * nxp + i;
         double val;
-        switch (comp) {
-        case 0: val = (double)f.ex[c]; break;
-        case 1: val = (double)f.ey[c]; break;
-        case 2: val = (double)f.ez[c]; break;
-        case 3: val = (double)f.dx[c]; break;
-        case 4: val = (double)f.dy[c]; break;
-        case 5: val = (double)f.dz[c]; break;
-        case 6: val = (double)f.hx[c]; break;
-        case 7: val = (double)f.hy[c]; break;
-        case 8: val = (double)f.hz[c]; break;
-        default: {
+        if (comp < 9) {
+            val = field_at(f, dv, comp, c);
+        } else {
             const double x = (double)f.ex[c], y = (double)f.ey[c], z = (double)f.ez[c];
             val = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y)), __dmul_rn(z, z)));
-        }
         }
         out[t] = (O)val;
     }
 }
 
+/* The nine field values of one cell. */
+template <typename R>
+__global__ void point_gather(const Fields<R> f, const DView<R> dv, int64_t c, double* out9)
+{
+    if (threadIdx.x < 9) out9[threadIdx.x] = field_at(f, dv, threadIdx.x, c);
+}
+
 /* Whole component to file order [i][j][k]. */
 template <typename R>
-__global__ void gather_volume(const R* src, int nx, int ny, int nz, int nxp, double* out)
+__global__ void gather_volume(const Fields<R> f, const DView<R> dv, int comp, int nx, int ny, int nz, int nxp, double* out)
 {
     const int64_t n = (int64_t)nx * ny * nz;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x) {
         const int k = (int)(t % nz);
         const int64_t ij = t / nz;
         const int j = (int)(ij % ny), i = (int)(ij / ny);
-        out[t] = (double)src[((int64_t)k * ny + j) * nxp + i];
+        out[t] = field_at(f, dv, comp, ((int64_t)k * ny + j) * nxp + i);
     }
 }
+
+/* Where D of one cell is: its pool slot, else M^-1 (fast modes) */
+struct DCell {
+    int32_t slot;
+    double dm[9];
+};
 
 /* Probe row appended at count[0]: 9 fields at cf, then r and v of pool slot
  * (3*natom each, times rv_unit: the stored state is scaled in FP32).
  * count[1] is raised instead of writing past cap. */
 template <typename R>
-__global__ void probe_record_counted(const Fields<R> f, int64_t cf, const R* r, const R* v, double rv_unit,
+__global__ void probe_record_counted(const Fields<R> f, const R* dp, const DCell dc, int64_t cf, const R* r, const R* v, double rv_unit,
                                      int64_t nslot, int64_t slot, int n3, double* rows, int32_t* count, int cap,
                                      int row_len)
 {
@@ -294,8 +386,14 @@ __global__ void probe_record_counted(const Fields<R> f, int64_t cf, const R* r, 
     double* out = rows + (int64_t)row * row_len;
     const int t = threadIdx.x;
     if (t < 9) {
-        const R* p[9] = {f.ex, f.ey, f.ez, f.dx, f.dy, f.dz, f.hx, f.hy, f.hz};
-        out[t] = (double)p[t][cf];
+        if (t < 3 || t > 5) {
+            out[t] = (double)(t == 0 ? f.ex : t == 1 ? f.ey : t == 2 ? f.ez : t == 6 ? f.hx : t == 7 ? f.hy : f.hz)[cf];
+        } else if (f.dx) {
+            out[t] = (double)(t == 3 ? f.dx : t == 4 ? f.dy : f.dz)[cf];
+        } else {
+            const double* m = dc.dm + 3 * (t - 3);
+            out[t] = dc.slot >= 0 ? (double)dp[(int64_t)(t - 3) * nslot + dc.slot] : d_of_e<R>(m, f.ex[cf], f.ey[cf], f.ez[cf]);
+        }
     } else if (t < 9 + 2 * n3) {
         const int q = t - 9;
         out[t] = rv_unit * ((q < n3) ? (double)r[(int64_t)q * nslot + slot] : (double)v[(int64_t)(q - n3) * nslot + slot]);
@@ -319,7 +417,7 @@ __device__ __forceinline__ void dft_accumulate(double x, const double* ph, int n
 
 /* Running DFT sample of one plane; skipped when flag == 0. */
 template <typename R>
-__global__ void dft_sample(const R* src, int64_t plane_off, int nx, int ny, int nxp, int nfreq,
+__global__ void dft_sample(const Fields<R> fld, const DView<R> dv, int comp, int64_t plane_off, int nx, int ny, int nxp, int nfreq,
                            int cast_f32, const double* step_in, int flag_off, int phasor_off,
                            double* acc)
 {
@@ -328,7 +426,7 @@ __global__ void dft_sample(const R* src, int64_t plane_off, int nx, int ny, int 
     const double* ph = step_in + phasor_off;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x) {
         const int j = (int)(t / nx), i = (int)(t % nx);
-        double x = (double)src[plane_off + (int64_t)j * nxp + i];
+        double x = field_at(fld, dv, comp, plane_off + (int64_t)j * nxp + i);
         if (cast_f32) x = (double)(float)x;
         dft_accumulate(x, ph, nfreq, acc, n, t);
     }
@@ -348,45 +446,56 @@ __device__ __forceinline__ void dft_fold(const StepArgs<R>& a, R* const* e3, int
         const int k = a.dft_z[q];
         if (k < k0 || k >= k1 || a.src_val[a.dft_off[q]] == 0.0) continue;
         const int cp = a.dft_comp[q];
-        const R* src = cp == 0 ? e3[0] : cp == 1 ? e3[1] : cp == 2 ? e3[2] : cp == 3 ? a.f.dx : cp == 4 ? a.f.dy : a.f.dz;
-        double x = (double)src[(k * a.ny + j) * a.nxp + i];
+        const int c = (k * a.ny + j) * a.nxp + i;
+        double x;
+        if (cp < 3) {
+            x = (double)(cp == 0 ? e3[0] : cp == 1 ? e3[1] : e3[2])[c];
+        } else {
+            Fields<R> f = a.f;
+            f.ex = e3[0];
+            f.ey = e3[1];
+            f.ez = e3[2];
+            x = d_at(f, a.dv, cp - 3, c);
+        }
         if (a.dft_cast[q]) x = (double)(float)x;
         dft_accumulate(x, a.src_val + a.dft_off[q] + 1, a.dft_nfreq[q], a.dft_acc[q], (int64_t)a.nx * a.ny,
                        (int64_t)j * a.nx + i);
     }
 }
 
-/* The monitor row of probe_record_counted taken by the E sweep
- * (StepArgs::probe_*): the thread of column (i, j), after its z march over
- * planes k0 .. k1-1 that hold the field cell, reads back the E and D it
- * stored there, H (e3, h3: the arrays the step's sweeps wrote), and the r
- * and v it stored for the atom cell of the same column and chunk.  It is the
- * one thread of the launch that touches the row counter. */
+/* The monitor row of probe_record_counted taken by the sweeps
+ * (StepArgs::probe_*): after its z march over planes k0 .. k1-1, the thread of
+ * column (i, j) reads back the E, D and H of the field cell (e3, h3: the arrays
+ * the step's launches wrote), and the one whose planes hold the atom cell its r
+ * and v. */
 template <typename R>
 __device__ __forceinline__ void probe_fold(const StepArgs<R>& a, R* const* e3, R* const* h3, int i, int j, int k0, int k1)
 {
-    if (!a.probe_rows || i != a.probe_i || j != a.probe_j || a.probe_kf < k0 || a.probe_kf >= k1) return;
-    const int row = a.probe_count[0];
+    if (i != a.probe_i || j != a.probe_j) return;
+    const bool fields = a.probe_kf >= k0 && a.probe_kf < k1, atoms = a.probe_n3 && a.probe_ka >= k0 && a.probe_ka < k1;
+    if (!fields && !atoms) return;
+    const int row = (int)a.src_val[a.probe_off];
     if (row >= a.probe_cap) {
-        a.probe_count[1] = 1;
+        if (fields) a.probe_count[1] = 1;
         return;
     }
-    const int64_t c = ((int64_t)a.probe_kf * a.ny + j) * a.nxp + i;
     double* out = a.probe_rows + (int64_t)row * (9 + 2 * a.probe_n3);
-    out[0] = (double)e3[0][c];
-    out[1] = (double)e3[1][c];
-    out[2] = (double)e3[2][c];
-    out[3] = (double)a.f.dx[c];
-    out[4] = (double)a.f.dy[c];
-    out[5] = (double)a.f.dz[c];
-    out[6] = (double)h3[0][c];
-    out[7] = (double)h3[1][c];
-    out[8] = (double)h3[2][c];
-    for (int q = 0; q < a.probe_n3; ++q) {
+    if (fields) {
+        const int64_t c = ((int64_t)a.probe_kf * a.ny + j) * a.nxp + i;
+        Fields<R> f = a.f;
+        f.ex = e3[0];
+        f.ey = e3[1];
+        f.ez = e3[2];
+        f.hx = h3[0];
+        f.hy = h3[1];
+        f.hz = h3[2];
+        for (int q = 0; q < 9; ++q) out[q] = field_at(f, a.dv, q, c);
+        a.probe_count[0] = row + 1;
+    }
+    for (int q = 0; atoms && q < a.probe_n3; ++q) {
         out[9 + q] = a.rv_unit * (double)a.r[(int64_t)q * a.nslot + a.probe_slot];
         out[9 + a.probe_n3 + q] = a.rv_unit * (double)a.v[(int64_t)q * a.nslot + a.probe_slot];
     }
-    a.probe_count[0] = row + 1;
 }
 
 /* ------------------------------------------------------------ diagnostics */
@@ -490,15 +599,14 @@ struct FrameHead {
 /* Field values (Ex Ey Ez Dx Dy Dz Hx Hy Hz) at device cell c, and r, v of the
  * atom cell c (none when its material has no atoms). */
 template <typename R>
-__device__ __forceinline__ void frame_cell(const Fields<R>& f, const uint8_t* mat, const int32_t* slot,
+__device__ __forceinline__ void frame_cell(const Fields<R>& f, const DView<R>& dv, const uint8_t* mat, const int32_t* slot,
                                            const MatCoef<R>* mc, const R* r, const R* v, double rv_unit,
                                            int64_t nslot, int64_t cf, int64_t ca, double* point9, double* rr,
                                            double* vv, int32_t* natom)
 {
     const int t = threadIdx.x;
     if (point9 && t < 9) {
-        const R* p[9] = {f.ex, f.ey, f.ez, f.dx, f.dy, f.dz, f.hx, f.hy, f.hz};
-        point9[t] = (double)p[t][cf];
+        point9[t] = field_at(f, dv, t, cf);
     }
     if (ca < 0) return;
     const int na = mc[mat[ca]].natom;
@@ -516,7 +624,7 @@ __device__ __forceinline__ void frame_cell(const Fields<R>& f, const uint8_t* ma
  * none) and the cell's (-1: none); probe_count: the probe row counter
  * (nullptr: no probe).  Thread 0 writes every natom field. */
 template <typename R>
-__global__ void frame_gather(const Fields<R> f, const uint8_t* mat, const int32_t* slot, const MatCoef<R>* mc,
+__global__ void frame_gather(const Fields<R> f, const DView<R> dv, const uint8_t* mat, const int32_t* slot, const MatCoef<R>* mc,
                              const R* r, const R* v, double rv_unit, int64_t nslot, int nx, int ny, int nz, int nxp,
                              int n3max,
                              const DiagPartial* fin, int has_point, int64_t point_c, int64_t cell_c,
@@ -539,15 +647,15 @@ __global__ void frame_gather(const Fields<R> f, const uint8_t* mat, const int32_
             const int j = (int)(cell % ny);
             const int i = (int)(cell / ny);
             const int64_t c = ((int64_t)k * ny + j) * nxp + i;
-            frame_cell(f, mat, slot, mc, r, v, rv_unit, nslot, c, c, head->diag_point, head->diag_r, head->diag_v,
+            frame_cell(f, dv, mat, slot, mc, r, v, rv_unit, nslot, c, c, head->diag_point, head->diag_r, head->diag_v,
                        &head->diag_natom);
         }
     }
     if (has_point)
-        frame_cell<R>(f, mat, slot, mc, r, v, rv_unit, nslot, point_c, -1, head->point, nullptr, nullptr, nullptr);
+        frame_cell<R>(f, dv, mat, slot, mc, r, v, rv_unit, nslot, point_c, -1, head->point, nullptr, nullptr, nullptr);
     if (cell_c >= 0) {
         if (t == 0) head->cell_natom = 0;
-        frame_cell<R>(f, mat, slot, mc, r, v, rv_unit, nslot, cell_c, cell_c, nullptr, head->cell_r, head->cell_v,
+        frame_cell<R>(f, dv, mat, slot, mc, r, v, rv_unit, nslot, cell_c, cell_c, nullptr, head->cell_r, head->cell_v,
                       &head->cell_natom);
     }
     if (t == 0) {

@@ -30,6 +30,7 @@
 #include <vector>
 
 #include "php_fdtd.h"
+#include "php_internal.h"
 #include "php_serve.h"
 
 namespace {
@@ -52,7 +53,9 @@ struct Job {
     php_dft_request dft{};
     std::vector<double> freqs;
 
-    uint64_t bytes = 0;
+    uint64_t bytes = 0;           /* device bytes charged to the budget */
+    uint64_t more = 0;            /* what second field buffers would add */
+    bool split = false;           /* they fit when the job was admitted */
     php_ctx* ctx = nullptr;
     cudaStream_t stream = nullptr;
     int dft_id = -1;
@@ -111,7 +114,7 @@ bool build_job(php_server* s, Job* j)
      * chunks (fewer halo re-reads) instead of splitting its z range until its
      * own blocks fill the GPU */
     if (j->desc.z_chunk <= 0) j->desc.z_chunk = 8;
-    int rc = php_create(&j->desc, &j->ctx);
+    int rc = php_create_buffers(&j->desc, j->split, &j->ctx);
     if (rc) {
         set_error(j, rc, php_last_error(nullptr));
         return false;
@@ -183,6 +186,11 @@ void admission_loop(php_server* s)
         Job* j = s->queued.front();
         s->queued.pop_front();
         s->active++;
+        if (j->more && s->used + j->bytes + j->more <= s->d.memory_budget) {
+            j->split = true;
+            j->bytes += j->more;
+            j->info.device_bytes = j->bytes;
+        }
         s->used += j->bytes;
         s->peak_bytes = std::max(s->peak_bytes, s->used);
         j->info.t_admit = now_since(s->t0);
@@ -424,7 +432,7 @@ int php_batch_submit(php_server* s, const php_desc* desc, int32_t nsteps, const 
         }
     }
     uint64_t est = 0;
-    if (!rc) rc = php_estimate_bytes(&j->desc, &est);
+    if (!rc) rc = php_estimate_buffers(&j->desc, &est, &j->more);
     if (rc) {
         std::lock_guard<std::mutex> g(s->mu);
         s->err = "php_batch_submit: invalid description";

@@ -3,7 +3,9 @@
  * the TMA plane-ring sweeps of php_sweeps_tma.cuh and the one-launch step of
  * php_sweep_fused.cuh:
  *
+ *   h_update        H += dt (curl E / kappa + psi_H)          fdtd.c:3123-3231
  *   d_update        D += dt (curl H / kappa + psi_D) - eps''  fdtd.c:3238-3356
+ *   e_only_add      E += M dD of the cells that keep E alone  fdtd.c:3404-3461
  *   e_cell_values   D -> E (rotation, eps^-1 or ADE, loss)    fdtd.c:3404-3503
  *   e_update        tensor ADE and the ion equations of motion fdtd.c:3463-3528
  *
@@ -71,6 +73,45 @@ __device__ __forceinline__ void rot_back(int flags, R cs, R sn, R& u0, R& u1, R&
     }
 }
 
+/* A block's CPML coefficients in shared memory: three per cell of the tile
+ * along x (32), then along y (ROWS): kd, b, cd of the D update, kh, b, ch of
+ * the H update, kappa, b, c in the strict mode.  Read from global memory once
+ * per block; the per-plane loads of them (through an L1 that the stage ring
+ * leaves little of) were a chain of cache misses in every plane. */
+template <typename R, bool STRICT, bool H>
+__device__ __forceinline__ void pml_table(const StepArgs<R>& a, R* tab, int i0, int j0, int rows, int tid)
+{
+    if (tid < 32 + rows) {
+        const bool x = tid < 32;
+        const AxisTab<R>& t = x ? a.tx : a.ty;
+        const int q = x ? min(i0 + tid, a.nx - 1) : min(j0 + tid - 32, a.ny - 1);
+        tab[3 * tid] = STRICT ? t.kappa[q] : H ? t.kh[q] : t.kd[q];
+        tab[3 * tid + 1] = t.b[q];
+        tab[3 * tid + 2] = STRICT ? t.c[q] : H ? t.ch[q] : t.cd[q];
+    }
+}
+__host__ __device__ constexpr int pml_table_len(int rows) { return 3 * (32 + rows); }
+
+/* the same three of plane k along z (uniform over the block), read where the
+ * plane lies in the CPML; elsewhere kappa = 1, b and c are not used */
+template <typename R>
+struct ZCoef {
+    R k, b, c;
+};
+template <typename R, bool STRICT, bool H>
+__device__ __forceinline__ ZCoef<R> z_coef(const StepArgs<R>& a, int sz, int k)
+{
+    ZCoef<R> z{STRICT ? R(1) : H ? a.khp[2] : a.kdp[2], R(0), R(0)};
+    if (sz >= 0) {
+        z.k = ldg_nh((STRICT ? a.tz.kappa : H ? a.tz.kh : a.tz.kd) + k);
+        z.b = ldg_nh(a.tz.b + k);
+        z.c = ldg_nh((STRICT ? a.tz.c : H ? a.tz.ch : a.tz.cd) + k);
+    }
+    return z;
+}
+template <typename R>
+__device__ __forceinline__ int z_slot(const StepArgs<R>& a, int k) { return pml_slot(k + a.z_off, a.nzg, a.L); }
+
 /* CPML state of one cell read before its update: the z slot of the plane
  * and the old psi values of every PML axis the cell lies in (zero
  * elsewhere).  Loading them apart from the update lets a kernel issue these
@@ -79,19 +120,18 @@ template <typename R>
 struct CellPsi {
     int sz;
     R xy, xz, yx, yz, zx, zy;
-    R kdz;                     /* dt / (dz kappa_z), FP32/FP64 fast paths */
+    ZCoef<R> z;
 };
 
 /* psi_D of fdtd.c:3258-3334 (the reads) */
-template <typename R>
-__device__ __forceinline__ void load_psi_d(const StepArgs<R>& a, int i, int j, int k, int sx, int sy, CellPsi<R>& ps)
+template <typename R, bool STRICT = false>
+__device__ __forceinline__ void load_psi_d(const StepArgs<R>& a, int i, int j, int k, int sx, int sy, bool cell, CellPsi<R>& ps)
 {
     const int L2 = 2 * a.L;
-    ps.sz = ldg_nh(a.tz.slot + k);
-    /* FP64: the z profile with the other early loads (measured faster);
-     * FP32 reads it in d_update (measured faster there) */
-    ps.kdz = sizeof(R) == 8 ? ldg_nh(a.tz.kd + k) : R(0);
+    ps.sz = z_slot(a, k);
+    ps.z = z_coef<R, STRICT, false>(a, ps.sz, k);
     ps.xy = ps.xz = ps.yx = ps.yz = ps.zx = ps.zy = R(0);
+    if (!cell) return;
     if (sx >= 0) {
         const int q = (k * a.ny + j) * L2 + sx;
         ps.xy = a.psi.dxy[q];
@@ -124,7 +164,7 @@ __device__ __forceinline__ void prefetch_psi_d(const StepArgs<R>& a, int i, int 
         asm volatile("prefetch.global.L1 [%0];" ::"l"(a.psi.dyx + q));
         asm volatile("prefetch.global.L1 [%0];" ::"l"(a.psi.dyz + q));
     }
-    const int sz = ldg_nh(a.tz.slot + k);
+    const int sz = z_slot(a, k);
     if (sz >= 0) {
         const int q = (sz * a.ny + j) * a.nxp + i;
         asm volatile("prefetch.global.L1 [%0];" ::"l"(a.psi.dzx + q));
@@ -134,11 +174,12 @@ __device__ __forceinline__ void prefetch_psi_d(const StepArgs<R>& a, int i, int 
 
 /* D sweep (fdtd.c:3238-3343) for one interior cell; hx0..hz0 are H at the
  * cell, hxk/hyk at k-1, hz_jm/hx_jm at j-1, hz_im/hy_im at i-1; ps holds the
- * old psi values (load_psi_d). */
+ * old psi values (load_psi_d), xt and yt are the cell's entries of the
+ * block's coefficient table (pml_table). */
 template <typename R, bool STRICT>
 __device__ __forceinline__ void d_update(const StepArgs<R>& a, int i, int j, int k, int sx, int sy, R hx0, R hy0,
                                          R hz0, R hxk, R hyk, R hz_jm, R hx_jm, R hz_im, R hy_im,
-                                         const CellPsi<R>& ps, R& dx, R& dy, R& dz)
+                                         const CellPsi<R>& ps, const R* xt, const R* yt, R& dx, R& dy, R& dz)
 {
     const int L2 = 2 * a.L;
     const int sz = ps.sz;
@@ -151,20 +192,20 @@ __device__ __forceinline__ void d_update(const StepArgs<R>& a, int i, int j, int
         const double dHx_dy = SOp::div(SOp::sub(hx0, hx_jm), a.dys);
         double kappa_x = 1.0, kappa_y = 1.0, kappa_z = 1.0;
         if (sx >= 0) { /* fdtd.c:3258-3285 */
-            kappa_x = ldg_nh(a.tx.kappa + i);
-            const double b = ldg_nh(a.tx.b + i), cc = ldg_nh(a.tx.c + i);
+            kappa_x = xt[0];
+            const double b = xt[1], cc = xt[2];
             const int q = (k * a.ny + j) * L2 + sx;
             a.psi.dxy[q] = SOp::add(SOp::mul(b, ps.xy), SOp::mul(cc, -dHz_dx));
             a.psi.dxz[q] = SOp::add(SOp::mul(b, ps.xz), SOp::mul(cc, dHy_dx));
         }
         if (sy >= 0) { /* fdtd.c:3288-3315 */
-            kappa_y = ldg_nh(a.ty.kappa + j);
-            const double b = ldg_nh(a.ty.b + j), cc = ldg_nh(a.ty.c + j);
+            kappa_y = yt[0];
+            const double b = yt[1], cc = yt[2];
             const int q = (k * L2 + sy) * a.nxp + i;
             a.psi.dyx[q] = SOp::add(SOp::mul(b, ps.yx), SOp::mul(cc, dHz_dy));
             a.psi.dyz[q] = SOp::add(SOp::mul(b, ps.yz), SOp::mul(cc, -dHx_dy));
         }
-        if (sz >= 0) kappa_z = ldg_nh(a.tz.kappa + k); /* fdtd.c:3318-3334 */
+        kappa_z = ps.z.k; /* fdtd.c:3318-3334 */
         /* fdtd.c:3337-3339 */
         const double ux = SOp::add(SOp::add(SOp::add(SOp::div(dHz_dy, kappa_y), ps.yx), SOp::div(-dHy_dz, kappa_z)), ps.zx);
         const double uy = SOp::add(SOp::add(SOp::add(SOp::div(-dHz_dx, kappa_x), ps.xy), SOp::div(dHx_dz, kappa_z)), ps.zy);
@@ -173,7 +214,7 @@ __device__ __forceinline__ void d_update(const StepArgs<R>& a, int i, int j, int
         dy = SOp::add(dy, SOp::mul(a.dt, uy));
         dz = SOp::add(dz, SOp::mul(a.dt, uz));
         if (sz >= 0) { /* fdtd.c:3340-3343 */
-            const double b = ldg_nh(a.tz.b + k), cc = ldg_nh(a.tz.c + k);
+            const double b = ps.z.b, cc = ps.z.c;
             const int qz = (sz * a.ny + j) * a.nxp + i;
             a.psi.dzx[qz] = SOp::add(SOp::mul(b, ps.zx), SOp::mul(cc, -dHy_dz));
             a.psi.dzy[qz] = SOp::add(SOp::mul(b, ps.zy), SOp::mul(cc, dHx_dz));
@@ -181,29 +222,28 @@ __device__ __forceinline__ void d_update(const StepArgs<R>& a, int i, int j, int
     } else {
         const R dHzy = hz0 - hz_jm, dHyz = hy0 - hyk, dHxz = hx0 - hxk;
         const R dHzx = hz0 - hz_im, dHyx = hy0 - hy_im, dHxy = hx0 - hx_jm;
-        const R kdx = ldg(a.tx.kd + i), kdy = ldg(a.ty.kd + j);
-        const R kdz = sizeof(R) == 8 ? ps.kdz : ldg_nh(a.tz.kd + k);
+        const R kdx = xt[0], kdy = yt[0], kdz = ps.z.k;
         /* psi terms enter as zeros outside the PML */
-        R ux = kdy * dHzy - kdz * dHyz + ps.yx + ps.zx;
-        R uy = -kdx * dHzx + kdz * dHxz + ps.xy + ps.zy;
-        R uz = kdx * dHyx - kdy * dHxy + ps.xz + ps.yz;
+        R ux = (curl2(kdy, dHzy, kdz, dHyz) + ps.yx) + ps.zx;
+        R uy = (curl2(kdz, dHxz, kdx, dHzx) + ps.xy) + ps.zy;
+        R uz = (curl2(kdx, dHyx, kdy, dHxy) + ps.xz) + ps.yz;
         if (sx >= 0) {
-            const R b = ldg_nh(a.tx.b + i), cd = ldg_nh(a.tx.cd + i);
+            const R b = xt[1], cd = xt[2];
             const int q = (k * a.ny + j) * L2 + sx;
-            a.psi.dxy[q] = b * ps.xy - cd * dHzx;
-            a.psi.dxz[q] = b * ps.xz + cd * dHyx;
+            a.psi.dxy[q] = curl2(b, ps.xy, cd, dHzx);
+            a.psi.dxz[q] = curl2(b, ps.xz, -cd, dHyx);
         }
         if (sy >= 0) {
-            const R b = ldg_nh(a.ty.b + j), cd = ldg_nh(a.ty.cd + j);
+            const R b = yt[1], cd = yt[2];
             const int q = (k * L2 + sy) * a.nxp + i;
-            a.psi.dyx[q] = b * ps.yx + cd * dHzy;
-            a.psi.dyz[q] = b * ps.yz - cd * dHxy;
+            a.psi.dyx[q] = curl2(b, ps.yx, -cd, dHzy);
+            a.psi.dyz[q] = curl2(b, ps.yz, cd, dHxy);
         }
         if (sz >= 0) {
-            const R b = ldg_nh(a.tz.b + k), cd = ldg_nh(a.tz.cd + k);
+            const R b = ps.z.b, cd = ps.z.c;
             const int q = (sz * a.ny + j) * a.nxp + i;
-            a.psi.dzx[q] = b * ps.zx - cd * dHyz;
-            a.psi.dzy[q] = b * ps.zy + cd * dHxz;
+            a.psi.dzx[q] = curl2(b, ps.zx, cd, dHyz);
+            a.psi.dzy[q] = curl2(b, ps.zy, -cd, dHxz);
         }
         dx += ux;
         dy += uy;
@@ -211,7 +251,90 @@ __device__ __forceinline__ void d_update(const StepArgs<R>& a, int i, int j, int
     }
 }
 
-/* FP32: E = iso * D from the kernel parameters for plain isotropic cells
+/* H of one cell (fast modes): the six E differences of its curl, the CPML
+ * terms xy xz yx yz zx zy (zero outside the PML) */
+template <typename R>
+__device__ __forceinline__ void h_update(R khx, R khy, R khz, R dEyz, R dEzy, R dEzx, R dExz, R dExy, R dEyx,
+                                         R pxy, R pxz, R pyx, R pyz, R pzx, R pzy, R& hx, R& hy, R& hz)
+{
+    hx += (curl2(khz, dEyz, khy, dEzy) + pyx) + pzx;
+    hy += (curl2(khx, dEzx, khz, dExz) + pxy) + pzy;
+    hz += (curl2(khy, dExy, khx, dEyx) + pxz) + pyz;
+}
+
+/* the eps'' term of a lossy cell (fdtd.c:3349-3353): u -= q E */
+template <typename R>
+__device__ __forceinline__ void loss_sub(const R* q, R ex, R ey, R ez, R& ux, R& uy, R& uz)
+{
+    ux -= fma_(q[0], ex, fma_(q[1], ey, q[2] * ez));
+    uy -= fma_(q[3], ex, fma_(q[4], ey, q[5] * ez));
+    uz -= fma_(q[6], ex, fma_(q[7], ey, q[8] * ez));
+}
+
+/* Cells that keep E alone (kEOnly): E = M D for a fixed M, so
+ * E^{n+1} = E^n + M (D^{n+1} - D^n).  The increment u is summed on its own,
+ * as for the D that other cells keep, and enters E with one rounding per
+ * product: against a 64-bit run the FP32 fields are as close as with D kept
+ * (E = M D rounds the sum in D and the product). */
+template <typename R>
+__device__ __forceinline__ void iso_add(R s, R ux, R uy, R uz, R& ex, R& ey, R& ez)
+{
+    ex = fma_(s, ux, ex);
+    ey = fma_(s, uy, ey);
+    ez = fma_(s, uz, ez);
+}
+template <typename R>
+__device__ __forceinline__ void e_only_add(const R* m, R ux, R uy, R uz, R& ex, R& ey, R& ez)
+{
+    ex += fma_(m[0], ux, fma_(m[1], uy, m[2] * uz));
+    ey += fma_(m[3], ux, fma_(m[4], uy, m[5] * uz));
+    ez += fma_(m[6], ux, fma_(m[7], uy, m[8] * uz));
+}
+
+/* D of a pool cell: D += u.  FP32 carries what the sum rounds off to the next
+ * step: the lattice integrates E = M (D - P) twice, so the slow drift of a
+ * plain sum's rounding (a static charge) is the largest error of r and v,
+ * several times that of the fields.  w holds the three components' remainders
+ * in 10 bits each, in units of 2^-10 ulp of the D they belong to: one word per
+ * cell read and written. */
+template <typename R>
+__device__ __forceinline__ void pool_add(const StepArgs<R>& a, int64_t slot, R ux, R uy, R uz, R& dx, R& dy, R& dz)
+{
+    const int64_t ns = a.nslot;
+    const R* __restrict__ dp = a.Dp + slot;
+    dx = dp[0];
+    dy = dp[ns];
+    dz = dp[2 * ns];
+    if constexpr (sizeof(R) == 4) {
+        if (a.Dc) {
+            const uint32_t w = a.Dc[slot];
+            uint32_t out = 0;
+            auto add = [&](float& d, float u, int sh) {
+                const int q = (int)(w << (22 - sh)) >> 22;
+                /* 2^(exponent of d) 2^-33 */
+                const float y = fma_((float)q, __fmul_rn(__uint_as_float(__float_as_uint(d) & 0x7f800000u), 0x1p-33f), u);
+                const float s = __fadd_rn(d, y), t = __fsub_rn(s, d);
+                const float e = __fadd_rn(__fsub_rn(d, __fsub_rn(s, t)), __fsub_rn(y, t)); /* d + y - s, exactly */
+                const uint32_t ex = (__float_as_uint(s) >> 23) & 255u;
+                int n = 0;
+                if (ex > 40u && ex < 254u) n = __float2int_rn(__fmul_rn(e, __uint_as_float((287u - ex) << 23)));
+                n = max(-511, min(511, n));
+                out |= ((uint32_t)n & 1023u) << sh;
+                d = s;
+            };
+            add(dx, ux, 0);
+            add(dy, uy, 10);
+            add(dz, uz, 20);
+            a.Dc[slot] = out;
+            return;
+        }
+    }
+    dx += ux;
+    dy += uy;
+    dz += uz;
+}
+
+/* FP32: iso from the kernel parameters for plain isotropic cells
  * (measured 2 % faster on the 256^3 tip workload; FP64 measured slower) */
 #ifndef PHP_ISO_PARAM
 #define PHP_ISO_PARAM 1
@@ -293,15 +416,6 @@ __device__ __forceinline__ void e_update(const StepArgs<R>& a, const MatCoef<R>&
                                          const IonPre* pre = nullptr)
 {
     const int flags = m.flags;
-    if constexpr (!STRICT) {
-        if (flags & kIso) { /* vacuum and isotropic lossless dielectrics */
-            const R s = m.eps_inv[0];
-            ex = s * dx;
-            ey = s * dy;
-            ez = s * dz;
-            return;
-        }
-    }
     int64_t slot = -1;
     if (pre) slot = pre->slot;
     else if (flags & (kAde | kAtoms)) slot = a.slot[c];
@@ -513,97 +627,105 @@ __device__ __forceinline__ void e_update(const StepArgs<R>& a, const MatCoef<R>&
     ez = nc;
 }
 
-/* One cell of the fused sweep once its H values are known: D update on
- * the interior with the lossy eps'' term (fdtd.c:3238-3356), the sources of
- * this step (fdtd.c:3363-3396), D -> E / ADE / ions (fdtd.c:3404-3528).  The
- * new D and E come back in dx..dz and ex_out..ez_out; the caller stores
- * them (e_cell below in place, he_sweep_tma E into the new level). */
-template <typename R, bool STRICT, int NAMAX>
-__device__ __forceinline__ void e_cell_values(const StepArgs<R>& a, int i, int j, int k, int c, bool interior, int sx,
-                                              int sy, R hx0, R hy0, R hz0, R hxk, R hyk, R hz_jm, R hx_jm, R hz_im,
-                                              R hy_im, R& dx, R& dy, R& dz, int mid, const MatCoef<R>* mcs,
-                                              const CellPsi<R>* pre, R& ex_out, R& ey_out, R& ez_out,
-                                              const IonPre* ipre = nullptr)
+/* One cell of the fused sweep once its H values are known, fast modes: D
+ * increment on the interior with the lossy eps'' term (fdtd.c:3238-3356), the
+ * sources of this step (fdtd.c:3363-3396), then E += M dD where E is kept
+ * alone, else D from its pool, D -> E / ADE / ions (fdtd.c:3404-3528).  ex..ez
+ * hold E^n on entry and E^{n+1} on return (atom cells without loss do not
+ * read the old one); the caller stores them. */
+template <typename R, int NAMAX>
+__device__ __forceinline__ void e_cell_fast(const StepArgs<R>& a, int i, int j, int k, int c, bool interior, int sx,
+                                            int sy, R hx0, R hy0, R hz0, R hxk, R hyk, R hz_jm, R hx_jm, R hz_im,
+                                            R hy_im, int mid, const CellPsi<R>& ps, const R* xt, const R* yt, R& ex, R& ey,
+                                            R& ez, int slot_pre)
 {
-    const R* __restrict__ exp_ = a.f.ex;
-    const R* __restrict__ eyp = a.f.ey;
-    const R* __restrict__ ezp = a.f.ez;
-    /* plain isotropic cells take E = iso * D without the material record */
-    const R iso = (!STRICT && PHP_ISO_PARAM && sizeof(R) == 4 && mid < kIsoMats) ? a.iso[mid] : R(0);
-    /* mcs: the block's shared-memory copy of the first kSmemMats records */
-    const MatCoef<R>* mp = iso != R(0) ? nullptr : ((mcs && mid < a.nmat) ? &mcs[mid] : &a.mc[mid]);
-    const int flags = mp ? mp->flags : kIso;
-    R ex = R(0), ey = R(0), ez = R(0);
-    if (flags & (kLossy | kAde)) { ex = exp_[c]; ey = eyp[c]; ez = ezp[c]; }
-    /* FP32 sums this step's D increment on its own before adding it to D:
-     * the ADE update needs the increment without D's rounding */
-    constexpr bool kInc = !STRICT && sizeof(R) == 4;
-    R ix = R(0), iy = R(0), iz = R(0);
-    R& ux = kInc ? ix : dx;
-    R& uy = kInc ? iy : dy;
-    R& uz = kInc ? iz : dz;
+    /* plain isotropic cells take iso without the material record */
+    const R iso = (PHP_ISO_PARAM && sizeof(R) == 4 && mid < kIsoMats) ? a.iso[mid] : R(0);
+    const MatCoef<R>* mp = iso != R(0) ? nullptr : &a.mc[mid];
+    const bool dmc = mid == a.dmc_id;
+    const int flags = !mp ? kIso | kEOnly : dmc ? a.dmc.flags : mp->flags;
+    R ux = R(0), uy = R(0), uz = R(0);
     if (interior) {
-        CellPsi<R> ps;
-        if (pre) ps = *pre;
-        else load_psi_d(a, i, j, k, sx, sy, ps);
-        d_update<R, STRICT>(a, i, j, k, sx, sy, hx0, hy0, hz0, hxk, hyk, hz_jm, hx_jm, hz_im, hy_im, ps, ux, uy, uz);
-        if (flags & kLossy) { /* fdtd.c:3349-3353 */
-            const R* q = mp->eps_im;
-            if constexpr (STRICT) {
-                dx = SOp::sub(dx, SOp::mul(SOp::mul(a.c1, SOp::add(SOp::add(SOp::mul(q[0], ex), SOp::mul(q[1], ey)), SOp::mul(q[2], ez))), a.eps0));
-                dy = SOp::sub(dy, SOp::mul(SOp::mul(a.c1, SOp::add(SOp::add(SOp::mul(q[3], ex), SOp::mul(q[4], ey)), SOp::mul(q[5], ez))), a.eps0));
-                dz = SOp::sub(dz, SOp::mul(SOp::mul(a.c1, SOp::add(SOp::add(SOp::mul(q[6], ex), SOp::mul(q[7], ey)), SOp::mul(q[8], ez))), a.eps0));
-            } else {
-                ux -= q[0] * ex + q[1] * ey + q[2] * ez;
-                uy -= q[3] * ex + q[4] * ey + q[5] * ez;
-                uz -= q[6] * ex + q[7] * ey + q[8] * ez;
+        d_update<R, false>(a, i, j, k, sx, sy, hx0, hy0, hz0, hxk, hyk, hz_jm, hx_jm, hz_im, hy_im, ps, xt, yt, ux, uy, uz);
+        if (flags & kLossy) loss_sub(mp->eps_im, ex, ey, ez, ux, uy, uz);
+    }
+    /* sources, in source order (fdtd.c:3363-3396) */
+    for (int s = 0; s < a.nsrc; ++s) {
+        if (a.src_cell[s] != c) continue;
+        if (sizeof(R) == 4 && (flags & kEOnly)) {
+            /* E of the cell in double (StepArgs::src_acc) */
+            double* acc = a.src_acc + 3 * s;
+            double u[3] = {(double)ux, (double)uy, (double)uz};
+            for (int t = s; t < a.nsrc; ++t)
+                if (a.src_cell[t] == c) u[a.src_comp[t]] += a.src_val[t] * a.dt;
+            const double iso_d = (flags & kIso) ? (double)(mp ? mp->eps_inv[0] : iso) : 0.0;
+            for (int q = 0; q < 3; ++q) {
+                const double d = (flags & kIso) ? iso_d * u[q]
+                                                : (double)mp->em[3 * q] * u[0] + (double)mp->em[3 * q + 1] * u[1] +
+                                                      (double)mp->em[3 * q + 2] * u[2];
+                acc[q] = __dadd_rn(acc[q], d);
             }
+            ex = (R)acc[0];
+            ey = (R)acc[1];
+            ez = (R)acc[2];
+            return;
+        }
+        const R add = R(a.src_val[s] * a.dt);
+        if (a.src_comp[s] == 0) ux += add;
+        else if (a.src_comp[s] == 1) uy += add;
+        else if (a.src_comp[s] == 2) uz += add;
+    }
+    if (flags & kIso) {
+        iso_add(mp ? mp->eps_inv[0] : iso, ux, uy, uz, ex, ey, ez);
+    } else if (flags & kEOnly) {
+        e_only_add(mp->em, ux, uy, uz, ex, ey, ez);
+    } else {
+        IonPre ip;
+        ip.slot = slot_pre >= 0 ? slot_pre : a.slot[c];
+        const int64_t ns = a.nslot;
+        R* __restrict__ dp = a.Dp + ip.slot;
+        R dx, dy, dz;
+        pool_add(a, ip.slot, ux, uy, uz, dx, dy, dz);
+        if (dmc) e_update<R, false, 0>(a, a.dmc, c, dx, dy, dz, ux, uy, uz, ex, ey, ez, &ip);
+        else if (NAMAX > 0 && !(flags & kAtoms)) e_update<R, false, 0>(a, *mp, c, dx, dy, dz, ux, uy, uz, ex, ey, ez, &ip);
+        else e_update<R, false, NAMAX>(a, *mp, c, dx, dy, dz, ux, uy, uz, ex, ey, ez, &ip);
+        dp[0] = dx;
+        dp[ns] = dy;
+        dp[2 * ns] = dz;
+    }
+}
+
+/* The same cell of the strict mode, every operation in the reference's
+ * order: D and E in place in the field arrays. */
+template <int NAMAX>
+__device__ __forceinline__ void e_cell_strict(const StepArgs<double>& a, int i, int j, int k, int c, bool interior, int sx,
+                                              int sy, double hx0, double hy0, double hz0, double hxk, double hyk,
+                                              double hz_jm, double hx_jm, double hz_im, double hy_im, double dx, double dy,
+                                              double dz, int mid, const CellPsi<double>& ps, const double* xt, const double* yt)
+{
+    const MatCoef<double>* mp = &a.mc[mid];
+    const int flags = mp->flags;
+    double ex = 0.0, ey = 0.0, ez = 0.0;
+    if (flags & (kLossy | kAde)) { ex = a.f.ex[c]; ey = a.f.ey[c]; ez = a.f.ez[c]; }
+    if (interior) {
+        d_update<double, true>(a, i, j, k, sx, sy, hx0, hy0, hz0, hxk, hyk, hz_jm, hx_jm, hz_im, hy_im, ps, xt, yt, dx, dy, dz);
+        if (flags & kLossy) { /* fdtd.c:3349-3353 */
+            const double* q = mp->eps_im;
+            dx = SOp::sub(dx, SOp::mul(SOp::mul(a.c1, SOp::add(SOp::add(SOp::mul(q[0], ex), SOp::mul(q[1], ey)), SOp::mul(q[2], ez))), a.eps0));
+            dy = SOp::sub(dy, SOp::mul(SOp::mul(a.c1, SOp::add(SOp::add(SOp::mul(q[3], ex), SOp::mul(q[4], ey)), SOp::mul(q[5], ez))), a.eps0));
+            dz = SOp::sub(dz, SOp::mul(SOp::mul(a.c1, SOp::add(SOp::add(SOp::mul(q[6], ex), SOp::mul(q[7], ey)), SOp::mul(q[8], ez))), a.eps0));
         }
     }
     /* sources, in source order (fdtd.c:3363-3396) */
     for (int s = 0; s < a.nsrc; ++s) {
         if (a.src_cell[s] == c) {
-            const double v = a.src_val[s];
-            if constexpr (STRICT) {
-                const double add = SOp::mul(v, a.dt);
-                if (a.src_comp[s] == 0) dx = SOp::add(dx, add);
-                else if (a.src_comp[s] == 1) dy = SOp::add(dy, add);
-                else if (a.src_comp[s] == 2) dz = SOp::add(dz, add);
-            } else {
-                const R add = R(v * a.dt);
-                if (a.src_comp[s] == 0) ux += add;
-                else if (a.src_comp[s] == 1) uy += add;
-                else if (a.src_comp[s] == 2) uz += add;
-            }
+            const double add = SOp::mul(a.src_val[s], a.dt);
+            if (a.src_comp[s] == 0) dx = SOp::add(dx, add);
+            else if (a.src_comp[s] == 1) dy = SOp::add(dy, add);
+            else if (a.src_comp[s] == 2) dz = SOp::add(dz, add);
         }
     }
-    if constexpr (kInc) {
-        dx += ix;
-        dy += iy;
-        dz += iz;
-    }
-    if (!mp) {
-        ex = iso * dx;
-        ey = iso * dy;
-        ez = iso * dz;
-    } else {
-        e_update<R, STRICT, NAMAX>(a, *mp, c, dx, dy, dz, ix, iy, iz, ex, ey, ez, ipre);
-    }
-    ex_out = ex;
-    ey_out = ey;
-    ez_out = ez;
-}
-
-/* e_cell_values with D and E stored to global memory */
-template <typename R, bool STRICT, int NAMAX>
-__device__ __forceinline__ void e_cell(const StepArgs<R>& a, int i, int j, int k, int c, bool interior, int sx, int sy,
-                                       R hx0, R hy0, R hz0, R hxk, R hyk, R hz_jm, R hx_jm, R hz_im, R hy_im, R dx, R dy,
-                                       R dz, int mid, const MatCoef<R>* mcs, const CellPsi<R>* pre,
-                                       const IonPre* ipre = nullptr)
-{
-    R ex, ey, ez;
-    e_cell_values<R, STRICT, NAMAX>(a, i, j, k, c, interior, sx, sy, hx0, hy0, hz0, hxk, hyk, hz_jm, hx_jm, hz_im, hy_im,
-                                    dx, dy, dz, mid, mcs, pre, ex, ey, ez, ipre);
+    e_update<double, true, NAMAX>(a, *mp, c, dx, dy, dz, 0.0, 0.0, 0.0, ex, ey, ez);
     a.f.dx[c] = dx;
     a.f.dy[c] = dy;
     a.f.dz[c] = dz;
