@@ -37,11 +37,12 @@ using namespace phpdev;
 namespace {
 
 constexpr int kMaxChunk = 256;      /* steps per recorded graph */
-/* steps per graph where a step has branches: recording and instantiating one
- * takes some 60 us per step then, 10 us without; every php_step call of more
- * steps replays it (its input rows come through page-locked slots of this
- * many steps, so that the same 512 steps are enqueued ahead) */
-constexpr int kBranchChunk = 16;
+/* steps per graph where a step is three to five sweep launches: recording and
+ * instantiating one takes some 35 us per step then (a launch without the
+ * programmatic attribute takes 4 us); php_step calls of more steps replay it,
+ * their input rows in page-locked slots of this many steps, so that the same
+ * 512 steps are enqueued ahead */
+constexpr int kListChunk = 64;
 constexpr int kProfKinds = PHP_PROFILE_KINDS; /* H sweep, E sweep, probe, DFT, ion pass, one-launch step */
 constexpr int kProbeCap = 8192;     /* probe rows held on the device */
 constexpr double kEpsInf = 20.0;    /* EPS_INF, fdtd.c:202 */
@@ -56,17 +57,6 @@ constexpr double kEpsInf = 20.0;    /* EPS_INF, fdtd.c:202 */
 constexpr double kIonScale32 = 281474976710656.0; /* 2^48 */
 
 thread_local std::string g_create_error; /* errors of php_create, per calling thread */
-
-/* Streams and events that fork a step's launches into branches while its
- * graph is recorded (only then: the recorded graph holds the branches).  Taken
- * from a pool, since creating streams takes milliseconds; the pool keeps at
- * most kSidePool of them, one per thread recording at a time. */
-struct SideStreams {
-    int device = 0;
-    cudaStream_t s[2] = {};
-    cudaEvent_t fork = nullptr, join[2] = {};
-};
-constexpr size_t kSidePool = 8;
 
 struct DftPlane {
     int comp, z, first, interval, nfreq, cast_f32;
@@ -104,9 +94,9 @@ struct php_ctx {
      * device busy does not queue behind their sweeps; `stream` (default
      * priority) takes over at the end of php_create */
     cudaStream_t setup = nullptr;
-    /* split: the H sweep of the rest runs beside the interior launch, and the
-     * E sweep's launches of the three kinds of blocks beside each other */
-    SideStreams* side = nullptr; /* while a graph is recorded */
+    /* launches recorded in the graph being captured (launch_chained), -1 when
+     * none is */
+    int chain = -1;
     /* page-locked staging of host -> device uploads (upload()) */
     void* up_buf[2] = {};
     cudaEvent_t up_ev[2] = {};
@@ -163,9 +153,9 @@ struct php_ctx {
     double* step_in = nullptr;   /* buffer the graph being recorded reads */
     double* step_in_dev[2] = {};  /* [kMaxChunk][row] each */
     double* step_in_host[2] = {}; /* pinned */
-    int max_chunk = kMaxChunk;    /* steps per graph: kMaxChunk or kBranchChunk */
+    int max_chunk = kMaxChunk;    /* steps per graph: kMaxChunk or kListChunk */
     /* copy out of a page-locked slot (max_chunk rows; 2 kMaxChunk rows in all) finished */
-    cudaEvent_t staged[2 * kMaxChunk / kBranchChunk] = {};
+    cudaEvent_t staged[2 * kMaxChunk / kListChunk] = {};
     int chunk_no = 0;
     int step_row = 0;
     int probe_off = 0;           /* offset of the monitor row's index in a step-input row */
@@ -819,10 +809,10 @@ static int split_launches(const php_ctx* ctx)
     return n;
 }
 
-static inline void prof_mark(php_ctx* ctx, int s_local, int kind, int end, cudaStream_t st = nullptr)
+static inline void prof_mark(php_ctx* ctx, int s_local, int kind, int end)
 {
     if (ctx->profile)
-        cudaEventRecordWithFlags(ctx->prof_ev[((size_t)s_local * kProfKinds + kind) * 2 + end], st ? st : ctx->stream,
+        cudaEventRecordWithFlags(ctx->prof_ev[((size_t)s_local * kProfKinds + kind) * 2 + end], ctx->stream,
                                  cudaEventRecordExternal);
 }
 
@@ -880,37 +870,54 @@ static void launch_ions(php_ctx* ctx)
     ion_update_cc<R, 64><<<grid, kIonTile, 0, st>>>(a);
 }
 
+/* A sweep launch.  While a graph is recorded each one but the first is a
+ * programmatic launch behind the one before it (chain_enter; not under
+ * php_profile_enable, whose events stand between the launches); beside: it
+ * does not depend on that one. */
+template <typename R, typename F>
+static void launch_chained(php_ctx* ctx, F kernel, dim3 grid, uint32_t smem, StepArgs<R>& a, const TmaMaps& maps, bool beside = false)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(kBlockX, kBlockY, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    const bool chained = ctx->chain > 0 && !ctx->profile;
+    if (chained) {
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+    }
+    if (ctx->chain >= 0) ctx->chain++;
+    a.beside = chained && beside;
+    cudaLaunchKernelEx(&cfg, kernel, a, maps);
+}
+
 /* The E sweep's launches over the block lists of its three kinds, beside each
- * other; a.f and maps as for one launch. */
+ * other (the first behind the launches before); a.f and maps as for one
+ * launch. */
 template <typename R, int NA>
 static void launch_e_lists(php_ctx* ctx, int s_local, StepArgs<R>& a, const TmaMaps& maps)
 {
-    const dim3 block(kBlockX, kBlockY, 1);
     const uint32_t smem = TmaGeom<R>::E_SMEM;
-    SideStreams& sd = *ctx->side;
-    auto fork = [&](int q) { cudaStreamWaitEvent(sd.s[q], sd.fork, 0); };
-    auto join = [&](int q) {
-        cudaEventRecord(sd.join[q], sd.s[q]);
-        cudaStreamWaitEvent(ctx->stream, sd.join[q], 0);
-    };
+    bool beside = false;
     prof_mark(ctx, s_local, 1, 0);
-    cudaEventRecord(sd.fork, ctx->stream);
     if (ctx->nlist[4]) { /* few blocks with long chains: first */
-        fork(0);
         a.list = ctx->lists[4];
-        e_sweep_tma<R, false, NA, kEGeneral><<<ctx->nlist[4], block, smem, sd.s[0]>>>(a, maps);
+        launch_chained(ctx, e_sweep_tma<R, false, NA, kEGeneral>, dim3(ctx->nlist[4]), smem, a, maps, beside);
+        beside = true;
     }
     if (ctx->nlist[3]) {
-        fork(1);
         a.list = ctx->lists[3];
-        e_sweep_tma<R, false, NA, kEAtoms><<<ctx->nlist[3], block, smem, sd.s[1]>>>(a, maps);
+        launch_chained(ctx, e_sweep_tma<R, false, NA, kEAtoms>, dim3(ctx->nlist[3]), smem, a, maps, beside);
+        beside = true;
     }
     if (ctx->nlist[2]) {
         a.list = ctx->lists[2];
-        e_sweep_tma<R, false, 0, kEPlain><<<ctx->nlist[2], block, smem, ctx->stream>>>(a, maps);
+        launch_chained(ctx, e_sweep_tma<R, false, 0, kEPlain>, dim3(ctx->nlist[2]), smem, a, maps, beside);
     }
-    if (ctx->nlist[4]) join(0);
-    if (ctx->nlist[3]) join(1);
     prof_mark(ctx, s_local, 1, 1);
     a.list = nullptr;
 }
@@ -919,7 +926,6 @@ template <typename R, bool STRICT, int NA>
 static void launch_step_t(php_ctx* ctx, int s_local, int& launches)
 {
     StepArgs<R> a = make_args<R>(ctx, s_local);
-    dim3 block(kBlockX, kBlockY, 1);
     const int nchunk = (ctx->nz + ctx->zchunk - 1) / ctx->zchunk;
     a.zc0 = ctx->zc_count < 0 ? 0 : ctx->zc_first;
     dim3 grid((ctx->nx + kBlockX - 1) / kBlockX, (ctx->ny + kBlockY - 1) / kBlockY,
@@ -927,24 +933,19 @@ static void launch_step_t(php_ctx* ctx, int s_local, int& launches)
     bool do_h = ctx->step_part & 1, do_e = ctx->step_part & 2;
     const bool do_rest = ctx->step_part & 4;
     if constexpr (!STRICT) {
-        if (ctx->split && ctx->side && do_h && do_e && grid.z > 0) {
+        if (ctx->split && do_h && do_e && grid.z > 0) {
             /* the interior and the H sweep of the rest read this level and
              * write the other; then the E sweep of the rest, whose H is the new
              * one */
             StepArgs<R> in = a;
             in.list = ctx->lists[0];
-            SideStreams& sd = *ctx->side;
-            cudaEventRecord(sd.fork, ctx->stream);
-            cudaStreamWaitEvent(sd.s[0], sd.fork, 0);
             prof_mark(ctx, s_local, 5, 0);
-            interior_sweep_tma<R><<<ctx->nlist[0], block, FusedGeom<R, true>::SMEM, ctx->stream>>>(in, ctx->maps);
+            launch_chained(ctx, interior_sweep_tma<R>, dim3(ctx->nlist[0]), FusedGeom<R, true>::SMEM, in, ctx->maps);
             prof_mark(ctx, s_local, 5, 1);
             a.list = ctx->lists[1];
-            prof_mark(ctx, s_local, 0, 0, sd.s[0]);
-            h_sweep_tma<R, STRICT><<<ctx->nlist[1], block, TmaGeom<R>::H_SMEM, sd.s[0]>>>(a, ctx->maps);
-            prof_mark(ctx, s_local, 0, 1, sd.s[0]);
-            cudaEventRecord(sd.join[0], sd.s[0]);
-            cudaStreamWaitEvent(ctx->stream, sd.join[0], 0);
+            prof_mark(ctx, s_local, 0, 0);
+            launch_chained(ctx, h_sweep_tma<R, STRICT>, dim3(ctx->nlist[1]), TmaGeom<R>::H_SMEM, a, ctx->maps, true);
+            prof_mark(ctx, s_local, 0, 1);
             TmaMaps me = ctx->maps;
             me.h_halo = ctx->maps_o.h_halo;
             launch_e_lists<R, NA>(ctx, s_local, a, me);
@@ -957,7 +958,7 @@ static void launch_step_t(php_ctx* ctx, int s_local, int& launches)
             prof_mark(ctx, s_local, 5, 0);
             const dim3 fgrid((ctx->nx + FusedGeom<R, false>::TX - 1) / FusedGeom<R, false>::TX, (ctx->ny + FusedGeom<R, false>::TY - 1) / FusedGeom<R, false>::TY,
                              (ctx->nz + ctx->zstep - 1) / ctx->zstep);
-            he_sweep_tma<R, NA><<<fgrid, block, FusedGeom<R, false>::SMEM, ctx->stream>>>(a, ctx->maps);
+            launch_chained(ctx, he_sweep_tma<R, NA>, fgrid, FusedGeom<R, false>::SMEM, a, ctx->maps);
             prof_mark(ctx, s_local, 5, 1);
             launches++;
             swap_levels(ctx);
@@ -967,12 +968,12 @@ static void launch_step_t(php_ctx* ctx, int s_local, int& launches)
     if (grid.z == 0) { /* an empty part: no sweep blocks */
     } else if (do_h) {
         prof_mark(ctx, s_local, 0, 0);
-        h_sweep_tma<R, STRICT><<<grid, block, TmaGeom<R>::H_SMEM, ctx->stream>>>(a, ctx->maps);
+        launch_chained(ctx, h_sweep_tma<R, STRICT>, grid, TmaGeom<R>::H_SMEM, a, ctx->maps);
         prof_mark(ctx, s_local, 0, 1);
         launches++;
     }
     if constexpr (!STRICT) {
-        if (ctx->by_class && ctx->side && do_e && ctx->zc_count < 0) {
+        if (ctx->by_class && do_e && ctx->zc_count < 0) {
             launch_e_lists<R, NA>(ctx, s_local, a, ctx->maps);
             launches += split_launches(ctx);
             do_e = false;
@@ -980,7 +981,7 @@ static void launch_step_t(php_ctx* ctx, int s_local, int& launches)
     }
     if (do_e && grid.z > 0) {
         prof_mark(ctx, s_local, 1, 0);
-        e_sweep_tma<R, STRICT, NA, kEAll><<<grid, block, TmaGeom<R>::E_SMEM, ctx->stream>>>(a, ctx->maps);
+        launch_chained(ctx, e_sweep_tma<R, STRICT, NA, kEAll>, grid, TmaGeom<R>::E_SMEM, a, ctx->maps);
         prof_mark(ctx, s_local, 1, 1);
         launches++;
     }
@@ -1285,55 +1286,6 @@ static void upload_release(php_ctx* ctx)
         ctx->up_buf[b] = nullptr;
         ctx->up_used[b] = false;
     }
-}
-
-static std::mutex g_side_mu;
-static std::vector<SideStreams*> g_side_free;
-
-static void side_destroy(SideStreams* s)
-{
-    for (int q = 0; q < 2; q++) {
-        if (s->join[q]) cudaEventDestroy(s->join[q]);
-        if (s->s[q]) cudaStreamDestroy(s->s[q]);
-    }
-    if (s->fork) cudaEventDestroy(s->fork);
-    delete s;
-}
-
-static SideStreams* side_get(int device)
-{
-    {
-        std::lock_guard<std::mutex> g(g_side_mu);
-        for (size_t q = 0; q < g_side_free.size(); q++)
-            if (g_side_free[q]->device == device) {
-                SideStreams* s = g_side_free[q];
-                g_side_free.erase(g_side_free.begin() + q);
-                return s;
-            }
-    }
-    SideStreams* s = new SideStreams();
-    s->device = device;
-    bool ok = cudaEventCreateWithFlags(&s->fork, cudaEventDisableTiming) == cudaSuccess;
-    for (int q = 0; q < 2 && ok; q++)
-        ok = cudaStreamCreateWithFlags(&s->s[q], cudaStreamNonBlocking) == cudaSuccess &&
-             cudaEventCreateWithFlags(&s->join[q], cudaEventDisableTiming) == cudaSuccess;
-    if (ok) return s;
-    cudaGetLastError();
-    side_destroy(s);
-    return nullptr;
-}
-
-static void side_put(SideStreams* s)
-{
-    if (!s) return;
-    {
-        std::lock_guard<std::mutex> g(g_side_mu);
-        if (g_side_free.size() < kSidePool) {
-            g_side_free.push_back(s);
-            return;
-        }
-    }
-    side_destroy(s);
 }
 
 static void ctx_free(php_ctx* ctx)
@@ -2107,7 +2059,7 @@ static int create_impl(const php_desc* desc, php_ctx* ctx)
         }
         ctx->by_class = !ctx->split && !ctx->fused && plan.on && plan.atom_id >= 0 && by_class_size(ctx);
         if (ctx->split || ctx->by_class) {
-            ctx->max_chunk = kBranchChunk;
+            ctx->max_chunk = kListChunk;
             std::vector<int4> hj, ej_all;
             if (ctx->split) {
                 plan.rest(ctx->prec == PHP_PREC_FP32 ? 8 : 4, hj, ej_all);
@@ -2274,22 +2226,14 @@ static int record_graph(php_ctx* ctx, int n, int b, cudaGraphExec_t* out)
     ctx->step_in = ctx->step_in_dev[b];
     step_fn fn = pick_step(ctx).launch;
     cudaGraph_t g = nullptr;
-    if (ctx->split || ctx->by_class) {
-        ctx->side = side_get(ctx->d.device);
-        if (!ctx->side) return fail(ctx, PHP_ERR_CUDA, "stream creation for a step's branches failed");
-    }
-    if (cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
-        side_put(ctx->side);
-        ctx->side = nullptr;
-        return fail(ctx, PHP_ERR_CUDA, "cudaStreamBeginCapture failed: %s", cudaGetErrorString(cudaGetLastError()));
-    }
+    CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
+    ctx->chain = 0;
     int launches = 0;
     for (int s = 0; s < n; s++) fn(ctx, s, launches);
     if (ctx->level != level) swap_levels(ctx);
     cudaError_t le = cudaGetLastError();
     cudaError_t ce = cudaStreamEndCapture(ctx->stream, &g);
-    side_put(ctx->side);
-    ctx->side = nullptr;
+    ctx->chain = -1;
     if (le != cudaSuccess) {
         if (g) cudaGraphDestroy(g);
         return fail(ctx, PHP_ERR_CUDA, "kernel launch during capture failed: %s", cudaGetErrorString(le));

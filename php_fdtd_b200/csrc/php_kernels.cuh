@@ -187,6 +187,9 @@ struct StepArgs {
      * A point source's own cell holds some 1e4 times the field of the
      * radiation zone, so the rounding of its sum is the largest error there. */
     double* src_acc;
+    /* programmatic launch chain: 1 when the launch before this one is one it
+     * does not depend on (it waits for it at its end; see chain_enter) */
+    int32_t beside;
     int32_t* err;              /* set to 1 by a block whose bounded wait gave up */
     int32_t stall_test;        /* failure-path test: the first H sweep block's wait gives up */
     /* where the sweeps write the new E, H and H CPML state.  The two sweeps of
@@ -268,6 +271,26 @@ __device__ __forceinline__ int32_t ldg_nh(const int32_t* p)
     int32_t v;
     asm volatile("ld.global.nc.s32 %0, [%1];" : "=r"(v) : "l"(p));
     return v;
+}
+
+/* The launches of recorded steps form a chain of programmatic launches: a
+ * launch may start once every block of the one before it has passed
+ * chain_enter, so its blocks fill the SMs that the last blocks of that one
+ * leave idle, and its set-up runs meanwhile.  A launch that depends on the one
+ * before waits in chain_enter for its completion, and only then lets the next
+ * one start.  One that does not (StepArgs::beside: its inputs come from
+ * launches further back, complete since the launch before it entered) waits at
+ * its end instead, in chain_leave, so that its own completion still implies
+ * that of all before it.  Launched without the attribute, both return at
+ * once. */
+__device__ __forceinline__ void chain_enter(int beside)
+{
+    if (!beside) asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void chain_leave(int beside, int tid)
+{
+    if (beside && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && tid == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 /* CPML slot of cell i of an axis of n cells: i at the low side, L + n - 1 - i

@@ -249,6 +249,7 @@ __global__ void __launch_bounds__(kBlockX * kBlockY, (kStepBlocks<R, NAMAX>))
         fence_barrier_init();
     }
     pml_table<R, false, false>(a, tab, i0, j0, G::TY, tid);
+    chain_enter(a.beside);
     __syncthreads();
     if (tid == 0) {
         for (int g = 0; g < max(SE, SH); ++g) {
@@ -580,6 +581,7 @@ __global__ void __launch_bounds__(kBlockX * kBlockY, (sizeof(R) == 8 ? PHP_INNER
         for (int s = 0; s < SE + SH; ++s) mbar_init(&ebar[s], 1);
         fence_barrier_init();
     }
+    chain_enter(a.beside);
     __syncthreads();
     if (tid == 0) {
         for (int g = 0; g < max(SE, SH); ++g) {
@@ -731,6 +733,7 @@ __global__ void __launch_bounds__(kBlockX * kBlockY, (sizeof(R) == 8 ? PHP_INNER
         if (a.ndft) dft_fold(a, a.enew, i, j + r, k0, k1); /* the new E */
         if (a.probe_rows) probe_fold(a, a.enew, a.hnew, i, j + r, k0, k1);
     }
+    chain_leave(a.beside, tid);
 }
 
 } // namespace phpdev

@@ -285,9 +285,12 @@ __global__ void __launch_bounds__(kBlockX * kBlockY, sizeof(R) == 4 ? PHP_H_MINB
     if (tid == 0) {
         for (int s = 0; s < G::HS + 1; ++s) mbar_init(&full[s], 1);
         fence_barrier_init();
-        for (int p = k0; p <= min(k1, k0 + G::HS - 1); ++p) issue(p);
     }
     const bool plain = !STRICT && job.cls;
+    if (!plain) pml_table<R, STRICT, true>(a, tab, i0, j0, G::TY, tid);
+    chain_enter(a.beside);
+    if (tid == 0)
+        for (int p = k0; p <= min(k1, k0 + G::HS - 1); ++p) issue(p);
     const bool active = (i < a.nx - 1) && (j < a.ny - 1);
     const int L2 = 2 * a.L;
     const int nxp = a.nxp, ny = a.ny;
@@ -312,10 +315,7 @@ __global__ void __launch_bounds__(kBlockX * kBlockY, sizeof(R) == 4 ? PHP_H_MINB
         if (p.sz >= 0) { p.zx = a.psi.hzx[qz]; p.zy = a.psi.hzy[qz]; }
     };
     Psi6 ps;
-    if (!plain) {
-        load_psi(k0, ps);
-        pml_table<R, STRICT, true>(a, tab, i0, j0, G::TY, tid);
-    }
+    if (!plain) load_psi(k0, ps);
     __syncthreads();
     if (a.stall_test && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) {
         /* failure-path test (StepArgs::stall_test): a bounded wait on the
@@ -372,6 +372,7 @@ __global__ void __launch_bounds__(kBlockX * kBlockY, sizeof(R) == 4 ? PHP_H_MINB
                 issue(k + G::HS);
             }
         }
+        chain_leave(a.beside, tid);
         return;
     }
 
@@ -504,6 +505,7 @@ __global__ void __launch_bounds__(kBlockX * kBlockY, sizeof(R) == 4 ? PHP_H_MINB
             issue(k + G::HS);
         }
     }
+    chain_leave(a.beside, tid);
 }
 
 /* ================================================================ E sweep */
@@ -558,8 +560,12 @@ __global__ void __launch_bounds__(kBlockX * kBlockY, (kEBlocks<R, NAMAX, CLS>))
     if (tid == 0) {
         for (int s = 0; s < G::ES; ++s) mbar_init(&full[s], 1);
         fence_barrier_init();
-        for (int p = k0 - 1; p <= min(k1 - 1, k0 - 1 + G::ES - 1); ++p) issue(p);
     }
+    const bool more = CLS == kEAtoms || CLS == kEGeneral || pm >= kPlainCpml; /* than the stencil */
+    if (more) pml_table<R, STRICT, false>(a, tab, i0, j0, G::TY, tid);
+    chain_enter(a.beside);
+    if (tid == 0)
+        for (int p = k0 - 1; p <= min(k1 - 1, k0 - 1 + G::ES - 1); ++p) issue(p);
     const bool active = (i < a.nx) && (j < a.ny);
     const bool interior = (i >= 1 && i < a.nx - 1 && j >= 1 && j < a.ny - 1);
     const int sx = active ? pml_slot(i, a.nx, a.L) : -1;
@@ -574,11 +580,10 @@ __global__ void __launch_bounds__(kBlockX * kBlockY, (kEBlocks<R, NAMAX, CLS>))
     const bool slots = !STRICT && a.slot != nullptr && active && (CLS == kEAtoms || CLS == kEGeneral || pm >= kPlainAtoms);
     CellPsi<R> ps;
     int slot = -1, mid = 0;
-    if (CLS == kEAtoms || CLS == kEGeneral || pm >= kPlainCpml) {
+    if (more) {
         if (first) load_psi_d<R, STRICT>(a, i, j, k0, sx, sy, interior, ps);
         if (slots) slot = ldg(a.slot + (k0 * a.ny + j) * a.nxp + i);
         if (pm == 255 && active) mid = ldg(a.mat + (k0 * a.ny + j) * a.nxp + i);
-        pml_table<R, STRICT, false>(a, tab, i0, j0, G::TY, tid);
     }
     __syncthreads();
 
@@ -787,6 +792,7 @@ __global__ void __launch_bounds__(kBlockX * kBlockY, (kEBlocks<R, NAMAX, CLS>))
      * chunk's planes */
     if (a.ndft) dft_fold(a, a.enew, i, j, k0, k1);
     if (a.probe_rows) probe_fold(a, a.enew, a.hnew, i, j, k0, k1);
+    chain_leave(a.beside, tid);
 }
 
 } // namespace phpdev
