@@ -44,6 +44,7 @@ constexpr int kMaxChunk = 256;      /* steps per recorded graph */
  * 512 steps are enqueued ahead */
 constexpr int kListChunk = 64;
 constexpr int kProfKinds = PHP_PROFILE_KINDS; /* H sweep, E sweep, probe, DFT, ion pass, one-launch step */
+constexpr size_t kDirectSlice = 256 << 10; /* bytes of a slice that its gather writes to host memory itself */
 constexpr int kProbeCap = 8192;     /* probe rows held on the device */
 constexpr double kEpsInf = 20.0;    /* EPS_INF, fdtd.c:202 */
 /* The FP32 path keeps the lattice state as 2^48 r and 2^48 v: early in a
@@ -253,7 +254,6 @@ struct php_ctx {
     };
     FrameSlot frames[PHP_FRAME_SLOTS];
     int32_t frame_next = 0;
-    FrameHead* frame_head_dev = nullptr;
     int32_t probe_t0 = 0;        /* step of the last probe read (rows pending = t - probe_t0) */
 };
 
@@ -2278,12 +2278,12 @@ static int relayout_step_inputs(php_ctx* ctx)
 }
 
 template <typename R>
-static void launch_gather_plane(php_ctx* ctx, int comp, int axis, int pos, bool f32)
+static void launch_gather_plane(php_ctx* ctx, int comp, int axis, int pos, bool f32, void* out)
 {
     const Fields<R> f = make_fields<R>(ctx);
     const DView<R> dv = make_dview<R>(ctx);
-    if (f32) gather_plane<R, float><<<296, 256, 0, ctx->stream>>>(f, dv, comp, axis, pos, ctx->nx, ctx->ny, ctx->nz, ctx->nxp, (float*)ctx->scratch);
-    else gather_plane<R, double><<<296, 256, 0, ctx->stream>>>(f, dv, comp, axis, pos, ctx->nx, ctx->ny, ctx->nz, ctx->nxp, (double*)ctx->scratch);
+    if (f32) gather_plane<R, float><<<296, 256, 0, ctx->stream>>>(f, dv, comp, axis, pos, ctx->nx, ctx->ny, ctx->nz, ctx->nxp, (float*)out);
+    else gather_plane<R, double><<<296, 256, 0, ctx->stream>>>(f, dv, comp, axis, pos, ctx->nx, ctx->ny, ctx->nz, ctx->nxp, (double*)out);
 }
 
 /* Fills pinned buffer b with the per-step inputs (source values, DFT
@@ -2333,13 +2333,14 @@ static int64_t point_index(const php_ctx* ctx, const int32_t* p)
 }
 
 template <typename R>
-static void launch_frame_gather(php_ctx* ctx, const DiagPartial* fin, int has_point, int64_t pc, int64_t cc)
+static void launch_frame_gather(php_ctx* ctx, const DiagPartial* parts, int nparts, int has_point, int64_t pc, int64_t cc,
+                                const double* rows, int64_t nrows, int row_len, double* rows_out, FrameHead* head)
 {
     frame_gather<R><<<1, 256, 0, ctx->stream>>>(make_fields<R>(ctx), make_dview<R>(ctx), ctx->mat, ctx->slot, (const MatCoef<R>*)ctx->mc, (const R*)ctx->r,
                                                  (const R*)ctx->v, ctx->rv_unit, ctx->nslot, ctx->nx, ctx->ny, ctx->nz, ctx->nxp,
-                                                 ctx->n3max, fin, has_point, pc, cc,
-                                                 ctx->probe ? ctx->probe_count : nullptr, ctx->err_flag,
-                                                 ctx->frame_head_dev);
+                                                 ctx->n3max, parts, nparts, has_point, pc, cc,
+                                                 ctx->probe ? ctx->probe_count : nullptr, rows, nrows, row_len, rows_out,
+                                                 ctx->err_flag, head);
 }
 
 extern "C" {
@@ -2602,8 +2603,8 @@ static int read_slice_impl(php_ctx* ctx, int32_t comp, char axis, int32_t positi
     size_t n;
     int rc = slice_geom(ctx, comp, axis, position, ax, pos, n);
     if (rc) return rc;
-    if (ctx->prec == PHP_PREC_FP32) launch_gather_plane<float>(ctx, comp, ax, pos, f32);
-    else launch_gather_plane<double>(ctx, comp, ax, pos, f32);
+    if (ctx->prec == PHP_PREC_FP32) launch_gather_plane<float>(ctx, comp, ax, pos, f32, ctx->scratch);
+    else launch_gather_plane<double>(ctx, comp, ax, pos, f32, ctx->scratch);
     CK(cudaGetLastError());
     const size_t bytes = n * (f32 ? sizeof(float) : sizeof(double));
     CK(cudaMemcpyAsync(ctx->host_stage, ctx->scratch, bytes, cudaMemcpyDeviceToHost, ctx->stream));
@@ -2729,13 +2730,13 @@ int php_read_cell_state(php_ctx* ctx, int32_t i, int32_t j, int32_t k, int32_t* 
     return PHP_OK;
 }
 
-/* Enqueues the two diagnostics passes; the result lands in *fin (scratch). */
-static int enqueue_diag(php_ctx* ctx, DiagPartial** fin_out)
+/* Enqueues the first diagnostics pass; *blocks_out partials in *part_out (scratch). */
+static int enqueue_diag(php_ctx* ctx, DiagPartial** part_out, int* blocks_out)
 {
-    const int blocks = 148 * 4;
+    const int blocks = (int)std::min<int64_t>(148 * 8, std::max<int64_t>(((int64_t)ctx->ny * ctx->nz + 15) / 16, (ctx->nslot + 1023) / 1024));
     DiagPartial* part = (DiagPartial*)ctx->scratch;
-    DiagPartial* fin = part + blocks;
-    *fin_out = fin;
+    *part_out = part;
+    *blocks_out = blocks;
     if (ctx->prec == PHP_PREC_FP32) {
         diag_pass1<float><<<blocks, 256, 0, ctx->stream>>>(make_fields<float>(ctx), ctx->nx, ctx->ny, ctx->nz, ctx->nxp, (const float*)ctx->r,
                                                            ctx->rv_unit, ctx->any_atoms ? ctx->nslot : 0, ctx->slot_cell, ctx->slot_n3,
@@ -2745,7 +2746,6 @@ static int enqueue_diag(php_ctx* ctx, DiagPartial** fin_out)
                                                             ctx->rv_unit, ctx->any_atoms ? ctx->nslot : 0, ctx->slot_cell, ctx->slot_n3,
                                                             std::max(ctx->n3max, 1), part);
     }
-    diag_pass2<<<1, 256, 0, ctx->stream>>>(part, blocks, fin);
     CK(cudaGetLastError());
     return PHP_OK;
 }
@@ -2774,9 +2774,13 @@ static void decode_diag(const php_ctx* ctx, const DiagPartial& h, php_diag* out)
 int php_diagnostics(php_ctx* ctx, php_diag* out)
 {
     if (!ctx || !out) return PHP_ERR_INPUT;
-    DiagPartial* fin = nullptr;
-    int rc = enqueue_diag(ctx, &fin);
+    DiagPartial* part = nullptr;
+    int blocks = 0;
+    int rc = enqueue_diag(ctx, &part, &blocks);
     if (rc) return rc;
+    DiagPartial* fin = part + blocks;
+    diag_pass2<<<1, 256, 0, ctx->stream>>>(part, blocks, fin);
+    CK(cudaGetLastError());
     DiagPartial h;
     CK(cudaMemcpyAsync(ctx->host_stage, fin, sizeof(DiagPartial), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
@@ -2864,10 +2868,6 @@ int php_frame_begin(php_ctx* ctx, const php_frame_req* req, int32_t* ticket)
                      req->cell[2] >= ctx->nz))
         return fail(ctx, PHP_ERR_INPUT, "cell (%d,%d,%d) outside the grid", req->cell[0], req->cell[1], req->cell[2]);
     if (req->probe && !ctx->probe) return fail(ctx, PHP_ERR_STATE, "no probe set");
-    if (!ctx->frame_head_dev) {
-        int rc = dalloc(ctx, (void**)&ctx->frame_head_dev, sizeof(FrameHead));
-        if (rc) return rc;
-    }
     const int32_t tk = ctx->frame_next;
     php_ctx::FrameSlot& F = ctx->frames[tk % PHP_FRAME_SLOTS];
     /* the oldest frame must have been released (bounded wait) */
@@ -2895,29 +2895,33 @@ int php_frame_begin(php_ctx* ctx, const php_frame_req* req, int32_t* ticket)
     }
     if (!F.head || !F.slice) return fail(ctx, PHP_ERR_OOM, "page-locked host allocation failed");
 
-    DiagPartial* fin = nullptr;
+    DiagPartial* part = nullptr;
+    int nparts = 0;
     if (req->diag) {
-        int rc = enqueue_diag(ctx, &fin);
+        int rc = enqueue_diag(ctx, &part, &nparts);
         if (rc) return rc;
     }
     const int64_t pc = has_point ? point_index(ctx, req->point) : 0;
     const int64_t cc = has_cell ? point_index(ctx, req->cell) : -1;
-    if (ctx->prec == PHP_PREC_FP32) launch_frame_gather<float>(ctx, fin, has_point, pc, cc);
-    else launch_frame_gather<double>(ctx, fin, has_point, pc, cc);
+    /* many rows (a long interval, a large lattice) by a copy, ahead of the
+     * gather that resets their counter */
+    const double* rows_dev = req->probe ? ctx->probe_rows : nullptr;
+    const bool copy_rows = rows * row_len * (int64_t)sizeof(double) > 65536;
+    if (req->probe && copy_rows)
+        CK(cudaMemcpyAsync(F.rows, rows_dev, (size_t)rows * row_len * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+    double* rows_out = req->probe && !copy_rows ? F.rows : nullptr;
+    if (ctx->prec == PHP_PREC_FP32) launch_frame_gather<float>(ctx, part, nparts, has_point, pc, cc, rows_dev, rows, row_len, rows_out, F.head);
+    else launch_frame_gather<double>(ctx, part, nparts, has_point, pc, cc, rows_dev, rows, row_len, rows_out, F.head);
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(F.head, ctx->frame_head_dev, sizeof(FrameHead), cudaMemcpyDeviceToHost, ctx->stream));
+    if (req->probe) ctx->probe_t0 = ctx->t;
     if (req->slice_comp >= 0) {
-        if (ctx->prec == PHP_PREC_FP32) launch_gather_plane<float>(ctx, req->slice_comp, ax, pos, true);
-        else launch_gather_plane<double>(ctx, req->slice_comp, ax, pos, true);
+        /* a small slice straight into the page-locked buffer, a large one by a copy */
+        const bool direct = slice_n * sizeof(float) <= kDirectSlice;
+        float* dst = direct ? F.slice : (float*)ctx->scratch;
+        if (ctx->prec == PHP_PREC_FP32) launch_gather_plane<float>(ctx, req->slice_comp, ax, pos, true, dst);
+        else launch_gather_plane<double>(ctx, req->slice_comp, ax, pos, true, dst);
         CK(cudaGetLastError());
-        CK(cudaMemcpyAsync(F.slice, ctx->scratch, slice_n * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
-    }
-    if (req->probe) {
-        if (rows > 0)
-            CK(cudaMemcpyAsync(F.rows, ctx->probe_rows, (size_t)rows * row_len * sizeof(double), cudaMemcpyDeviceToHost,
-                               ctx->stream));
-        CK(cudaMemsetAsync(ctx->probe_count, 0, 2 * sizeof(int32_t), ctx->stream));
-        ctx->probe_t0 = ctx->t;
+        if (!direct) CK(cudaMemcpyAsync(F.slice, ctx->scratch, slice_n * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
     }
     CK(cudaEventRecord(F.done, ctx->stream));
     F.ticket = tk;
@@ -3007,20 +3011,18 @@ int php_dft_read(php_ctx* ctx, int32_t id, double* out, int32_t* nsamples)
     if (!ctx || !out) return PHP_ERR_INPUT;
     if (id < 0 || id >= (int)ctx->dft.size()) return fail(ctx, PHP_ERR_INPUT, "no DFT plane %d", id);
     const DftPlane& p = ctx->dft[id];
-    /* the device keeps [nfreq][ny][nx][2] (x fastest for the samplers);
-     * the caller gets [nfreq][nx][ny][2] */
-    const size_t nx = ctx->nx, ny = ctx->ny;
-    std::vector<double> dev((size_t)p.nfreq * nx * ny * 2);
-    CK(cudaMemcpyAsync(dev.data(), p.acc, dev.size() * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+    /* the device keeps [nfreq][ny][nx][2] (x fastest for the samplers); the
+     * caller gets [nfreq][nx][ny][2], transposed on the device (three planes
+     * of 512 x 512: 5 ms on the host) */
+    const int64_t total = (int64_t)p.nfreq * ctx->nx * ctx->ny, chunk = (int64_t)(ctx->scratch_bytes / sizeof(double2));
+    for (int64_t o = 0; o < total; o += chunk) {
+        const int64_t n = std::min(chunk, total - o);
+        dft_reorder<<<(unsigned)std::min<int64_t>((n + 255) / 256, 148 * 8), 256, 0, ctx->stream>>>((const double2*)p.acc, ctx->nx, ctx->ny, o, n,
+                                                                                      (double2*)ctx->scratch);
+        CK(cudaGetLastError());
+        CK(cudaMemcpyAsync(out + 2 * o, ctx->scratch, (size_t)n * sizeof(double2), cudaMemcpyDeviceToHost, ctx->stream));
+    }
     CK(cudaStreamSynchronize(ctx->stream));
-    for (size_t f = 0; f < (size_t)p.nfreq; f++)
-        for (size_t j = 0; j < ny; j++)
-            for (size_t i = 0; i < nx; i++) {
-                const double* src = &dev[((f * ny + j) * nx + i) * 2];
-                double* dst = out + ((f * nx + i) * ny + j) * 2;
-                dst[0] = src[0];
-                dst[1] = src[1];
-            }
     if (nsamples) *nsamples = p.nsamples;
     return PHP_OK;
 }

@@ -455,6 +455,19 @@ __global__ void dft_sample(const Fields<R> fld, const DView<R> dv, int comp, int
     }
 }
 
+/* Accumulators [nfreq][ny][nx] to elements o0 .. o0+n-1 of the caller's order
+ * [nfreq][nx][ny].  A plane's accumulators fit the L2, so the strided 16-byte
+ * reads cost no more than a tiled transpose would; the copy out bounds it. */
+__global__ void __launch_bounds__(256) dft_reorder(const double2* acc, int nx, int ny, int64_t o0, int64_t n, double2* out)
+{
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n; t += stride) {
+        const int64_t fi = (o0 + t) / ny, f = fi / nx;
+        const int j = (int)(o0 + t - fi * ny), i = (int)(fi - f * nx);
+        out[t] = acc[(f * ny + j) * nx + i];
+    }
+}
+
 /* The same samples taken by the E sweep (StepArgs::dft_*): after a block's z
  * march over planes k0 .. k1-1, each of its threads reads back the E or D
  * values it stored at cell (i, j) of every registered plane in that range
@@ -541,42 +554,69 @@ __device__ __forceinline__ void diag_merge(DiagPartial& a, const DiagPartial& b)
     }
 }
 
+/* The reference's loop-order key of coordinate q of pool slot s */
+__device__ __forceinline__ int64_t diag_key(const int64_t* slot_cell, int64_t s, int q, int ny, int nz, int nxp, int n3max)
+{
+    const int64_t c = slot_cell[s], jk = c / nxp;
+    const int i = (int)(c % nxp), j = (int)(jk % ny), k = (int)(jk / ny);
+    return (((int64_t)i * ny + j) * nz + k) * (int64_t)n3max + q;
+}
+
 /* Pass 1 over cells (|E|, |Ex|) and pool slots (|r|, times rv_unit); one
  * partial per block into scratch.  slot_cell maps a pool slot to its device
- * cell index. */
+ * cell index.  Bound by HBM: E once and r once.  The square root is taken of
+ * the largest sum (it rounds monotonically), the pool's cell is decoded only
+ * where a new maximum or a tie needs its key, rows are read 16 bytes per
+ * lane, and a slot's coordinates eight loads at a time: 1.6 GB of E (512 x 512
+ * x 256, FP64) or of r (16 atoms) took 0.8 ms with a root, a division by the
+ * row length and one load in flight per cell. */
 template <typename R>
 __global__ void __launch_bounds__(256) diag_pass1(const Fields<R> f, int nx, int ny, int nz, int nxp,
                                                   const R* r, double rv_unit, int64_t nslot, const int64_t* slot_cell,
                                                   const int32_t* slot_n3, int n3max, DiagPartial* scratch)
 {
     DiagPartial acc{0.0, 0.0, 0.0, INT64_MAX};
-    const int64_t ncell = (int64_t)nx * ny * nz;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < ncell; t += stride) {
-        const int i = (int)(t % nx);
-        const int64_t jk = t / nx;
-        const int64_t c = jk * nxp + i;
-        const double x = (double)f.ex[c], y = (double)f.ey[c], z = (double)f.ez[c];
-        const double e = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y)), __dmul_rn(z, z)));
-        acc.max_e = fmax(acc.max_e, e);
-        acc.max_ex = fmax(acc.max_ex, fabs(x));
-    }
-    for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < nslot; s += stride) {
-        const int n3 = slot_n3[s];
-        if (!n3) continue;
-        const int64_t c = slot_cell[s];
-        const int i = (int)(c % nxp);
-        const int64_t jk = c / nxp;
-        const int j = (int)(jk % ny), k = (int)(jk / ny);
-        const int64_t base = (((int64_t)i * ny + j) * nz + k) * (int64_t)n3max;
-        for (int q = 0; q < n3; ++q) {
-            const double rv = rv_unit * fabs((double)r[(int64_t)q * nslot + s]);
-            if (rv > acc.max_r || (rv == acc.max_r && rv > 0.0 && base + q < acc.key_r)) {
-                acc.max_r = rv;
-                acc.key_r = base + q;
+    constexpr int V = 16 / (int)sizeof(R);
+    struct alignas(16) Vec { R v[V]; };
+    const int lane = threadIdx.x & 31;
+    const int64_t rows = (int64_t)ny * nz, warps = (int64_t)gridDim.x * (blockDim.x / 32);
+    for (int64_t row = (int64_t)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32; row < rows; row += warps) {
+        const Vec* x = reinterpret_cast<const Vec*>(f.ex + row * nxp);
+        const Vec* y = reinterpret_cast<const Vec*>(f.ey + row * nxp);
+        const Vec* z = reinterpret_cast<const Vec*>(f.ez + row * nxp);
+#pragma unroll 2
+        for (int t = lane; t < nxp / V; t += 32) {
+            const Vec a = x[t], b = y[t], c = z[t];
+#pragma unroll
+            for (int q = 0; q < V; ++q) {
+                if (t * V + q >= nx) continue; /* padding */
+                const double u = (double)a.v[q], v = (double)b.v[q], w = (double)c.v[q];
+                acc.max_e = fmax(acc.max_e, __dadd_rn(__dadd_rn(__dmul_rn(u, u), __dmul_rn(v, v)), __dmul_rn(w, w)));
+                acc.max_ex = fmax(acc.max_ex, fabs(u));
             }
         }
     }
+    acc.max_e = __dsqrt_rn(acc.max_e);
+    R best = R(0); /* |r| as stored */
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < nslot; s += stride) {
+        const int n3 = slot_n3[s];
+        for (int q0 = 0; q0 < n3; q0 += 8) {
+            R v[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) v[q] = q0 + q < n3 ? r[(int64_t)(q0 + q) * nslot + s] : R(0);
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const R m = v[q] < R(0) ? -v[q] : v[q];
+                if (m >= best && m > R(0)) {
+                    const int64_t key = diag_key(slot_cell, s, q0 + q, ny, nz, nxp, n3max);
+                    if (m > best || key < acc.key_r) acc.key_r = key;
+                    best = m;
+                }
+            }
+        }
+    }
+    acc.max_r = rv_unit * (double)best;
     __shared__ DiagPartial sh[256];
     sh[threadIdx.x] = acc;
     __syncthreads();
@@ -587,7 +627,9 @@ __global__ void __launch_bounds__(256) diag_pass1(const Fields<R> f, int nx, int
     if (threadIdx.x == 0) scratch[blockIdx.x] = sh[0];
 }
 
-__global__ void __launch_bounds__(256) diag_pass2(const DiagPartial* scratch, int n, DiagPartial* out)
+/* the partials of pass 1 reduced by one block of 256 threads; every thread
+ * gets the result */
+__device__ __forceinline__ DiagPartial diag_reduce(const DiagPartial* scratch, int n)
 {
     DiagPartial acc{0.0, 0.0, 0.0, INT64_MAX};
     for (int t = threadIdx.x; t < n; t += blockDim.x) diag_merge(acc, scratch[t]);
@@ -598,17 +640,23 @@ __global__ void __launch_bounds__(256) diag_pass2(const DiagPartial* scratch, in
         if ((int)threadIdx.x < w) diag_merge(sh[threadIdx.x], sh[threadIdx.x + w]);
         __syncthreads();
     }
-    if (threadIdx.x == 0) *out = sh[0];
+    return sh[0];
+}
+
+__global__ void __launch_bounds__(256) diag_pass2(const DiagPartial* scratch, int n, DiagPartial* out)
+{
+    const DiagPartial d = diag_reduce(scratch, n);
+    if (threadIdx.x == 0) *out = d;
 }
 
 /* ---------------------------------------------------------- output frames */
 
 constexpr int kFrameMaxN3 = 192; /* 3 N for N <= 64 atoms */
 
-/* The small part of an output frame (php_frame_begin), gathered on the
- * device and copied to page-locked host memory in one piece. */
+/* The small part of an output frame (php_frame_begin), written by the device
+ * into page-locked host memory. */
 struct FrameHead {
-    DiagPartial diag;                                       /* diag_pass2 result */
+    DiagPartial diag;                                       /* diagnostics */
     double diag_point[9];                                   /* fields at the max |r| cell */
     double diag_r[kFrameMaxN3], diag_v[kFrameMaxN3];        /* r, v there */
     double point[9];                                        /* fields at the requested point */
@@ -642,21 +690,24 @@ __device__ __forceinline__ void frame_cell(const Fields<R>& f, const DView<R>& d
     }
 }
 
-/* One block.  fin: the diagnostics of this frame (nullptr: none); the
- * point's device index (k may be -1 or nz, the halo planes; has_point 0:
- * none) and the cell's (-1: none); probe_count: the probe row counter
- * (nullptr: no probe).  Thread 0 writes every natom field. */
+/* One block of 256 threads.  parts: the partials of this frame's diagnostics
+ * (nullptr: none); the point's device index (k may be -1 or nz, the halo
+ * planes; has_point 0: none) and the cell's (-1: none); probe_count: the probe
+ * row counter (nullptr: no probe), reset where `rows` (nrows of them) go with
+ * the frame.  head and rows_out are page-locked host memory, written over
+ * PCIe: a frame of a small grid is a few launches, and a copy or a memset
+ * costs as much as one (32^3 grid: frame 69 us with three copies, a memset and
+ * the reduction in a launch of its own).  Thread 0 writes every natom field. */
 template <typename R>
-__global__ void frame_gather(const Fields<R> f, const DView<R> dv, const uint8_t* mat, const int32_t* slot, const MatCoef<R>* mc,
-                             const R* r, const R* v, double rv_unit, int64_t nslot, int nx, int ny, int nz, int nxp,
-                             int n3max,
-                             const DiagPartial* fin, int has_point, int64_t point_c, int64_t cell_c,
-                             const int32_t* probe_count,
+__global__ void __launch_bounds__(256) frame_gather(const Fields<R> f, const DView<R> dv, const uint8_t* mat, const int32_t* slot,
+                             const MatCoef<R>* mc, const R* r, const R* v, double rv_unit, int64_t nslot, int nx, int ny, int nz,
+                             int nxp, int n3max, const DiagPartial* parts, int nparts, int has_point, int64_t point_c,
+                             int64_t cell_c, int32_t* probe_count, const double* rows, int64_t nrows, int row_len, double* rows_out,
                              const int32_t* err, FrameHead* head)
 {
     const int t = threadIdx.x;
-    if (fin) {
-        const DiagPartial d = *fin;
+    if (parts) {
+        const DiagPartial d = diag_reduce(parts, nparts);
         if (t == 0) {
             head->diag = d;
             head->diag_natom = 0;
@@ -681,9 +732,12 @@ __global__ void frame_gather(const Fields<R> f, const DView<R> dv, const uint8_t
         frame_cell<R>(f, dv, mat, slot, mc, r, v, rv_unit, nslot, cell_c, cell_c, nullptr, head->cell_r, head->cell_v,
                       &head->cell_natom);
     }
+    if (rows_out)
+        for (int64_t q = t; q < nrows * row_len; q += blockDim.x) rows_out[q] = rows[q];
     if (t == 0) {
         head->probe_count[0] = probe_count ? probe_count[0] : 0;
         head->probe_count[1] = probe_count ? probe_count[1] : 0;
+        if (rows) probe_count[0] = probe_count[1] = 0;
         head->err = *err;
     }
 }

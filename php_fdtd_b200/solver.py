@@ -377,7 +377,7 @@ class Simulation:
         out = np.empty((nf, self.nx, self.ny, 2), dtype=np.float64)
         ns = C.c_int32()
         self._ck(self._lib.php_dft_read(self._ctx, pid, out.ctypes.data_as(C.POINTER(C.c_double)), C.byref(ns)))
-        return out[..., 0] + 1j * out[..., 1], ns.value
+        return out.view(np.complex128)[..., 0], ns.value
 
     @property
     def memory_bytes(self) -> int:
