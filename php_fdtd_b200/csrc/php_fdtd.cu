@@ -839,7 +839,8 @@ static void launch_ions(php_ctx* ctx)
     a.dfrag = (const double*)ctx->ion_dfrag;
     a.bsplit = (const uint32_t*)ctx->ion_bsplit;
     a.nslot = ctx->nslot;
-    a.ntiles = (int32_t)((ctx->nslot + kIonTile - 1) / kIonTile);
+    const int tile = ctx->ion_pipe ? ion_tile<R>() : kIonTile;
+    a.ntiles = (int32_t)((ctx->nslot + tile - 1) / tile);
     a.dt = ctx->d.dt;
     a.err = ctx->err_flag;
     cudaStream_t st = ctx->stream;
@@ -851,16 +852,16 @@ static void launch_ions(php_ctx* ctx)
     ion_pipe<R, NP, S><<<grid, IonPipe<R, NP, S>::THREADS, IonPipe<R, NP, S>::SMEM, st>>>(a, ctx->ion_maps, n3)
         if constexpr (sizeof(R) == 4) {
             switch (ctx->ion_np) {
-            case 16: PHP_ION_PIPE(16, 3); break;
-            case 32: PHP_ION_PIPE(32, 3); break;
-            case 48: PHP_ION_PIPE(48, 3); break;
-            default: PHP_ION_PIPE(64, 2); break;
+            case 16: PHP_ION_PIPE(16, 6); break;
+            case 32: PHP_ION_PIPE(32, 6); break;
+            case 48: PHP_ION_PIPE(48, 4); break;
+            default: PHP_ION_PIPE(64, 3); break;
             }
         } else {
             switch (ctx->ion_np) {
-            case 16: PHP_ION_PIPE(16, 2); break;
-            case 32: PHP_ION_PIPE(32, 2); break;
-            default: PHP_ION_PIPE(48, 2); break;
+            case 16: PHP_ION_PIPE(16, 6); break;
+            case 32: PHP_ION_PIPE(32, 6); break;
+            default: PHP_ION_PIPE(48, 4); break;
             }
         }
 #undef PHP_ION_PIPE
@@ -1449,16 +1450,17 @@ static int setup_ion_pass(php_ctx* ctx, const std::vector<MatD>& mats, const std
     ctx->ion_pipe = ctx->prec == PHP_PREC_FP32 ? np <= 64 : np <= 48;
     if (ctx->ion_pipe) {
         const CUtensorMapDataType dt = ctx->prec == PHP_PREC_FP32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64;
-        rc = encode_map(ctx, &ctx->ion_maps.r, ctx->r, dt, rs, (uint64_t)ctx->nslot, (uint64_t)n3, 1, kIonTile, (uint32_t)n3);
-        if (!rc) rc = encode_map(ctx, &ctx->ion_maps.v, ctx->v, dt, rs, (uint64_t)ctx->nslot, (uint64_t)n3, 1, kIonTile, (uint32_t)n3);
+        const uint32_t cells = ctx->prec == PHP_PREC_FP32 ? ion_tile<float>() : ion_tile<double>();
+        rc = encode_map(ctx, &ctx->ion_maps.r, ctx->r, dt, rs, (uint64_t)ctx->nslot, (uint64_t)n3, 1, cells, (uint32_t)n3);
+        if (!rc) rc = encode_map(ctx, &ctx->ion_maps.v, ctx->v, dt, rs, (uint64_t)ctx->nslot, (uint64_t)n3, 1, cells, (uint32_t)n3);
         if (rc) return rc;
         cudaError_t e;
         if (ctx->prec == PHP_PREC_FP32)
-            e = np == 16 ? ion_pipe_attr<float, 16, 3>() : np == 32 ? ion_pipe_attr<float, 32, 3>()
-              : np == 48 ? ion_pipe_attr<float, 48, 3>() : ion_pipe_attr<float, 64, 2>();
+            e = np == 16 ? ion_pipe_attr<float, 16, 6>() : np == 32 ? ion_pipe_attr<float, 32, 6>()
+              : np == 48 ? ion_pipe_attr<float, 48, 4>() : ion_pipe_attr<float, 64, 3>();
         else
-            e = np == 16 ? ion_pipe_attr<double, 16, 2>() : np == 32 ? ion_pipe_attr<double, 32, 2>()
-                         : ion_pipe_attr<double, 48, 2>();
+            e = np == 16 ? ion_pipe_attr<double, 16, 6>() : np == 32 ? ion_pipe_attr<double, 32, 6>()
+                         : ion_pipe_attr<double, 48, 4>();
         if (e != cudaSuccess) return fail(ctx, PHP_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     }
     return PHP_OK;
@@ -1936,10 +1938,10 @@ static int create_impl(const php_desc* desc, php_ctx* ctx)
         if (rc) return rc;
     }
     /* the one-launch step (he_sweep_tma) on a whole domain in the fast
-     * modes, with PHP_FUSED=1 at create: it moves 12 % fewer bytes per step
-     * than the two sweeps but measured slower on B200 (occupancy: E and H
-     * with their halos in the stage ring, 80-125 registers), so the two
-     * sweeps are the default */
+     * modes, with PHP_FUSED=1 at create: it moves a third fewer field words
+     * than the two sweeps but measured slower (all classes in one kernel
+     * spill: 256^3 tip 517-680 us FP64 against 495), so the two sweeps, with
+     * the interior launch on large domains, are the default */
     {
         const char* fv = getenv("PHP_FUSED");
         ctx->fused = ctx->prec != PHP_PREC_FP64_STRICT && ctx->z_off == 0 && ctx->nz_glob == nz && fv && !strcmp(fv, "1");

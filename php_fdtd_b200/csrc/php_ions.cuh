@@ -17,16 +17,17 @@
  * step.  The arithmetic is the reference's; only its rounding order differs
  * from the fused form (FP64: within 1e-10 of the reference).
  *
- *  ion_pipe       the pass proper: a TMA-fed ring of pool tiles, two
+ *  ion_pipe       the pass proper: a TMA-fed ring of pool tiles, three
  *                 consumer warpgroups.  FP32 (mixed path) on the 5th-generation
- *                 tensor cores: per 128-cell tile, r is split into bf16 hi + lo,
+ *                 tensor cores: per 128-cell tile, r is split into bf16 hi + lo
+ *                 (kept in tensor memory),
  *                 DMM likewise (host), and D = r_hi DMM_hi^T + r_hi DMM_lo^T +
  *                 r_lo DMM_hi^T accumulates in FP32 in tensor memory
  *                 (tcgen05.mma kind::f16, M = 128, N = K = 3N padded to 16);
  *                 the epilogue reads D with tcgen05.ld and does the update.
  *                 The dropped r_lo DMM_lo term and the bf16 representation
  *                 leave about 2^-17 relative error in DMM . r.  FP64 (fast
- *                 plain path): FMA chains against DMM in shared memory.
+ *                 plain path): the FP64 tensor path.
  *  ion_update_cc  plain loads, FP64, one cell per thread: used where the
  *                 FP64 ring does not fit in shared memory (3N > 48).
  */
@@ -167,50 +168,69 @@ __device__ __forceinline__ uint32_t bf16x2_bits(__nv_bfloat16 lo_half, __nv_bflo
 
 /* ------------------------------------------------- pipelined ion pass
  *
- * One CTA per SM, persistent over 128-cell tiles.  Warp 8 streams the r
- * and v tiles of the pool (box 128 cells x 3N, cp.async.bulk.tensor, no
+ * One CTA per SM, persistent over tiles of 128 (FP32) or 64 (FP64) cells.
+ * Warp 8 streams the r and v tiles of the pool (cp.async.bulk.tensor, no
  * multicast) and the tiles' slot indices (cp.async.bulk) into a ring of S
- * stages; two consumer warpgroups take alternate tiles, so that one group's
- * tensor-core round trip or E gather overlaps the other's epilogue.  The
- * updated r, v go back from the stage with a tensor store.  FP32: DMM . r as
- * BF16 x 3 on tcgen05 (each group its own A buffers and TMEM columns); FP64:
- * CUDA-core FMA chains against DMM in shared memory.
+ * stages; three consumer warpgroups take tiles in turn, so that one group's
+ * contraction overlaps the others' updates.  The updated r, v go back from the
+ * stage with a tensor store.  FP32: DMM . r as BF16 x 3 on tcgen05, A (the
+ * cells' r, hi and lo) from tensor memory; FP64: mma.sync m8n8k4 (there is no
+ * f64 kind of tcgen05).
+ *
+ * FP32 is bound by HBM, FP64 by the FP64 MMAs and the update, which the groups
+ * overlap.  4.2 M cells of 16 atoms (256 x 256 x 64), FP32 3.38 GB, FP64 6.75
+ * GB: two groups, three FP32 stages with A in shared memory (one 8-warp group
+ * and two stages of 128 cells in FP64) took 681 and 1354 us; A in tensor
+ * memory and the fourth stage that it makes room for 656; the third group
+ * 542 and 1206 (0.95 and 0.86 of the copy bandwidth).  Without the
+ * contraction or without the update two groups took 580 and 1150.  FP64 boxes
+ * of 16 cells, swizzled, have a quarter of the bank conflicts, but 128-byte
+ * rows cost the copies more than that (1420 us with or without the compute).
  */
 struct IonMaps {
-    CUtensorMap r, v; /* pool [3N][ns] as (x = slot, y = coordinate), box 128 x 3N */
+    CUtensorMap r, v; /* pool [3N][ns] as (x = slot, y = coordinate), box of a tile x 3N */
 };
 
-template <int NP>
-__host__ __device__ constexpr int ion_cols() { return NP <= 32 ? 32 : 64; }
+/* cells of one tile of the ring */
+template <typename R>
+__host__ __device__ constexpr int ion_tile() { return sizeof(R) == 4 ? kIonTile : kIonTile / 2; }
 
 template <typename R, int NP, int S>
 struct IonPipe {
     static constexpr bool TC = sizeof(R) == 4;
-    /* consumer groups: FP32 two groups of 128 threads take alternate tiles
-     * (one accumulator row per thread); FP64 one group of 256 threads takes
-     * each tile, so that with two stages one tile loads while one computes */
-    static constexpr int CONSUMERS = 2 * kIonTile, THREADS = CONSUMERS + 32;
-    static constexpr int GT = TC ? kIonTile : 2 * kIonTile, GROUPS = CONSUMERS / GT;
-    static constexpr int CELLS_PER_WARP = kIonTile / (GT / 32);  /* FP64: 16 */
-    static_assert(CONSUMERS % GT == 0 && GT % kIonTile == 0 && CELLS_PER_WARP % 16 == 0, "consumer layout");
-    static constexpr uint32_t BOX = kIonTile * NP * sizeof(R);      /* one array's tile, NP rows */
-    /* per stage: r, v, then the slots' cell offsets (int64, 1024 B), atom
-     * coordinate counts (int32, 512 B) and material ids (uint8, 128 B) */
-    static constexpr uint32_t IDX = 2048;
-    /* then the crystal-frame inputs: Ex, Ey, Ez of the tile's cells, gathered
-     * by the producer warp with cp.async */
-    static constexpr uint32_t E_OFF = 2 * BOX + IDX;
-    static constexpr uint32_t EB = 3 * kIonTile * sizeof(R);
-    static constexpr uint32_t STAGE = 2 * BOX + IDX + EB;
-    static constexpr uint32_t A_BYTES = kIonTile * NP * 2;           /* bf16 rows of one group */
+    static constexpr int TILE = ion_tile<R>();
+    /* consumer groups of 128 threads take tiles in turn: FP32 one accumulator
+     * row (cell) per thread, FP64 16 cells per warp */
+    static constexpr int GT = 128, GROUPS = 3, CONSUMERS = GROUPS * GT, THREADS = CONSUMERS + 32;
+    static_assert(TC ? TILE == GT : TILE == 16 * (GT / 32), "consumer layout");
+    static constexpr uint32_t BOX = TILE * NP * sizeof(R);           /* one array's tile, NP rows */
+    static constexpr uint32_t STAGE = 2 * BOX;                       /* r, v */
+    /* per stage, apart: the slots' cell offsets (int64), atom coordinate counts
+     * (int32) and material ids (uint8), then Ex, Ey, Ez of the tile's cells,
+     * gathered by the producer warp with cp.async */
+    static constexpr uint32_t N3_OFF = 8 * TILE, MAT_OFF = 12 * TILE, E_OFF = 16 * TILE;
+    static constexpr uint32_t AUX = E_OFF + 3 * TILE * sizeof(R);
     static constexpr uint32_t B_BYTES = NP * NP * 2;
     /* FP64: DMM, -QeZM (the E step) and QeZV^T (P_ion) as m8n8k4 B fragments */
     static constexpr uint32_t FRAG_E = NP * NP, FRAG_P = FRAG_E + (NP / 8) * 32, FRAG_N = FRAG_P + (NP / 4) * 32;
-    static constexpr uint32_t OPS = TC ? GROUPS * 2 * A_BYTES + 2 * B_BYTES : FRAG_N * 8;
+    static constexpr uint32_t OPS = TC ? 2 * B_BYTES : FRAG_N * 8;
     /* FP32: the lattice's QeZV, QeZM (9N each, 9N <= 3 NP) */
     static constexpr uint32_t COEF = TC ? 2 * 3 * NP * sizeof(R) : 0;
-    static constexpr uint32_t SMEM = 1024 + S * STAGE + OPS + COEF + 256;
+    static constexpr uint32_t SMEM = 1024 + S * (STAGE + AUX) + OPS + COEF + 256;
+    /* FP32, columns of tensor memory: a group's accumulator, then its A rows
+     * as bf16 pairs (hi, lo) */
+    static constexpr int A_COL = NP <= 32 ? 32 : 64, GCOLS = (A_COL + NP + 31) / 32 * 32;
+    static constexpr int COLS = GROUPS * GCOLS <= 256 ? 256 : 512; /* allocated: a power of two */
+    static_assert(GROUPS * GCOLS <= COLS, "tensor memory of one SM");
 };
+
+/* eight 32-bit columns of this warp's lanes (tcgen05.wait::st before use) */
+__device__ __forceinline__ void tmem_store_x8(uint32_t addr, const uint32_t (&d)[8])
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(addr), "r"(d[0]), "r"(d[1]), "r"(d[2]),
+                 "r"(d[3]), "r"(d[4]), "r"(d[5]), "r"(d[6]), "r"(d[7])
+                 : "memory");
+}
 
 __device__ __forceinline__ void named_sync(int id, int n)
 {
@@ -283,11 +303,13 @@ __global__ void __launch_bounds__(IonPipe<R, NP, S>::THREADS, 1)
 {
     using P = IonPipe<R, NP, S>;
     static_assert(NP % 16 == 0 && NP >= 16 && NP <= 64, "3N padded to 16..64");
+    static_assert(P::STAGE % 128 == 0 && P::AUX % 16 == 0, "copy alignment");
     static_assert(P::SMEM <= 227u * 1024u, "shared memory of one CTA");
     extern __shared__ __align__(128) unsigned char dyn_smem[];
     unsigned char* base = dyn_smem + ((1024u - (smem_addr(dyn_smem) & 1023u)) & 1023u);
     unsigned char* stages = base;
-    unsigned char* ops = base + S * P::STAGE;
+    unsigned char* auxs = base + S * P::STAGE;
+    unsigned char* ops = auxs + S * P::AUX;
     R* coef = reinterpret_cast<R*>(ops + P::OPS);
     uint64_t* full = reinterpret_cast<uint64_t*>(ops + P::OPS + P::COEF);
     uint64_t* empty = full + S;
@@ -302,9 +324,8 @@ __global__ void __launch_bounds__(IonPipe<R, NP, S>::THREADS, 1)
      * the lattice's QeZV, QeZM (cells of other materials read global) */
     {
         const uint4* src = P::TC ? reinterpret_cast<const uint4*>(a.bsplit) : reinterpret_cast<const uint4*>(a.dfrag);
-        unsigned char* dst0 = P::TC ? ops + P::GROUPS * 2 * P::A_BYTES : ops;
-        const int n16 = (int)((P::TC ? 2 * P::B_BYTES : P::OPS) / 16);
-        uint4* dst = reinterpret_cast<uint4*>(dst0);
+        const int n16 = (int)(P::OPS / 16);
+        uint4* dst = reinterpret_cast<uint4*>(ops);
         for (int t = tid; t < n16; t += P::THREADS) dst[t] = src[t];
         if constexpr (P::TC)
             for (int t = tid; t < 6 * n3; t += P::THREADS) coef[t] = a.ion_coef[a.ion_off_ref + t];
@@ -312,7 +333,7 @@ __global__ void __launch_bounds__(IonPipe<R, NP, S>::THREADS, 1)
     if constexpr (P::TC) {
         if (warp == 0) {
             asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tmem_slot)),
-                         "r"(P::GROUPS * ion_cols<NP>()));
+                         "r"(P::COLS));
             asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
         }
     }
@@ -331,7 +352,7 @@ __global__ void __launch_bounds__(IonPipe<R, NP, S>::THREADS, 1)
     __syncthreads();
     if constexpr (P::TC) asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem0 = P::TC ? *tmem_slot : 0u;
-    const uint32_t tx_bytes = 2u * kIonTile * (uint32_t)n3 * (uint32_t)sizeof(R);
+    const uint32_t tx_bytes = 2u * P::TILE * (uint32_t)n3 * (uint32_t)sizeof(R);
     bool failed = false;
 
     if (warp == P::CONSUMERS / 32) {
@@ -342,7 +363,7 @@ __global__ void __launch_bounds__(IonPipe<R, NP, S>::THREADS, 1)
          * with one tensor store per array (the consumers never wait for it) */
         auto store_tile = [&](int kk) -> bool {
             if (!mbar_wait(&empty[kk % S], (kk / S) & 1)) return false;
-            const int x = ((int)blockIdx.x + kk * (int)gridDim.x) * kIonTile;
+            const int x = ((int)blockIdx.x + kk * (int)gridDim.x) * P::TILE;
             unsigned char* b = stages + (kk % S) * P::STAGE;
             tma_store_3d(&maps.r, b, x, 0, 0);
             tma_store_3d(&maps.v, b + P::BOX, x, 0, 0);
@@ -350,11 +371,11 @@ __global__ void __launch_bounds__(IonPipe<R, NP, S>::THREADS, 1)
             return true;
         };
         /* cell offsets of this lane's slots of tile kk (-1 past the pool) */
-        int64_t cells[kIonTile / 32];
+        int64_t cells[P::TILE / 32];
         auto fetch_cells = [&](int kk) {
-            const int64_t xk = (int64_t)((int)blockIdx.x + kk * (int)gridDim.x) * kIonTile;
+            const int64_t xk = (int64_t)((int)blockIdx.x + kk * (int)gridDim.x) * P::TILE;
 #pragma unroll
-            for (int u = 0; u < kIonTile / 32; ++u) {
+            for (int u = 0; u < P::TILE / 32; ++u) {
                 const int64_t sl = xk + lane + 32 * u;
                 cells[u] = sl < a.nslot ? a.slot_cell[sl] : -1;
             }
@@ -371,30 +392,31 @@ __global__ void __launch_bounds__(IonPipe<R, NP, S>::THREADS, 1)
                 failed = true;
                 break;
             }
-            const int x = ((int)blockIdx.x + k * (int)gridDim.x) * kIonTile;
+            const int x = ((int)blockIdx.x + k * (int)gridDim.x) * P::TILE;
             unsigned char* b = stages + st * P::STAGE;
+            unsigned char* ab = auxs + st * P::AUX;
             if (lane == 0) {
                 /* slots left in this tile: a multiple of 32 (the pool is padded) */
-                const uint32_t nrem = (uint32_t)min((int64_t)kIonTile, a.nslot - x);
+                const uint32_t nrem = (uint32_t)min((int64_t)P::TILE, a.nslot - x);
                 mbar_arrive_expect_tx(&full[st], tx_bytes + nrem * 13u);
                 tma_load_3d(b, &maps.r, &full[st], x, 0, 0);
                 tma_load_3d(b + P::BOX, &maps.v, &full[st], x, 0, 0);
-                bulk_load(b + 2 * P::BOX, a.slot_cell + x, nrem * 8u, &full[st]);
-                bulk_load(b + 2 * P::BOX + 1024, a.slot_n3 + x, nrem * 4u, &full[st]);
-                bulk_load(b + 2 * P::BOX + 1536, a.slot_mat + x, nrem, &full[st]);
+                bulk_load(ab, a.slot_cell + x, nrem * 8u, &full[st]);
+                bulk_load(ab + P::N3_OFF, a.slot_n3 + x, nrem * 4u, &full[st]);
+                bulk_load(ab + P::MAT_OFF, a.slot_mat + x, nrem, &full[st]);
             }
             /* E^{n+1} of the tile's cells, gathered ahead like the rest of the
              * stage (padding slots repeat the last cell; slots past the pool
              * are not read); their cell offsets were read one tile ahead */
-            R* es = reinterpret_cast<R*>(b + P::E_OFF);
+            R* es = reinterpret_cast<R*>(ab + P::E_OFF);
 #pragma unroll
-            for (int u = 0; u < kIonTile / 32; ++u) {
+            for (int u = 0; u < P::TILE / 32; ++u) {
                 const int t = lane + 32 * u;
                 const int64_t c = cells[u];
                 if (c >= 0) {
                     cp_async_ca<sizeof(R)>(es + t, a.ex + c);
-                    cp_async_ca<sizeof(R)>(es + kIonTile + t, a.ey + c);
-                    cp_async_ca<sizeof(R)>(es + 2 * kIonTile + t, a.ez + c);
+                    cp_async_ca<sizeof(R)>(es + P::TILE + t, a.ey + c);
+                    cp_async_ca<sizeof(R)>(es + 2 * P::TILE + t, a.ez + c);
                 }
             }
             cp_async_arrive_noinc(&full[st]);
@@ -411,51 +433,52 @@ __global__ void __launch_bounds__(IonPipe<R, NP, S>::THREADS, 1)
         if (lane == 0) bulk_wait0(); /* stores complete before the CTA leaves */
     } else {
         /* ------------------------------------------------------ consumers */
-        const int g = tid / P::GT, gi = tid % P::GT, gt = gi & (kIonTile - 1), bar_id = 1 + g;
-        /* FP64: threads gi >= 128 take part in the contraction only */
-        const bool cell_thread = gi < kIonTile;
+        const int g = tid / P::GT, gi = tid % P::GT, gt = gi & (P::TILE - 1), bar_id = 1 + g;
+        /* FP64: threads gi >= 64 take part in the contraction only */
+        const bool cell_thread = gi < P::TILE;
         const int64_t ns = a.nslot;
         const R dt = R(a.dt);
-        unsigned char* Ahi = ops + g * 2 * P::A_BYTES;
-        unsigned char* Alo = Ahi + P::A_BYTES;
-        const unsigned char* Bhi = ops + P::GROUPS * 2 * P::A_BYTES;
+        const unsigned char* Bhi = ops;
         const unsigned char* Blo = Bhi + P::B_BYTES;
         const double* Bfrag = reinterpret_cast<const double*>(ops);
-        const uint32_t tmem = tmem0 + (uint32_t)(g * ion_cols<NP>());
+        const uint32_t tmem = tmem0 + (uint32_t)(g * P::GCOLS);
+        /* this warp's 32 lanes (rows, cells) of the group's A columns */
+        const uint32_t tmem_a = tmem + (uint32_t)P::A_COL, tmem_row = (uint32_t)((warp & 3) * 32) << 16;
         uint32_t mphase = 0;
         for (int k = g; k < mine; k += P::GROUPS) {
             const int st = k % S;
-            const int64_t s = (int64_t)((int)blockIdx.x + k * (int)gridDim.x) * kIonTile + gt;
+            const int64_t s = (int64_t)((int)blockIdx.x + k * (int)gridDim.x) * P::TILE + gt;
             const bool got = mbar_wait(&full[st], (k / S) & 1);
             if (named_sync_or(bar_id, P::GT, !got)) {
                 failed = true;
                 break;
             }
             unsigned char* sb = stages + st * P::STAGE;
+            unsigned char* ab = auxs + st * P::AUX;
             R* rs = reinterpret_cast<R*>(sb);
             R* vs = reinterpret_cast<R*>(sb + P::BOX);
-            const int n3c = (cell_thread && s < ns) ? reinterpret_cast<const int32_t*>(sb + 2 * P::BOX + 1024)[gt] : 0;
+            const int n3c = (cell_thread && s < ns) ? reinterpret_cast<const int32_t*>(ab + P::N3_OFF)[gt] : 0;
             R e0 = R(0), e1 = R(0), e2 = R(0);
             const MatCoef<R>* mp = nullptr;
             if (n3c) {
-                const R* es = reinterpret_cast<const R*>(sb + P::E_OFF);
-                mp = &a.mc[(sb + 2 * P::BOX + 1536)[gt]];
+                const R* es = reinterpret_cast<const R*>(ab + P::E_OFF);
+                mp = &a.mc[(ab + P::MAT_OFF)[gt]];
                 e0 = es[gt];
-                e1 = es[kIonTile + gt];
-                e2 = es[2 * kIonTile + gt];
+                e1 = es[P::TILE + gt];
+                e2 = es[2 * P::TILE + gt];
                 rot_fwd<false>(mp->flags, mp->cs, mp->sn, e0, e1, e2);
             }
             R p0 = R(0), p1 = R(0), p2 = R(0);
             const R* qv = n3c ? (mp->ion_off == a.ion_off_ref ? coef : a.ion_coef + mp->ion_off) : nullptr;
             const R* qm = n3c ? qv + 3 * n3c : nullptr;
             if constexpr (P::TC) {
-                /* A rows (this cell) as bf16 hi + lo */
+                /* this cell's row of A as bf16 hi + lo, 16 coordinates (8 columns) at a time */
 #pragma unroll
-                for (int kc = 0; kc < NP / 8; ++kc) {
-                    uint32_t h[4], l[4];
+                for (int kc = 0; kc < NP / 16; ++kc) {
+                    uint32_t h[8], l[8];
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const int q = kc * 8 + 2 * u;
+                    for (int u = 0; u < 8; ++u) {
+                        const int q = kc * 16 + 2 * u;
                         const float x0 = q < n3 ? (float)rs[q * kIonTile + gt] : 0.f;
                         const float x1 = q + 1 < n3 ? (float)rs[(q + 1) * kIonTile + gt] : 0.f;
                         const __nv_bfloat16 h0 = __float2bfloat16_rn(x0), h1 = __float2bfloat16_rn(x1);
@@ -464,35 +487,32 @@ __global__ void __launch_bounds__(IonPipe<R, NP, S>::THREADS, 1)
                         h[u] = bf16x2_bits(h0, h1);
                         l[u] = bf16x2_bits(l0, l1);
                     }
-                    const uint32_t off = umma_kmajor_off(gt, kc * 8, kIonTile);
-                    *reinterpret_cast<uint4*>(Ahi + off) = make_uint4(h[0], h[1], h[2], h[3]);
-                    *reinterpret_cast<uint4*>(Alo + off) = make_uint4(l[0], l[1], l[2], l[3]);
+                    tmem_store_x8(tmem_a + tmem_row + (uint32_t)(kc * 8), h);
+                    tmem_store_x8(tmem_a + tmem_row + (uint32_t)(NP / 2 + kc * 8), l);
                 }
-                fence_proxy_async_smem();
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 named_sync(bar_id, P::GT);
                 if (gt == 0) {
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t idesc = umma_idesc_bf16(kIonTile, NP);
-                    const uint32_t sa_hi = smem_addr(Ahi), sa_lo = smem_addr(Alo);
                     const uint32_t sb_hi = smem_addr(Bhi), sb_lo = smem_addr(Blo);
 #pragma unroll
                     for (int ks = 0; ks < NP / 16; ++ks) {
-                        const uint32_t ao = umma_kmajor_off(0, ks * 16, kIonTile), bo = umma_kmajor_off(0, ks * 16, NP);
-                        const uint64_t dah = umma_smem_desc(sa_hi + ao, kIonTile * 16, 128);
-                        const uint64_t dal = umma_smem_desc(sa_lo + ao, kIonTile * 16, 128);
+                        const uint32_t bo = umma_kmajor_off(0, ks * 16, NP);
+                        const uint32_t dah = tmem_a + (uint32_t)(ks * 8), dal = tmem_a + (uint32_t)(NP / 2 + ks * 8);
                         const uint64_t dbh = umma_smem_desc(sb_hi + bo, NP * 16, 128);
                         const uint64_t dbl = umma_smem_desc(sb_lo + bo, NP * 16, 128);
                         const uint32_t acc0 = ks > 0 ? 1u : 0u;
                         asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                                     " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-                                     ::"r"(tmem), "l"(dah), "l"(dbh), "r"(idesc), "r"(acc0));
+                                     " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
+                                     ::"r"(tmem), "r"(dah), "l"(dbh), "r"(idesc), "r"(acc0));
                         asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                                     " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-                                     ::"r"(tmem), "l"(dah), "l"(dbl), "r"(idesc), "r"(1u));
+                                     " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
+                                     ::"r"(tmem), "r"(dah), "l"(dbl), "r"(idesc), "r"(1u));
                         asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                                     " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-                                     ::"r"(tmem), "l"(dal), "l"(dbh), "r"(idesc), "r"(1u));
+                                     " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
+                                     ::"r"(tmem), "r"(dal), "l"(dbh), "r"(idesc), "r"(1u));
                     }
                     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                                      smem_addr(&mma_bar[g]))
@@ -513,7 +533,7 @@ __global__ void __launch_bounds__(IonPipe<R, NP, S>::THREADS, 1)
 #pragma unroll
                 for (int cb = 0; cb < NP; cb += 16) {
                     uint32_t d[16];
-                    const uint32_t taddr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)cb;
+                    const uint32_t taddr = tmem + tmem_row + (uint32_t)cb;
                     asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
                                  : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]),
                                    "=r"(d[7]), "=r"(d[8]), "=r"(d[9]), "=r"(d[10]), "=r"(d[11]), "=r"(d[12]), "=r"(d[13]),
@@ -545,27 +565,26 @@ __global__ void __launch_bounds__(IonPipe<R, NP, S>::THREADS, 1)
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             } else {
                 /* FP64: DMM . r on the FP64 tensor path (mma.sync m8n8k4).
-                 * Each thread leaves its cell's crystal-frame E and the
-                 * offset of its QeZV, QeZM in the stage; then each warp
-                 * takes its 32 cells, 16 at a time: the accumulators hold
-                 * (DMM . r)[cell][q] for two 8-cell rows and all NP columns,
-                 * and the lanes that hold a (cell, q) pair update that
-                 * coordinate's r and v in the stage. */
-                R* es = reinterpret_cast<R*>(sb + P::E_OFF);
-                int64_t* qoff = reinterpret_cast<int64_t*>(sb + 2 * P::BOX); /* slot cells, no longer read */
-                const int32_t* n3s = reinterpret_cast<const int32_t*>(sb + 2 * P::BOX + 1024);
+                 * Each cell's thread leaves its crystal-frame E and the offset
+                 * of its QeZV, QeZM in the stage; then each warp takes 16
+                 * cells: the accumulators hold (DMM . r)[cell][q] for two
+                 * 8-cell rows and all NP columns, and the lanes that hold a
+                 * (cell, q) pair update that coordinate's r and v in the
+                 * stage. */
+                R* es = reinterpret_cast<R*>(ab + P::E_OFF);
+                int64_t* qoff = reinterpret_cast<int64_t*>(ab); /* slot cells, no longer read */
+                const int32_t* n3s = reinterpret_cast<const int32_t*>(ab + P::N3_OFF);
                 if (cell_thread) {
                     es[gt] = e0;
-                    es[kIonTile + gt] = e1;
-                    es[2 * kIonTile + gt] = e2;
+                    es[P::TILE + gt] = e1;
+                    es[2 * P::TILE + gt] = e2;
                     qoff[gt] = n3c ? (mp->ion_off == a.ion_off_ref ? -1 : (int64_t)mp->ion_off) : 0;
                 }
                 named_sync(bar_id, P::GT);
                 const int lane = tid & 31, grp = lane >> 2, tig = lane & 3;
-                const int64_t x0 = (int64_t)((int)blockIdx.x + k * (int)gridDim.x) * kIonTile;
-#pragma unroll 1
-                for (int pass = 0; pass < P::CELLS_PER_WARP / 16; ++pass) {
-                    const int cb = (gi >> 5) * P::CELLS_PER_WARP + pass * 16;
+                const int64_t x0 = (int64_t)((int)blockIdx.x + k * (int)gridDim.x) * P::TILE;
+                const int cb = (gi >> 5) * 16;
+                {
                     int n3l[2];
                     bool lat = true;
 #pragma unroll
@@ -587,8 +606,8 @@ __global__ void __launch_bounds__(IonPipe<R, NP, S>::THREADS, 1)
                     for (int ks = 0; ks < NP / 4; ++ks) {
                         const int kk = ks * 4 + tig;
                         /* rows past 3N hold no data: A is zero there */
-                        const double a0 = kk < n3 ? (double)rs[kk * kIonTile + cb + grp] : 0.0;
-                        const double a1 = kk < n3 ? (double)rs[kk * kIonTile + cb + 8 + grp] : 0.0;
+                        const double a0 = kk < n3 ? (double)rs[kk * P::TILE + cb + grp] : 0.0;
+                        const double a1 = kk < n3 ? (double)rs[kk * P::TILE + cb + 8 + grp] : 0.0;
 #pragma unroll
                         for (int nt = 0; nt < NP / 8; ++nt) {
                             const double b = Bfrag[(ks * (NP / 8) + nt) * 32 + lane];
@@ -597,8 +616,8 @@ __global__ void __launch_bounds__(IonPipe<R, NP, S>::THREADS, 1)
                         }
                     }
                     if (fold) {
-                        const double a0 = tig < 3 ? (double)es[tig * kIonTile + cb + grp] : 0.0;
-                        const double a1 = tig < 3 ? (double)es[tig * kIonTile + cb + 8 + grp] : 0.0;
+                        const double a0 = tig < 3 ? (double)es[tig * P::TILE + cb + grp] : 0.0;
+                        const double a1 = tig < 3 ? (double)es[tig * P::TILE + cb + 8 + grp] : 0.0;
 #pragma unroll
                         for (int nt = 0; nt < NP / 8; ++nt) {
                             const double b = Bfrag[P::FRAG_E + nt * 32 + lane];
@@ -627,7 +646,7 @@ __global__ void __launch_bounds__(IonPipe<R, NP, S>::THREADS, 1)
                                     const int q = nt * 8 + 2 * t + j;
                                     if (live_me && q < n3) {
                                         const R acc_q = -(R)(me < 8 ? v0 : v1);
-                                        const int o = q * kIonTile + cme;
+                                        const int o = q * P::TILE + cme;
                                         const R vq = vs[o];
                                         rs[o] = rs[o] + (vq * dt + R(0.5) * acc_q * dt * dt);
                                         vs[o] = vq + acc_q * dt;
@@ -640,8 +659,8 @@ __global__ void __launch_bounds__(IonPipe<R, NP, S>::THREADS, 1)
 #pragma unroll 4
                         for (int ks = 0; ks < NP / 4; ++ks) {
                             const int kk = ks * 4 + tig;
-                            const double a0 = kk < n3 ? (double)rs[kk * kIonTile + cb + grp] : 0.0;
-                            const double a1 = kk < n3 ? (double)rs[kk * kIonTile + cb + 8 + grp] : 0.0;
+                            const double a0 = kk < n3 ? (double)rs[kk * P::TILE + cb + grp] : 0.0;
+                            const double a1 = kk < n3 ? (double)rs[kk * P::TILE + cb + 8 + grp] : 0.0;
                             const double b = Bfrag[P::FRAG_P + ks * 32 + lane];
                             dmma_8x8x4(pa[0][0], pa[0][1], a0, b);
                             dmma_8x8x4(pa[1][0], pa[1][1], a1, b);
@@ -655,8 +674,7 @@ __global__ void __launch_bounds__(IonPipe<R, NP, S>::THREADS, 1)
                             }
                             if (n3l[mt] && tig == 1) a.pr[2 * ns + sl] = (R)pa[mt][0];
                         }
-                        continue;
-                    }
+                    } else {
 #pragma unroll
                     for (int mt = 0; mt < 2; ++mt) {
                         const int cl = cb + 8 * mt + grp;
@@ -667,7 +685,7 @@ __global__ void __launch_bounds__(IonPipe<R, NP, S>::THREADS, 1)
                             const int64_t qo = qoff[cl];
                             const R* zv = a.ion_coef + (qo < 0 ? (int64_t)a.ion_off_ref : qo);
                             const R* zm = zv + 3 * n3l[mt];
-                            const R ex0 = es[cl], ex1 = es[kIonTile + cl], ex2 = es[2 * kIonTile + cl];
+                            const R ex0 = es[cl], ex1 = es[P::TILE + cl], ex2 = es[2 * P::TILE + cl];
 #pragma unroll
                             for (int nt = 0; nt < NP / 8; ++nt)
 #pragma unroll
@@ -677,7 +695,7 @@ __global__ void __launch_bounds__(IonPipe<R, NP, S>::THREADS, 1)
                                         const int at = q / 3, dd = q - 3 * at;
                                         const R acc_q = zm[at * 9 + dd] * ex0 + zm[at * 9 + 3 + dd] * ex1 +
                                                         zm[at * 9 + 6 + dd] * ex2 - (R)acc[mt][nt][j];
-                                        const int o = q * kIonTile + cl;
+                                        const int o = q * P::TILE + cl;
                                         const R vq = vs[o];
                                         const R rn = rs[o] + (vq * dt + R(0.5) * acc_q * dt * dt);
                                         rs[o] = rn;
@@ -701,6 +719,7 @@ __global__ void __launch_bounds__(IonPipe<R, NP, S>::THREADS, 1)
                             a.pr[ns + sl] = q1;
                             a.pr[2 * ns + sl] = q2;
                         }
+                    }
                     }
                 }
             }
@@ -727,7 +746,7 @@ __global__ void __launch_bounds__(IonPipe<R, NP, S>::THREADS, 1)
         if (warp == 0) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem0),
-                         "r"(P::GROUPS * ion_cols<NP>()));
+                         "r"(P::COLS));
         }
     }
 }
