@@ -997,7 +997,7 @@ def main():
             "dtype": {"fp64": "f64", "fp32": "f32", "fp64-strict": "f64"}[args.precision], "data": "synthetic",
             "config": {"workload": workload_name(args), "grid": [cfg.nx, cfg.ny, cfg.nz], "cells": r["V"],
                        "precision": args.precision, "parallelism": f"replicas x{ws}" if ws > 1 else "single domain",
-                       "l2": "state 9 fields x cells > L2 (126 MB); no flush needed",
+                       "l2": "state (E and H at least, 6 fields x cells) > L2 (126 MB); no flush needed",
                        "per_step": ("interior H + E launch, H and E sweeps of the rest + monitor probe + running DFT (1 plane)"
                                     if "step" in r["roofline"]["sweeps"] else
                                     "H sweep + fused D/source/E/ADE sweep + monitor probe + running DFT (1 plane)"),

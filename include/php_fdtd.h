@@ -182,7 +182,11 @@ int php_create_slab(const php_desc* desc, int32_t z0, int32_t nz_local, php_ctx*
  *   1  E, halo plane nz    (received from the slab above)
  *   2  H, plane nz-1       (sent to the slab above, before the E sweep)
  *   3  H, halo plane -1    (received from the slab below)
- * Each plane is plane_bytes long (nx padded, times ny, elements). */
+ * Each plane is plane_bytes long (nx padded, times ny, elements).  The
+ * addresses hold for the context's life: from the first call of this
+ * function, php_step_half or php_step_part on, it updates E and H in place
+ * (a large domain's interior launch, which alternates between two buffers,
+ * is given up). */
 int php_halo_planes(php_ctx* ctx, int32_t which, void** ptrs3, uint64_t* plane_bytes);
 /* Half of one time step, enqueued on the context's stream without a graph:
  * half 0 = the H sweep; half 1 = the D/E sweep, ion pass, probe and DFT
@@ -316,7 +320,9 @@ int php_dft_read(php_ctx* ctx, int32_t id, double* out, int32_t* nsamples);
 /* Device bytes held by the context. */
 int php_memory_bytes(const php_ctx* ctx, uint64_t* bytes);
 /* Device bytes php_create would allocate for this description (before any
- * php_dft_add / php_probe_set); needs no device.  Used for admission
+ * php_dft_add / php_probe_set) at most: the second E and H buffers of a large
+ * domain's interior launch are counted, though php_create goes without them
+ * where memory is short; needs no device.  Used for admission
  * against a memory budget. */
 int php_estimate_bytes(const php_desc* desc, uint64_t* bytes);
 /* Number of kernel launches enqueued by the last php_step call. */
@@ -340,10 +346,12 @@ int php_stream(const php_ctx* ctx, void** stream);
 /* Per-kernel timing.  While enabled, the recorded step graphs carry CUDA
  * events around every sweep kernel and php_step accumulates their device
  * time: ms[0] H sweep, ms[1] fused D/E sweep, ms[2] probe, ms[3] DFT,
- * ms[4] ion pass of many-atom cells, ms[5] the one-launch step (H, D and E
- * in one sweep, which replaces [0] and [1] where it runs), with the number
- * of launches of each in launches[] (both arrays hold PHP_PROFILE_KINDS
- * entries).  Enabling or disabling resets the sums. */
+ * ms[4] ion pass of many-atom cells, ms[5] the launch that updates H and E in
+ * one march (of a large domain's interior, with [0] and [1] taking the other
+ * blocks, or of the whole domain with PHP_FUSED=1), with the number of steps
+ * in which each ran in launches[] (the E sweep's class launches count as one;
+ * [3] counts its launches; both arrays hold PHP_PROFILE_KINDS entries).
+ * Enabling or disabling resets the sums. */
 #define PHP_PROFILE_KINDS 6
 int php_profile_enable(php_ctx* ctx, int32_t enable);
 int php_profile_read(php_ctx* ctx, double* ms, int64_t* launches);

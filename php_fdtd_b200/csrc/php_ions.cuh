@@ -169,7 +169,7 @@ __device__ __forceinline__ uint32_t bf16x2_bits(__nv_bfloat16 lo_half, __nv_bflo
 /* ------------------------------------------------- pipelined ion pass
  *
  * One CTA per SM, persistent over tiles of 128 (FP32) or 64 (FP64) cells.
- * Warp 8 streams the r and v tiles of the pool (cp.async.bulk.tensor, no
+ * The last warp streams the r and v tiles of the pool (cp.async.bulk.tensor, no
  * multicast) and the tiles' slot indices (cp.async.bulk) into a ring of S
  * stages; three consumer warpgroups take tiles in turn, so that one group's
  * contraction overlaps the others' updates.  The updated r, v go back from the

@@ -282,7 +282,8 @@ __device__ __forceinline__ int32_t ldg_nh(const int32_t* p)
  * launches further back, complete since the launch before it entered) waits at
  * its end instead, in chain_leave, so that its own completion still implies
  * that of all before it.  Launched without the attribute, both return at
- * once. */
+ * once.  Per step, plain launches and the chain: 32^3 7.6 -> 6.4 us, 96^3
+ * two-atom slab FP64 55 -> 50 us, FP32 34.4 -> 34.0 us; 256^3 unchanged. */
 __device__ __forceinline__ void chain_enter(int beside)
 {
     if (!beside) asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -569,7 +570,9 @@ __device__ __forceinline__ int64_t diag_key(const int64_t* slot_cell, int64_t s,
  * where a new maximum or a tie needs its key, rows are read 16 bytes per
  * lane, and a slot's coordinates eight loads at a time: 1.6 GB of E (512 x 512
  * x 256, FP64) or of r (16 atoms) took 0.8 ms with a root, a division by the
- * row length and one load in flight per cell. */
+ * row length and one load in flight per cell; a frame of 256 x 256 x 128 with
+ * 16 atoms in half the cells (1.8 GB FP64) takes 0.45 ms now, 0.04 of it
+ * without the diagnostics. */
 template <typename R>
 __global__ void __launch_bounds__(256) diag_pass1(const Fields<R> f, int nx, int ny, int nz, int nxp,
                                                   const R* r, double rv_unit, int64_t nslot, const int64_t* slot_cell,
