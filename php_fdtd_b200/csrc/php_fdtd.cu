@@ -945,7 +945,7 @@ static void launch_step_t(php_ctx* ctx, int s_local, int& launches)
             prof_mark(ctx, s_local, 5, 1);
             a.list = ctx->lists[1];
             prof_mark(ctx, s_local, 0, 0);
-            launch_chained(ctx, h_sweep_tma<R, STRICT>, dim3(ctx->nlist[1]), TmaGeom<R>::H_SMEM, a, ctx->maps, true);
+            launch_chained(ctx, h_sweep_tma<R, STRICT, true>, dim3(ctx->nlist[1]), TmaGeom<R>::H_SMEM, a, ctx->maps, true);
             prof_mark(ctx, s_local, 0, 1);
             TmaMaps me = ctx->maps;
             me.h_halo = ctx->maps_o.h_halo;
@@ -969,7 +969,7 @@ static void launch_step_t(php_ctx* ctx, int s_local, int& launches)
     if (grid.z == 0) { /* an empty part: no sweep blocks */
     } else if (do_h) {
         prof_mark(ctx, s_local, 0, 0);
-        launch_chained(ctx, h_sweep_tma<R, STRICT>, grid, TmaGeom<R>::H_SMEM, a, ctx->maps);
+        launch_chained(ctx, h_sweep_tma<R, STRICT, false>, grid, TmaGeom<R>::H_SMEM, a, ctx->maps);
         prof_mark(ctx, s_local, 0, 1);
         launches++;
     }
@@ -1046,7 +1046,7 @@ static int fused_zstep(int tiles, int nz, int slots)
 template <typename R, bool STRICT, int NA>
 static int prepare_t(php_ctx* ctx)
 {
-    cudaError_t e = cudaFuncSetAttribute(h_sweep_tma<R, STRICT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(h_sweep_tma<R, STRICT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)TmaGeom<R>::H_SMEM);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(e_sweep_tma<R, STRICT, NA, kEAll>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1062,6 +1062,10 @@ static int prepare_t(php_ctx* ctx)
         if (e == cudaSuccess && ctx->split)
             e = cudaFuncSetAttribute(interior_sweep_tma<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)FusedGeom<R, true>::SMEM);
+    if constexpr (!STRICT)
+        if (e == cudaSuccess && ctx->split)
+            e = cudaFuncSetAttribute(h_sweep_tma<R, STRICT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)TmaGeom<R>::H_SMEM);
     if constexpr (!STRICT)
         if (e == cudaSuccess && ctx->fused)
             e = cudaFuncSetAttribute(he_sweep_tma<R, NA>, cudaFuncAttributeMaxDynamicSharedMemorySize,

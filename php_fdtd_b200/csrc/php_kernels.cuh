@@ -281,8 +281,14 @@ __device__ __forceinline__ int32_t ldg_nh(const int32_t* p)
  * one start.  One that does not (StepArgs::beside: its inputs come from
  * launches further back, complete since the launch before it entered) waits at
  * its end instead, in chain_leave, so that its own completion still implies
- * that of all before it.  Launched without the attribute, both return at
- * once.  Per step, plain launches and the chain: 32^3 7.6 -> 6.4 us, 96^3
+ * that of all before it.  Only a grid that waited is promised a view of what
+ * earlier ones wrote, its L1 included.  What one beside another reads is in L2
+ * before it starts (the launch before it entered after a wait for its writers,
+ * and started it after that), but a line of an earlier step may still be in an
+ * L1: the kernels that run so read what earlier launches wrote through L2
+ * (ld_state, prefetch_state, TMA); with these reads through L1 an interval of
+ * 256^3 took 23.2 ms FP64 and 14.7 ms FP32, through L2 23.3 and 15.0.  Launched
+ * without the attribute, both return at once.  Per step, plain launches and the chain: 32^3 7.6 -> 6.4 us, 96^3
  * two-atom slab FP64 55 -> 50 us, FP32 34.4 -> 34.0 us; 256^3 unchanged. */
 __device__ __forceinline__ void chain_enter(int beside)
 {
@@ -292,6 +298,40 @@ __device__ __forceinline__ void chain_enter(int beside)
 __device__ __forceinline__ void chain_leave(int beside, int tid)
 {
     if (beside && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && tid == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+/* State that an earlier launch wrote and this one does not before the read;
+ * CG: through L2, past the L1 (see chain_enter). */
+template <bool CG>
+__device__ __forceinline__ double ld_state(const double* p)
+{
+    if constexpr (!CG) return *p;
+    double v;
+    asm volatile("ld.global.cg.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
+template <bool CG>
+__device__ __forceinline__ float ld_state(const float* p)
+{
+    if constexpr (!CG) return *p;
+    float v;
+    asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+template <bool CG>
+__device__ __forceinline__ uint32_t ld_state(const uint32_t* p)
+{
+    if constexpr (!CG) return *p;
+    uint32_t v;
+    asm volatile("ld.global.cg.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+/* its line, requested ahead of the read */
+template <bool CG>
+__device__ __forceinline__ void prefetch_state(const void* p)
+{
+    if constexpr (CG) asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+    else asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
 }
 
 /* CPML slot of cell i of an axis of n cells: i at the low side, L + n - 1 - i
@@ -430,12 +470,14 @@ __global__ void probe_record_counted(const Fields<R> f, const R* dp, const DCell
  * phasors of this step (ph[2f], ph[2f+1]), t = j * nx + i of n = nx * ny
  * (x fastest, so that a warp's cells along x update adjacent accumulators;
  * php_dft_read hands them out in [f][i][j] order). */
+template <bool CG>
 __device__ __forceinline__ void dft_accumulate(double x, const double* ph, int nfreq, double* acc, int64_t n, int64_t t)
 {
     for (int f = 0; f < nfreq; ++f) {
         double* a = acc + ((int64_t)f * n + t) * 2;
-        a[0] += x * ph[2 * f];
-        a[1] += x * ph[2 * f + 1];
+        const double re = ld_state<CG>(a), im = ld_state<CG>(a + 1);
+        a[0] = re + x * ld_state<CG>(ph + 2 * f);
+        a[1] = im + x * ld_state<CG>(ph + 2 * f + 1);
     }
 }
 
@@ -452,7 +494,7 @@ __global__ void dft_sample(const Fields<R> fld, const DView<R> dv, int comp, int
         const int j = (int)(t / nx), i = (int)(t % nx);
         double x = field_at(fld, dv, comp, plane_off + (int64_t)j * nxp + i);
         if (cast_f32) x = (double)(float)x;
-        dft_accumulate(x, ph, nfreq, acc, n, t);
+        dft_accumulate<false>(x, ph, nfreq, acc, n, t);
     }
 }
 
@@ -475,13 +517,13 @@ __global__ void __launch_bounds__(256) dft_reorder(const double2* acc, int nx, i
  * that this step samples (e3: the E arrays the sweep wrote).  A cell's
  * accumulators belong to the one thread that updates the cell; no register
  * is held for this inside the march. */
-template <typename R>
+template <bool CG, typename R>
 __device__ __forceinline__ void dft_fold(const StepArgs<R>& a, R* const* e3, int i, int j, int k0, int k1)
 {
     if (i >= a.nx || j >= a.ny) return;
     for (int q = 0; q < a.ndft; ++q) {
         const int k = a.dft_z[q];
-        if (k < k0 || k >= k1 || a.src_val[a.dft_off[q]] == 0.0) continue;
+        if (k < k0 || k >= k1 || ld_state<CG>(a.src_val + a.dft_off[q]) == 0.0) continue;
         const int cp = a.dft_comp[q];
         const int c = (k * a.ny + j) * a.nxp + i;
         double x;
@@ -495,7 +537,7 @@ __device__ __forceinline__ void dft_fold(const StepArgs<R>& a, R* const* e3, int
             x = d_at(f, a.dv, cp - 3, c);
         }
         if (a.dft_cast[q]) x = (double)(float)x;
-        dft_accumulate(x, a.src_val + a.dft_off[q] + 1, a.dft_nfreq[q], a.dft_acc[q], (int64_t)a.nx * a.ny,
+        dft_accumulate<CG>(x, a.src_val + a.dft_off[q] + 1, a.dft_nfreq[q], a.dft_acc[q], (int64_t)a.nx * a.ny,
                        (int64_t)j * a.nx + i);
     }
 }
@@ -505,13 +547,13 @@ __device__ __forceinline__ void dft_fold(const StepArgs<R>& a, R* const* e3, int
  * column (i, j) reads back the E, D and H of the field cell (e3, h3: the arrays
  * the step's launches wrote), and the one whose planes hold the atom cell its r
  * and v. */
-template <typename R>
+template <bool CG, typename R>
 __device__ __forceinline__ void probe_fold(const StepArgs<R>& a, R* const* e3, R* const* h3, int i, int j, int k0, int k1)
 {
     if (i != a.probe_i || j != a.probe_j) return;
     const bool fields = a.probe_kf >= k0 && a.probe_kf < k1, atoms = a.probe_n3 && a.probe_ka >= k0 && a.probe_ka < k1;
     if (!fields && !atoms) return;
-    const int row = (int)a.src_val[a.probe_off];
+    const int row = (int)ld_state<CG>(a.src_val + a.probe_off);
     if (row >= a.probe_cap) {
         if (fields) a.probe_count[1] = 1;
         return;
@@ -523,10 +565,8 @@ __device__ __forceinline__ void probe_fold(const StepArgs<R>& a, R* const* e3, R
         f.ex = e3[0];
         f.ey = e3[1];
         f.ez = e3[2];
-        f.hx = h3[0];
-        f.hy = h3[1];
-        f.hz = h3[2];
-        for (int q = 0; q < 9; ++q) out[q] = field_at(f, a.dv, q, c);
+        for (int q = 0; q < 6; ++q) out[q] = field_at(f, a.dv, q, c);
+        for (int q = 0; q < 3; ++q) out[6 + q] = (double)ld_state<CG>(h3[q] + c);
         a.probe_count[0] = row + 1;
     }
     for (int q = 0; atoms && q < a.probe_n3; ++q) {

@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(kBlockX * kBlockY, (kStepBlocks<R, NAMAX>))
 #pragma unroll
                 for (int r = 0; r < ROWS; ++r) {
                     if (ih && j + r < a.ny - 1) h_psi_prefetch(a, slot_i, slot_j[r], sz1, i, j + r, p + 1);
-                    if (iin && j + r >= 1 && j + r < a.ny - 1) prefetch_psi_d(a, i, j + r, p + 1, slot_i, slot_j[r]);
+                    if (iin && j + r >= 1 && j + r < a.ny - 1) prefetch_psi_d<false>(a, i, j + r, p + 1, slot_i, slot_j[r]);
                 }
                 if (halo_upd) h_psi_prefetch(a, pml_slot(ci, a.nx, a.L), pml_slot(cj, a.ny, a.L), sz1, ci, cj, p + 1);
             }
@@ -528,8 +528,8 @@ __global__ void __launch_bounds__(kBlockX * kBlockY, (kStepBlocks<R, NAMAX>))
     }
 #pragma unroll 1
     for (int r = 0; r < ROWS; ++r) {
-        if (a.ndft) dft_fold(a, a.enew, i, j + r, k0, k1); /* the new E */
-        if (a.probe_rows) probe_fold(a, a.enew, a.hnew, i, j + r, k0, k1);
+        if (a.ndft) dft_fold<false>(a, a.enew, i, j + r, k0, k1); /* the new E */
+        if (a.probe_rows) probe_fold<false>(a, a.enew, a.hnew, i, j + r, k0, k1);
     }
 }
 
@@ -730,8 +730,8 @@ __global__ void __launch_bounds__(kBlockX * kBlockY, (sizeof(R) == 8 ? PHP_INNER
     }
 #pragma unroll 1
     for (int r = 0; r < ROWS; ++r) {
-        if (a.ndft) dft_fold(a, a.enew, i, j + r, k0, k1); /* the new E */
-        if (a.probe_rows) probe_fold(a, a.enew, a.hnew, i, j + r, k0, k1);
+        if (a.ndft) dft_fold<false>(a, a.enew, i, j + r, k0, k1); /* the new E */
+        if (a.probe_rows) probe_fold<false>(a, a.enew, a.hnew, i, j + r, k0, k1);
     }
     chain_leave(a.beside, tid);
 }

@@ -124,7 +124,7 @@ struct CellPsi {
 };
 
 /* psi_D of fdtd.c:3258-3334 (the reads) */
-template <typename R, bool STRICT = false>
+template <typename R, bool STRICT = false, bool CG = false>
 __device__ __forceinline__ void load_psi_d(const StepArgs<R>& a, int i, int j, int k, int sx, int sy, bool cell, CellPsi<R>& ps)
 {
     const int L2 = 2 * a.L;
@@ -134,41 +134,41 @@ __device__ __forceinline__ void load_psi_d(const StepArgs<R>& a, int i, int j, i
     if (!cell) return;
     if (sx >= 0) {
         const int q = (k * a.ny + j) * L2 + sx;
-        ps.xy = a.psi.dxy[q];
-        ps.xz = a.psi.dxz[q];
+        ps.xy = ld_state<CG>(a.psi.dxy + q);
+        ps.xz = ld_state<CG>(a.psi.dxz + q);
     }
     if (sy >= 0) {
         const int q = (k * L2 + sy) * a.nxp + i;
-        ps.yx = a.psi.dyx[q];
-        ps.yz = a.psi.dyz[q];
+        ps.yx = ld_state<CG>(a.psi.dyx + q);
+        ps.yz = ld_state<CG>(a.psi.dyz + q);
     }
     if (ps.sz >= 0) {
         const int q = (ps.sz * a.ny + j) * a.nxp + i;
-        ps.zx = a.psi.dzx[q];
-        ps.zy = a.psi.dzy[q];
+        ps.zx = ld_state<CG>(a.psi.dzx + q);
+        ps.zy = ld_state<CG>(a.psi.dzy + q);
     }
 }
 
-/* the lines load_psi_d reads at plane k, requested into L1 a plane ahead */
-template <typename R>
+/* the lines load_psi_d reads at plane k, requested a plane ahead */
+template <bool CG, typename R>
 __device__ __forceinline__ void prefetch_psi_d(const StepArgs<R>& a, int i, int j, int k, int sx, int sy)
 {
     const int L2 = 2 * a.L;
     if (sx >= 0) {
         const int q = (k * a.ny + j) * L2 + sx;
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(a.psi.dxy + q));
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(a.psi.dxz + q));
+        prefetch_state<CG>(a.psi.dxy + q);
+        prefetch_state<CG>(a.psi.dxz + q);
     }
     if (sy >= 0) {
         const int q = (k * L2 + sy) * a.nxp + i;
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(a.psi.dyx + q));
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(a.psi.dyz + q));
+        prefetch_state<CG>(a.psi.dyx + q);
+        prefetch_state<CG>(a.psi.dyz + q);
     }
     const int sz = z_slot(a, k);
     if (sz >= 0) {
         const int q = (sz * a.ny + j) * a.nxp + i;
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(a.psi.dzx + q));
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(a.psi.dzy + q));
+        prefetch_state<CG>(a.psi.dzx + q);
+        prefetch_state<CG>(a.psi.dzy + q);
     }
 }
 
@@ -297,17 +297,17 @@ __device__ __forceinline__ void e_only_add(const R* m, R ux, R uy, R uz, R& ex, 
  * several times that of the fields.  w holds the three components' remainders
  * in 10 bits each, in units of 2^-10 ulp of the D they belong to: one word per
  * cell read and written. */
-template <typename R>
+template <typename R, bool CG = false>
 __device__ __forceinline__ void pool_add(const StepArgs<R>& a, int64_t slot, R ux, R uy, R uz, R& dx, R& dy, R& dz)
 {
     const int64_t ns = a.nslot;
     const R* __restrict__ dp = a.Dp + slot;
-    dx = dp[0];
-    dy = dp[ns];
-    dz = dp[2 * ns];
+    dx = ld_state<CG>(dp);
+    dy = ld_state<CG>(dp + ns);
+    dz = ld_state<CG>(dp + 2 * ns);
     if constexpr (sizeof(R) == 4) {
         if (a.Dc) {
-            const uint32_t w = a.Dc[slot];
+            const uint32_t w = ld_state<CG>(a.Dc + slot);
             uint32_t out = 0;
             auto add = [&](float& d, float u, int sh) {
                 const int q = (int)(w << (22 - sh)) >> 22;
@@ -410,7 +410,7 @@ struct IonPre {
  * entry (lab frame) and E^{n+1} on return; dx..dz are D^{n+1}; ix..iz are
  * D^{n+1} - D^n as summed before rounding into D (FP32 only).  pre: the
  * slot already read, or null. */
-template <typename R, bool STRICT, int NAMAX>
+template <typename R, bool STRICT, int NAMAX, bool CG = false>
 __device__ __forceinline__ void e_update(const StepArgs<R>& a, const MatCoef<R>& m, int c,
                                          R dx, R dy, R dz, R ix, R iy, R iz, R& ex, R& ey, R& ez,
                                          const IonPre* pre = nullptr)
@@ -440,8 +440,8 @@ __device__ __forceinline__ void e_update(const StepArgs<R>& a, const MatCoef<R>&
                     /* 32-bit element offsets: the host keeps few-atom pools
                      * below 2^32 elements */
                     const uint32_t o = (uint32_t)q * (uint32_t)ns + (uint32_t)slot;
-                    rold[q] = q < n3 ? a.r[o] : R(0);
-                    vold[q] = q < n3 ? a.v[o] : R(0);
+                    rold[q] = q < n3 ? ld_state<CG>(a.r + o) : R(0);
+                    vold[q] = q < n3 ? ld_state<CG>(a.v + o) : R(0);
                 }
             }
             auto ion_pr = [&](const auto& C) {
@@ -450,10 +450,10 @@ __device__ __forceinline__ void e_update(const StepArgs<R>& a, const MatCoef<R>&
                     if constexpr (VREG) {
                         rq = rold[q];
                     } else {
-                        rq = a.r[(int64_t)q * ns + slot];
+                        rq = ld_state<CG>(a.r + (int64_t)q * ns + slot);
                         rold[q] = rq;
-                        /* v is read after E^{n+1}: bring it into L1 now */
-                        asm volatile("prefetch.global.L1 [%0];" ::"l"(a.v + (int64_t)q * ns + slot));
+                        /* v is read after E^{n+1}: request it now */
+                        prefetch_state<CG>(a.v + (int64_t)q * ns + slot);
                     }
                     const int at = q / 3, d = q - 3 * at;
                     const R q0 = C.zv(at * 9 + 0 * 3 + d);
@@ -478,9 +478,9 @@ __device__ __forceinline__ void e_update(const StepArgs<R>& a, const MatCoef<R>&
     if constexpr (!STRICT && NAMAX == 0) {
         /* many-atom cells: P_ion = QeZV . r^n left by the ion pass */
         if ((flags & kAtoms) && a.pr) {
-            pr0 = a.pr[slot];
-            pr1 = a.pr[ns + slot];
-            pr2 = a.pr[2 * ns + slot];
+            pr0 = ld_state<CG>(a.pr + slot);
+            pr1 = ld_state<CG>(a.pr + ns + slot);
+            pr2 = ld_state<CG>(a.pr + 2 * ns + slot);
         }
     }
 
@@ -605,7 +605,7 @@ __device__ __forceinline__ void e_update(const StepArgs<R>& a, const MatCoef<R>&
                 const int64_t o = VREG ? (int64_t)((uint32_t)q * (uint32_t)ns + (uint32_t)slot) : (int64_t)q * ns + slot;
                 R vq;
                 if constexpr (VREG) vq = vold[q];
-                else vq = a.v[o];
+                else vq = ld_state<CG>(a.v + o);
                 if constexpr (STRICT) {
                     a.r[o] = SOp::add(rold[q], SOp::add(SOp::mul(vq, a.dt), SOp::mul(SOp::mul(SOp::mul(0.5, acc), a.dt), a.dt)));
                     a.v[o] = SOp::add(vq, SOp::mul(acc, a.dt));

@@ -83,7 +83,7 @@ constexpr uint32_t kWaitLimit = 1u << 24;
  * plane ahead, into registers (256^3 tip workload, fused sweep of the rest 114
  * -> 110 us); where r and v sit in registers too, and in the strict mode, after
  * the plane before it is done (two-atom fused sweep, 512 x 512 x 256: 480 ->
- * 450 us).  FP64: before the plane's wait, its lines requested into L1 a plane
+ * 450 us).  FP64: before the plane's wait, its lines requested a plane
  * ahead (the same sweep 785 us; after the plane before it 851 us). */
 enum : int { kPsiAhead = 0, kPsiAfter = 1, kPsiTop = 2 };
 template <typename R, bool STRICT, bool VREG>
@@ -226,10 +226,10 @@ struct TmaGeom {
 struct SweepJob {
     int bx, by, k0, k1, cls;
 };
-template <typename R>
+template <bool LIST, typename R>
 __device__ __forceinline__ SweepJob sweep_job(const StepArgs<R>& a, const uint8_t* cls, int dflt)
 {
-    if (a.list) {
+    if constexpr (LIST) {
         const int4 e = a.list[blockIdx.x];
         return SweepJob{e.x & 0xffff, e.x >> 16, e.y, e.z, e.w};
     }
@@ -253,7 +253,7 @@ __device__ __forceinline__ unsigned char* ring_base(unsigned char* dyn)
 #ifndef PHP_H_MINBLOCKS32
 #define PHP_H_MINBLOCKS32 6
 #endif
-template <typename R, bool STRICT>
+template <typename R, bool STRICT, bool LIST>
 __global__ void __launch_bounds__(kBlockX * kBlockY, sizeof(R) == 4 ? PHP_H_MINBLOCKS32 : 4) h_sweep_tma(const __grid_constant__ StepArgs<R> a,
                                                                  const __grid_constant__ TmaMaps tm)
 {
@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(kBlockX * kBlockY, sizeof(R) == 4 ? PHP_H_MINB
     R* const tab = reinterpret_cast<R*>(smem + G::HS * G::STAGE + 128);
 
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * G::TX + tx;
-    const SweepJob job = sweep_job(a, a.plain_h, 0);
+    const SweepJob job = sweep_job<LIST>(a, a.plain_h, 0);
     const int i0 = job.bx * G::TX, j0 = job.by * G::TY;
     const int i = i0 + tx, j = j0 + ty;
     const int k0 = job.k0, k1 = job.k1;
@@ -310,9 +310,9 @@ __global__ void __launch_bounds__(kBlockX * kBlockY, sizeof(R) == 4 ? PHP_H_MINB
         p.xy = p.xz = p.yx = p.yz = p.zx = p.zy = R(0);
         if (!active) return;
         const int qx = (k * ny + j) * L2 + sx, qy = (k * L2 + sy) * nxp + i, qz = (p.sz * ny + j) * nxp + i;
-        if (sx >= 0) { p.xy = a.psi.hxy[qx]; p.xz = a.psi.hxz[qx]; }
-        if (sy >= 0) { p.yx = a.psi.hyx[qy]; p.yz = a.psi.hyz[qy]; }
-        if (p.sz >= 0) { p.zx = a.psi.hzx[qz]; p.zy = a.psi.hzy[qz]; }
+        if (sx >= 0) { p.xy = ld_state<LIST>(a.psi.hxy + qx); p.xz = ld_state<LIST>(a.psi.hxz + qx); }
+        if (sy >= 0) { p.yx = ld_state<LIST>(a.psi.hyx + qy); p.yz = ld_state<LIST>(a.psi.hyz + qy); }
+        if (p.sz >= 0) { p.zx = ld_state<LIST>(a.psi.hzx + qz); p.zy = ld_state<LIST>(a.psi.hzy + qz); }
     };
     Psi6 ps;
     if (!plain) load_psi(k0, ps);
@@ -392,18 +392,18 @@ __global__ void __launch_bounds__(kBlockX * kBlockY, sizeof(R) == 4 ? PHP_H_MINB
                 const int sz1 = z_slot(a, k + 1);
                 if (sx >= 0) {
                     const int q = ((k + 1) * ny + j) * L2 + sx;
-                    asm volatile("prefetch.global.L1 [%0];" ::"l"(a.psi.hxy + q));
-                    asm volatile("prefetch.global.L1 [%0];" ::"l"(a.psi.hxz + q));
+                    prefetch_state<LIST>(a.psi.hxy + q);
+                    prefetch_state<LIST>(a.psi.hxz + q);
                 }
                 if (sy >= 0) {
                     const int q = ((k + 1) * L2 + sy) * nxp + i;
-                    asm volatile("prefetch.global.L1 [%0];" ::"l"(a.psi.hyx + q));
-                    asm volatile("prefetch.global.L1 [%0];" ::"l"(a.psi.hyz + q));
+                    prefetch_state<LIST>(a.psi.hyx + q);
+                    prefetch_state<LIST>(a.psi.hyz + q);
                 }
                 if (sz1 >= 0) {
                     const int q = (sz1 * ny + j) * nxp + i;
-                    asm volatile("prefetch.global.L1 [%0];" ::"l"(a.psi.hzx + q));
-                    asm volatile("prefetch.global.L1 [%0];" ::"l"(a.psi.hzy + q));
+                    prefetch_state<LIST>(a.psi.hzx + q);
+                    prefetch_state<LIST>(a.psi.hzy + q);
                 }
             }
         }
@@ -537,7 +537,8 @@ __global__ void __launch_bounds__(kBlockX * kBlockY, (kEBlocks<R, NAMAX, CLS>))
     R* const tab = reinterpret_cast<R*>(smem + G::ES * G::STAGE + 128);
 
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * G::TX + tx;
-    const SweepJob job = sweep_job(a, a.plain_blk, 255);
+    constexpr bool CG = CLS == kEPlain || CLS == kEAtoms; /* launches beside others */
+    const SweepJob job = sweep_job<CLS != kEAll>(a, a.plain_blk, 255);
     const int i0 = job.bx * G::TX, j0 = job.by * G::TY;
     const int i = i0 + tx, j = j0 + ty;
     const int k0 = job.k0, k1 = job.k1;
@@ -581,7 +582,7 @@ __global__ void __launch_bounds__(kBlockX * kBlockY, (kEBlocks<R, NAMAX, CLS>))
     CellPsi<R> ps;
     int slot = -1, mid = 0;
     if (more) {
-        if (first) load_psi_d<R, STRICT>(a, i, j, k0, sx, sy, interior, ps);
+        if (first) load_psi_d<R, STRICT, CG>(a, i, j, k0, sx, sy, interior, ps);
         if (slots) slot = ldg(a.slot + (k0 * a.ny + j) * a.nxp + i);
         if (pm == 255 && active) mid = ldg(a.mat + (k0 * a.ny + j) * a.nxp + i);
     }
@@ -661,31 +662,31 @@ __global__ void __launch_bounds__(kBlockX * kBlockY, (kEBlocks<R, NAMAX, CLS>))
                 const R iso = CLS != kEAtoms && pm < kPlainTensor ? a.iso[pm - kPlainCpml] : R(0);
                 for (int k = k0; k < k1; ++k) {
                     CellPsi<R> pn;
-                    if (mode == kPsiAhead && k + 1 < k1) load_psi_d(a, i, j, k + 1, sx, sy, interior, pn);
+                    if (mode == kPsiAhead && k + 1 < k1) load_psi_d<R, false, CG>(a, i, j, k + 1, sx, sy, interior, pn);
                     if (mode == kPsiTop) {
-                        if (!first || k > k0) load_psi_d(a, i, j, k, sx, sy, interior, ps);
-                        if (interior && k + 1 < k1) prefetch_psi_d(a, i, j, k + 1, sx, sy);
+                        if (!first || k > k0) load_psi_d<R, false, CG>(a, i, j, k, sx, sy, interior, ps);
+                        if (interior && k + 1 < k1) prefetch_psi_d<CG>(a, i, j, k + 1, sx, sy);
                     }
                     const int c = (k * a.ny + j) * a.nxp + i;
                     IonPre ip;
                     ip.slot = slot;
                     if constexpr (NAMAX <= 4 && CLS != kEPlain) {
                         if (atoms && active) {
-                            /* its D, and r and v (or P_ion), into L1 ahead of their reads */
+                            /* its D, and r and v (or P_ion), requested ahead of their reads */
                             constexpr int QN = 3 * NAMAX;
                             const int n3 = 3 * a.amc.natom;
-                            if (a.Dc) asm volatile("prefetch.global.L1 [%0];" ::"l"(a.Dc + ip.slot));
+                            if (a.Dc) prefetch_state<CG>(a.Dc + ip.slot);
 #pragma unroll
                             for (int q = 0; q < 3; ++q) {
-                                asm volatile("prefetch.global.L1 [%0];" ::"l"(a.Dp + q * a.nslot + ip.slot));
-                                if (NAMAX == 0) asm volatile("prefetch.global.L1 [%0];" ::"l"(a.pr + q * a.nslot + ip.slot));
+                                prefetch_state<CG>(a.Dp + q * a.nslot + ip.slot);
+                                if (NAMAX == 0) prefetch_state<CG>(a.pr + q * a.nslot + ip.slot);
                             }
 #pragma unroll
                             for (int q = 0; q < QN; ++q) {
                                 const int64_t o = (int64_t)q * a.nslot + ip.slot;
                                 if (q < n3) {
-                                    asm volatile("prefetch.global.L1 [%0];" ::"l"(a.r + o));
-                                    asm volatile("prefetch.global.L1 [%0];" ::"l"(a.v + o));
+                                    prefetch_state<CG>(a.r + o);
+                                    prefetch_state<CG>(a.v + o);
                                 }
                             }
                         }
@@ -715,8 +716,8 @@ __global__ void __launch_bounds__(kBlockX * kBlockY, (kEBlocks<R, NAMAX, CLS>))
                             const int64_t ns = a.nslot;
                             R* __restrict__ dp = a.Dp + ip.slot;
                             R dx, dy, dz;
-                            pool_add(a, ip.slot, ux, uy, uz, dx, dy, dz);
-                            e_update<R, false, NAMAX>(a, a.amc, c, dx, dy, dz, ux, uy, uz, ex, ey, ez, &ip);
+                            pool_add<R, CG>(a, ip.slot, ux, uy, uz, dx, dy, dz);
+                            e_update<R, false, NAMAX, CG>(a, a.amc, c, dx, dy, dz, ux, uy, uz, ex, ey, ez, &ip);
                             dp[0] = dx;
                             dp[ns] = dy;
                             dp[2 * ns] = dz;
@@ -726,7 +727,7 @@ __global__ void __launch_bounds__(kBlockX * kBlockY, (kEBlocks<R, NAMAX, CLS>))
                         a.enew[2][c] = ez;
                     }
                     if (mode == kPsiAhead) ps = pn;
-                    if (mode == kPsiAfter && k + 1 < k1) load_psi_d(a, i, j, k + 1, sx, sy, interior, ps);
+                    if (mode == kPsiAfter && k + 1 < k1) load_psi_d<R, false, CG>(a, i, j, k + 1, sx, sy, interior, ps);
                     if (atoms && slots && k + 1 < k1) slot = ldg(a.slot + ((k + 1) * a.ny + j) * a.nxp + i);
                     if (!next(k, ok)) break;
                 }
@@ -735,21 +736,21 @@ __global__ void __launch_bounds__(kBlockX * kBlockY, (kEBlocks<R, NAMAX, CLS>))
                  * requested before the stage wait */
                 for (int k = k0; k < k1; ++k) {
                     CellPsi<R> pn;
-                    if (mode == kPsiAhead && k + 1 < k1) load_psi_d(a, i, j, k + 1, sx, sy, interior, pn);
+                    if (mode == kPsiAhead && k + 1 < k1) load_psi_d<R, false, CG>(a, i, j, k + 1, sx, sy, interior, pn);
                     if (mode == kPsiTop) {
-                        if (!first || k > k0) load_psi_d(a, i, j, k, sx, sy, interior, ps);
-                        if (interior && k + 1 < k1) prefetch_psi_d(a, i, j, k + 1, sx, sy);
+                        if (!first || k > k0) load_psi_d<R, false, CG>(a, i, j, k, sx, sy, interior, ps);
+                        if (interior && k + 1 < k1) prefetch_psi_d<CG>(a, i, j, k + 1, sx, sy);
                     }
                     if (slot >= 0) {
                         const int64_t ns = a.nslot;
 #pragma unroll
                         for (int q = 0; q < 3; ++q) {
-                            asm volatile("prefetch.global.L1 [%0];" ::"l"(a.Dp + q * ns + slot));
+                            prefetch_state<CG>(a.Dp + q * ns + slot);
                             if (a.P) {
-                                asm volatile("prefetch.global.L1 [%0];" ::"l"(a.P + q * ns + slot));
-                                asm volatile("prefetch.global.L1 [%0];" ::"l"(a.Po + q * ns + slot));
+                                prefetch_state<CG>(a.P + q * ns + slot);
+                                prefetch_state<CG>(a.Po + q * ns + slot);
                             }
-                            if (NAMAX == 0 && a.pr) asm volatile("prefetch.global.L1 [%0];" ::"l"(a.pr + q * ns + slot));
+                            if (NAMAX == 0 && a.pr) prefetch_state<CG>(a.pr + q * ns + slot);
                         }
                     }
                     const bool ok = wait(k);
@@ -765,7 +766,7 @@ __global__ void __launch_bounds__(kBlockX * kBlockY, (kEBlocks<R, NAMAX, CLS>))
                         a.enew[2][c] = ez;
                     }
                     if (mode == kPsiAhead) ps = pn;
-                    if (mode == kPsiAfter && k + 1 < k1) load_psi_d(a, i, j, k + 1, sx, sy, interior, ps);
+                    if (mode == kPsiAfter && k + 1 < k1) load_psi_d<R, false, CG>(a, i, j, k + 1, sx, sy, interior, ps);
                     if (slots && k + 1 < k1) slot = ldg(a.slot + ((k + 1) * a.ny + j) * a.nxp + i);
                     if (active && k + 1 < k1) mid = ldg(a.mat + ((k + 1) * a.ny + j) * a.nxp + i);
                     if (!next(k, ok)) break;
@@ -790,8 +791,8 @@ __global__ void __launch_bounds__(kBlockX * kBlockY, (kEBlocks<R, NAMAX, CLS>))
     }
     /* after the march: the running DFT samples and the monitor row of this
      * chunk's planes */
-    if (a.ndft) dft_fold(a, a.enew, i, j, k0, k1);
-    if (a.probe_rows) probe_fold(a, a.enew, a.hnew, i, j, k0, k1);
+    if (a.ndft) dft_fold<CG>(a, a.enew, i, j, k0, k1);
+    if (a.probe_rows) probe_fold<CG>(a, a.enew, a.hnew, i, j, k0, k1);
     chain_leave(a.beside, tid);
 }
 
