@@ -327,6 +327,7 @@ __global__ void __launch_bounds__(kBlockX * kBlockY, sizeof(R) == 4 ? PHP_H_MINB
                 atomicExch(a.err, 1);
                 ring_drain(full, G::HS, h_loads_issued(k0, k0, k1, G::HS));
             }
+            chain_leave(a.beside, tid);
             return;
         }
     }
