@@ -843,6 +843,7 @@ static void launch_ions(php_ctx* ctx)
     a.ntiles = (int32_t)((ctx->nslot + tile - 1) / tile);
     a.dt = ctx->d.dt;
     a.err = ctx->err_flag;
+    a.stall_test = ctx->stall_test;
     cudaStream_t st = ctx->stream;
     if (ctx->ion_pipe) {
         /* one persistent CTA per SM */

@@ -55,6 +55,7 @@ struct IonArgs {
     int32_t ion_off_ref;         /* the lattice's QeZV/QeZM block, staged in shared memory */
     double dt;
     int32_t* err;
+    int32_t stall_test;          /* failure-path test: the first group of ion_pipe's first block gives up on its first tile */
 };
 
 constexpr int kIonTile = 128;
@@ -315,7 +316,6 @@ __global__ void __launch_bounds__(IonPipe<R, NP, S>::THREADS, 1)
     uint64_t* empty = full + S;
     uint64_t* mma_bar = empty + S;                                 /* one per group */
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mma_bar + P::GROUPS);
-    volatile int32_t* consumed = reinterpret_cast<volatile int32_t*>(tmem_slot + 1);
 
     const int tid = threadIdx.x, warp = tid >> 5;
     const int mine = a.ntiles > (int)blockIdx.x ? (a.ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
@@ -344,7 +344,6 @@ __global__ void __launch_bounds__(IonPipe<R, NP, S>::THREADS, 1)
             mbar_init(&empty[q], 1);
         }
         for (int g = 0; g < P::GROUPS; ++g) mbar_init(&mma_bar[g], 1);
-        *consumed = 0;
         fence_barrier_init();
     }
     fence_proxy_async_smem();
@@ -354,6 +353,8 @@ __global__ void __launch_bounds__(IonPipe<R, NP, S>::THREADS, 1)
     const uint32_t tmem0 = P::TC ? *tmem_slot : 0u;
     const uint32_t tx_bytes = 2u * P::TILE * (uint32_t)n3 * (uint32_t)sizeof(R);
     bool failed = false;
+    /* the failure-path test's waits give up early */
+    const uint32_t limit = a.stall_test ? kStallPolls : kWaitLimit;
 
     if (warp == P::CONSUMERS / 32) {
         /* ------------------------------------------------------ producer */
@@ -362,7 +363,7 @@ __global__ void __launch_bounds__(IonPipe<R, NP, S>::THREADS, 1)
         /* lane 0: once the consumers are done with tile kk, its stage goes back
          * with one tensor store per array (the consumers never wait for it) */
         auto store_tile = [&](int kk) -> bool {
-            if (!mbar_wait(&empty[kk % S], (kk / S) & 1)) return false;
+            if (!mbar_wait_n(&empty[kk % S], (kk / S) & 1, limit)) return false;
             const int x = ((int)blockIdx.x + kk * (int)gridDim.x) * P::TILE;
             unsigned char* b = stages + (kk % S) * P::STAGE;
             tma_store_3d(&maps.r, b, x, 0, 0);
@@ -427,8 +428,10 @@ __global__ void __launch_bounds__(IonPipe<R, NP, S>::THREADS, 1)
             for (int kk = max(0, mine - S); kk < mine && !failed; ++kk) failed = !store_tile(kk);
         if (failed && lane == 0) {
             atomicExch(a.err, 1);
-            /* loads issued and not consumed land before the CTA leaves */
-            for (int k = *consumed; k < issued; ++k) mbar_wait(&full[k % S], (k / S) & 1);
+            /* the loads in flight land before the CTA leaves.  The groups take
+             * tiles in turn, so a tile may be left behind by one group while the
+             * others finish later ones: any of the last S loads may be open */
+            ring_drain(full, S, (uint32_t)issued);
         }
         if (lane == 0) bulk_wait0(); /* stores complete before the CTA leaves */
     } else {
@@ -448,7 +451,9 @@ __global__ void __launch_bounds__(IonPipe<R, NP, S>::THREADS, 1)
         for (int k = g; k < mine; k += P::GROUPS) {
             const int st = k % S;
             const int64_t s = (int64_t)((int)blockIdx.x + k * (int)gridDim.x) * P::TILE + gt;
-            const bool got = mbar_wait(&full[st], (k / S) & 1);
+            /* (the test's wait: no MMA of the group has been committed yet) */
+            const bool stall = a.stall_test && blockIdx.x == 0 && k == 0;
+            const bool got = mbar_wait_n(stall ? &mma_bar[g] : &full[st], stall ? 0 : (k / S) & 1, limit);
             if (named_sync_or(bar_id, P::GT, !got)) {
                 failed = true;
                 break;
@@ -518,7 +523,7 @@ __global__ void __launch_bounds__(IonPipe<R, NP, S>::THREADS, 1)
                                      smem_addr(&mma_bar[g]))
                                  : "memory");
                 }
-                const bool done = mbar_wait(&mma_bar[g], mphase);
+                const bool done = mbar_wait_n(&mma_bar[g], mphase, limit);
                 mphase ^= 1u;
                 if (named_sync_or(bar_id, P::GT, !done)) {
                     failed = true;
@@ -733,10 +738,7 @@ __global__ void __launch_bounds__(IonPipe<R, NP, S>::THREADS, 1)
              * proxy fence, the barrier and the arrival) */
             fence_proxy_async_smem();
             named_sync(bar_id, P::GT);
-            if (gi == 0) {
-                atomicMax((int32_t*)consumed, k + 1);
-                mbar_arrive(&empty[st]);
-            }
+            if (gi == 0) mbar_arrive(&empty[st]);
         }
         if (failed && gi == 0) atomicExch(a.err, 1);
     }

@@ -2,11 +2,13 @@
 reach, without a GPU fault: a wait on a barrier that nothing arrives on gives
 up, the launch finishes (its loads in flight and the launches beside it
 awaited), the status comes back, and the device and a new context work on.
-The H sweep beside the interior launch."""
+The H sweep beside the interior launch, and a group of the ion pass that leaves
+its first tile behind while the other groups finish later ones."""
 import numpy as np
 import pytest
 
 from php_fdtd_b200 import Material, PhpError, Simulation, Source, make_desc
+from php_fdtd_b200.workloads import lattice_data
 
 pytestmark = pytest.mark.gpu
 
@@ -44,3 +46,21 @@ def test_h_sweep_beside_the_interior_launch(precision, monkeypatch):
     src = [Source(type=1, x=50, y=30, z=20, component="z", frequency=1.5e15)]
     desc = make_desc(med, [Material()], src, dx=DL, dy=DL, dz=DL, dt=DT, pml_thickness=5, precision=precision)
     _stalls_and_recovers(desc, monkeypatch, PHP_FUSED="2")
+
+
+# tiles per block: one (a group without a second tile), and more than the ring holds
+@pytest.mark.parametrize("cells", [100, 130 * 60 * 18])
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_group_of_the_ion_pass(precision, cells, monkeypatch):
+    natom, (nx, ny, nz) = 16, (130, 60, 20)
+    rng = np.random.default_rng(natom)
+    z = rng.uniform(-0.5, 0.5, size=(natom, 3, 3)) + rng.choice([-3.0, 3.0], size=natom)[:, None, None] * np.eye(3)
+    z -= z.mean(axis=0)
+    qv, qm, dmm = lattice_data(z, rng.uniform(10.0, 90.0, natom), list(rng.uniform(300.0, 1000.0, 3 * natom)), natom, 12.0 * natom)
+    mats = [Material(), Material(eps_re=(4.9, 0, 0, 0, 4.9, 0, 0, 0, 2.95), natom=natom, qezv=qv, qezm=qm, dmm=dmm)]
+    med = np.zeros((nz, ny, nx), np.int32)
+    med.reshape(-1)[nx * ny:][:cells] = 1
+    med = np.ascontiguousarray(med.transpose(2, 1, 0))
+    src = [Source(type=1, x=nx // 2, y=ny // 2, z=3, component="z", frequency=4.0e13)]
+    desc = make_desc(med, mats, src, dx=DL, dy=DL, dz=DL, dt=DT, pml_thickness=0, precision=precision, source_frequency=4.0e13)
+    _stalls_and_recovers(desc, monkeypatch)
