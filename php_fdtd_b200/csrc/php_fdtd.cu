@@ -372,7 +372,16 @@ struct MatD {
 /* em = R^T eps^-1 R lf (1 - lt) / eps0, the map from D to E that the fast
  * modes apply (fdtd.c:3429-3503), and its inverse.  Where eps^-1 is close to
  * singular (its real part can be, for complex eps) the increment form would
- * lose digits, and D has no read-out from E: those materials keep D. */
+ * lose digits, and D has no read-out from E: those materials keep D.  So do
+ * those whose D would be read out with fewer correct digits than it was held
+ * in: M^-1 of a rounded E has up to kDSpread = max over rows of |M^-1| |M|
+ * (Skeel's condition number) roundings.  It is 1 for a diagonal M of any
+ * contrast and the contrast of eps for one turned by 45 degrees.  Error of D
+ * over that of a stored D, and of E over E = M D (one cell, 1000 oscillating
+ * increments, single precision, largest of 2 axes x 3 angles): 1.8 and 1.4 at a
+ * contrast of 2, 3.1 and 1.2 at 4, 8.5 and 1.5 at 8, 33 and 1.7 at 32, 170 and
+ * 1.8 at 250.  The limit admits the first of these; both precisions alike. */
+constexpr double kDSpread = 2.0;
 static void derive_e_only(const php_desc& d, MatD& o)
 {
     double rot[3][3] = {{1, 0, 0}, {0, 1, 0}, {0, 0, 1}}, m[3][3], inv[3][3];
@@ -401,6 +410,14 @@ static void derive_e_only(const php_desc& d, MatD& o)
     if (inverse3(s, inv)) return;
     for (int a = 0; a < 9; a++) big_inv = std::max(big_inv, fabs(inv[a / 3][a % 3]));
     if (!(big_inv < 256.0)) return;
+    double spread = 0.0;
+    for (int a = 0; a < 3; a++) {
+        double row = 0.0;
+        for (int b = 0; b < 3; b++)
+            for (int c = 0; c < 3; c++) row += fabs(inv[a][b] * s[b][c]);
+        spread = std::max(spread, row);
+    }
+    if (!(spread <= kDSpread * (1.0 + 1e-9))) return;
     for (int a = 0; a < 9; a++) {
         o.em[a] = m[a / 3][a % 3] / d.epsilon0;
         o.dm[a] = inv[a / 3][a % 3] / big * d.epsilon0;
