@@ -332,8 +332,8 @@ int php_last_launch_count(const php_ctx* ctx, int32_t* launches);
  * D/E sweep blocks of one plain isotropic material on the stencil-only path,
  * [1] such blocks with CPML or domain-edge cells, [2] blocks of the one
  * lossy or anisotropic material whose record rides in the kernel
- * parameters, [3] blocks of the few-atom lattice whose ions the fused sweep
- * updates, [4] all other fused-sweep blocks (the general per-cell path),
+ * parameters, [3] blocks of one atom material (or, in a domain without atoms,
+ * of one material that keeps D beside E), [4] all other fused-sweep blocks (the general per-cell path),
  * [5] H sweep blocks on the stencil-only path, [6] other H sweep blocks,
  * [7] the total number of blocks of one sweep.  The strict mode runs every
  * block on the general path.  No counterpart in the reference, which has

@@ -164,11 +164,13 @@ struct StepArgs {
     R tns_em[9], tns_im[9];
     int32_t tns_flags;
     /* the material record of the few-atom material whose ion coefficients
-     * are in ion_k, for blocks of that material alone (kPlainAtoms) */
+     * are in ion_k (or of the lattice of the ion pass, or, in a domain without
+     * atoms, of a material that keeps D), for blocks of that material alone
+     * (kPlainAtoms) */
     MatCoef<R> amc;
-    /* the record of the ADE material (without atoms) filling the most cells,
-     * -1 for none: the general path reads some 30 of its values per cell as
-     * constant-bank operands instead of loads */
+    /* the record of the material with pool cells but no atoms (ADE, or D kept
+     * beside E) that fills the most cells, -1 for none: the general path reads
+     * some 30 of its values per cell as constant-bank operands instead of loads */
     MatCoef<R> dmc;
     int32_t dmc_id;
     int64_t nslot;

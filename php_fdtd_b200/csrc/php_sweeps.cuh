@@ -647,7 +647,7 @@ __device__ __forceinline__ void e_cell_fast(const StepArgs<R>& a, int i, int j, 
     R ux = R(0), uy = R(0), uz = R(0);
     if (interior) {
         d_update<R, false>(a, i, j, k, sx, sy, hx0, hy0, hz0, hxk, hyk, hz_jm, hx_jm, hz_im, hy_im, ps, xt, yt, ux, uy, uz);
-        if (flags & kLossy) loss_sub(mp->eps_im, ex, ey, ez, ux, uy, uz);
+        if (flags & kLossy) loss_sub(dmc ? a.dmc.eps_im : mp->eps_im, ex, ey, ez, ux, uy, uz);
     }
     /* sources, in source order (fdtd.c:3363-3396) */
     for (int s = 0; s < a.nsrc; ++s) {

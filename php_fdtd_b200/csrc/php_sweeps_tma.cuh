@@ -680,7 +680,7 @@ __global__ void __launch_bounds__(kBlockX * kBlockY, (kEBlocks<R, NAMAX, CLS>))
 #pragma unroll
                             for (int q = 0; q < 3; ++q) {
                                 prefetch_state<CG>(a.Dp + q * a.nslot + ip.slot);
-                                if (NAMAX == 0) prefetch_state<CG>(a.pr + q * a.nslot + ip.slot);
+                                if (NAMAX == 0 && a.pr) prefetch_state<CG>(a.pr + q * a.nslot + ip.slot);
                             }
 #pragma unroll
                             for (int q = 0; q < QN; ++q) {
