@@ -712,8 +712,9 @@ struct FrameHead {
     int32_t pad_;
 };
 
-/* Field values (Ex Ey Ez Dx Dy Dz Hx Hy Hz) at device cell c, and r, v of the
- * atom cell c (none when its material has no atoms). */
+/* Field values (Ex Ey Ez Dx Dy Dz Hx Hy Hz) at device cell cf, and r, v of the
+ * atom cell ca (none when its material has no atoms, or ca < 0), zeros past
+ * them: the head's memory is not cleared between frames. */
 template <typename R>
 __device__ __forceinline__ void frame_cell(const Fields<R>& f, const DView<R>& dv, const uint8_t* mat, const int32_t* slot,
                                            const MatCoef<R>* mc, const R* r, const R* v, double rv_unit,
@@ -724,14 +725,14 @@ __device__ __forceinline__ void frame_cell(const Fields<R>& f, const DView<R>& d
     if (point9 && t < 9) {
         point9[t] = field_at(f, dv, t, cf);
     }
-    if (ca < 0) return;
-    const int na = mc[mat[ca]].natom;
+    if (!rr) return;
+    const int na = ca >= 0 ? mc[mat[ca]].natom : 0;
     const int64_t s = (na > 0 && slot) ? slot[ca] : -1;
     if (t == 0) *natom = s >= 0 ? na : 0;
-    if (s < 0) return;
-    for (int q = t; q < 3 * na && q < kFrameMaxN3; q += blockDim.x) {
-        rr[q] = rv_unit * (double)r[(int64_t)q * nslot + s];
-        vv[q] = rv_unit * (double)v[(int64_t)q * nslot + s];
+    for (int q = t; q < kFrameMaxN3; q += blockDim.x) {
+        const bool live = s >= 0 && q < 3 * na;
+        rr[q] = live ? rv_unit * (double)r[(int64_t)q * nslot + s] : 0.0;
+        vv[q] = live ? rv_unit * (double)v[(int64_t)q * nslot + s] : 0.0;
     }
 }
 
@@ -753,10 +754,7 @@ __global__ void __launch_bounds__(256) frame_gather(const Fields<R> f, const DVi
     const int t = threadIdx.x;
     if (parts) {
         const DiagPartial d = diag_reduce(parts, nparts);
-        if (t == 0) {
-            head->diag = d;
-            head->diag_natom = 0;
-        }
+        if (t == 0) head->diag = d;
         if (d.max_r > 0.0 && d.key_r != INT64_MAX) {
             /* reference loop order (i, j, k, coordinate), as php_diagnostics decodes it */
             const int64_t n3 = n3max > 1 ? n3max : 1;
@@ -768,15 +766,16 @@ __global__ void __launch_bounds__(256) frame_gather(const Fields<R> f, const DVi
             const int64_t c = ((int64_t)k * ny + j) * nxp + i;
             frame_cell(f, dv, mat, slot, mc, r, v, rv_unit, nslot, c, c, head->diag_point, head->diag_r, head->diag_v,
                        &head->diag_natom);
+        } else {
+            if (t < 9) head->diag_point[t] = 0.0;
+            frame_cell<R>(f, dv, mat, slot, mc, r, v, rv_unit, nslot, 0, -1, nullptr, head->diag_r, head->diag_v, &head->diag_natom);
         }
     }
     if (has_point)
         frame_cell<R>(f, dv, mat, slot, mc, r, v, rv_unit, nslot, point_c, -1, head->point, nullptr, nullptr, nullptr);
-    if (cell_c >= 0) {
-        if (t == 0) head->cell_natom = 0;
+    if (cell_c >= 0)
         frame_cell<R>(f, dv, mat, slot, mc, r, v, rv_unit, nslot, cell_c, cell_c, nullptr, head->cell_r, head->cell_v,
                       &head->cell_natom);
-    }
     if (rows_out)
         for (int64_t q = t; q < nrows * row_len; q += blockDim.x) rows_out[q] = rows[q];
     if (t == 0) {
