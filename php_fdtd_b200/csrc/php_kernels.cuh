@@ -345,11 +345,13 @@ __host__ __device__ __forceinline__ int pml_slot(int i, int n, int L)
 
 /* ========================================================== small kernels */
 
-/* one row of M^-1 E, rounded as a stored D would be */
+/* one row of M^-1 E, rounded as a stored D would be; a component that does not
+ * enter stays out even where it overflowed */
 template <typename R>
 __device__ __forceinline__ double d_of_e(const double* m, R ex, R ey, R ez)
 {
-    return (double)(R)__fma_rn(m[0], (double)ex, __fma_rn(m[1], (double)ey, m[2] * (double)ez));
+    const double x = m[0] != 0.0 ? (double)ex : 0.0, y = m[1] != 0.0 ? (double)ey : 0.0, z = m[2] != 0.0 ? (double)ez : 0.0;
+    return (double)(R)__fma_rn(m[0], x, __fma_rn(m[1], y, m[2] * z));
 }
 
 /* D component q of device cell c, halo planes included (zero) */

@@ -1,6 +1,7 @@
-"""Read-outs of what the device did not write: an output frame of a domain whose
-diagnostics found no displacement, after the same page-locked memory held
-another context's."""
+"""Read-outs of what the device did not write or cannot represent: an output
+frame of a domain whose diagnostics found no displacement, after the same
+page-locked memory held another context's, and D of a cell whose E overflowed in
+one component."""
 import numpy as np
 import pytest
 
@@ -37,3 +38,15 @@ def test_frame_without_a_displacement_is_zero(precision):
             np.testing.assert_array_equal(fr["diag_cell"]["point"], np.zeros(9))
             assert not len(fr["diag_cell"]["r"]) or not np.any(fr["diag_cell"]["r"])
             assert not len(fr["cell"]["r"]) or not np.any(fr["cell"]["r"])
+
+
+@pytest.mark.parametrize("mat", [Material(), Material(eps_re=(2.0, 0, 0, 0, 3.0, 0, 0, 0, 2.5))])
+def test_d_of_the_components_that_stayed_finite(mat):
+    """A source so strong that Ez of its cell overflows single precision in the
+    first step: Dx and Dy of the cell do not depend on Ez."""
+    with Simulation(_desc([mat], amplitude=1e60, type=0, t0=0.0, tau=1e-15)) as sim:
+        sim.step(1)
+        p = sim.read_point(16, 10, 6)
+        assert np.isinf(p[2]) and p[0] == 0 and p[1] == 0
+        assert p[3] == 0 and p[4] == 0 and np.isinf(p[5])
+        assert np.array_equal(sim.read_volume("Dx"), np.zeros(SHAPE))
