@@ -2107,6 +2107,7 @@ static int create_impl(const php_desc* desc, php_ctx* ctx)
             }
             std::vector<int4> ej[3];
             for (const int4& e : ej_all) ej[e.w == 255 ? 2 : e.w == kPlainAtoms ? 1 : 0].push_back(e);
+            if (!ctx->split) plan.inner.clear(); /* found, but too small a share or no memory */
             const std::vector<int4>* jobs[5] = {&plan.inner, &hj, &ej[0], &ej[1], &ej[2]};
             for (int q = 0; q < 5; q++) {
                 ctx->nlist[q] = (int)jobs[q]->size();
