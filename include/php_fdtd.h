@@ -320,10 +320,12 @@ int php_dft_read(php_ctx* ctx, int32_t id, double* out, int32_t* nsamples);
 /* Device bytes held by the context. */
 int php_memory_bytes(const php_ctx* ctx, uint64_t* bytes);
 /* Device bytes php_create would allocate for this description (before any
- * php_dft_add / php_probe_set) at most: the second E and H buffers of a large
- * domain's interior launch are counted, though php_create goes without them
- * where memory is short; needs no device.  Used for admission
- * against a memory budget. */
+ * php_dft_add / php_probe_set) at most; needs no device.  The second E and H
+ * buffers of a large domain's interior launch are counted where php_create
+ * would take that launch (by the domain's size and plain interior; never with
+ * PHP_FUSED=0, which a caller with a tight budget may set for both calls),
+ * though php_create goes without them where less than half of the device's
+ * memory would stay free.  Used for admission against a memory budget. */
 int php_estimate_bytes(const php_desc* desc, uint64_t* bytes);
 /* Number of kernel launches enqueued by the last php_step call. */
 int php_last_launch_count(const php_ctx* ctx, int32_t* launches);

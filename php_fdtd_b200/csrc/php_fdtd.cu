@@ -639,6 +639,15 @@ static double source_value(const php_source_desc* s, double time)
     }
 }
 
+/* fdtd.c:3375-3393: sources outside the grid or with an unknown component are
+ * skipped (their value still goes to source.txt) */
+static bool source_cell(const php_desc& d, const php_source_desc& S, int (&c)[3], int& comp)
+{
+    c[0] = S.x, c[1] = S.y, c[2] = S.z;
+    comp = S.component == 'x' ? 0 : S.component == 'y' ? 1 : S.component == 'z' ? 2 : -1;
+    return c[0] >= 0 && c[0] < d.nx && c[1] >= 0 && c[1] < d.ny && c[2] >= 0 && c[2] < d.nz && comp >= 0;
+}
+
 /* ------------------------------------------------------------ kernel args */
 
 /* Whether the E sweep samples DFT plane q itself (StepArgs::dft_*): the first
@@ -1502,7 +1511,6 @@ static bool is_iso(const MatD& s)
  * third launch costs what the interior saves. */
 constexpr int64_t kSplitCells = 8 << 20;
 constexpr double kSplitShare = 0.4;
-static bool split_size(const php_desc& d) { return (int64_t)d.nx * d.ny * d.nz >= kSplitCells; }
 
 /* Whether the E sweep in place takes a launch per kind of block, where atom
  * blocks want other registers than the rest: from about 74^3 cells (two-atom
@@ -1523,6 +1531,7 @@ struct BlockPlan {
     std::vector<int> pml_before[3]; /* CPML cells of the axis below each index */
     const int16_t* uni = nullptr;
     bool on = false;
+    bool forced = false;            /* the interior launch whatever the domain's size (PHP_FUSED=2) */
     int atom_id = -1, tns_id = -1;
     std::vector<std::array<int, 3>> src;
     std::vector<char> iso;
@@ -1668,6 +1677,64 @@ struct BlockPlan {
         std::stable_sort(ej.begin(), ej.end(), order);
     }
 };
+
+/* The plan of a whole domain or a slab: what the classes are chosen from. */
+static void plan_classes(const php_desc& d, const std::vector<MatD>& mats, const AxisD* axes, const std::vector<int16_t>& uni,
+                         BlockPlan& plan)
+{
+    const bool strict = d.precision == PHP_PREC_FP64_STRICT;
+    plan.nx = d.nx, plan.ny = d.ny, plan.nz = d.nz;
+    plan.gx = (d.nx + kBlockX - 1) / kBlockX, plan.gy = (d.ny + kBlockY - 1) / kBlockY;
+    plan.set_axes(axes);
+    plan.uni = uni.data();
+    const char* pv = getenv("PHP_PLAIN");
+    const char* tv = getenv("PHP_PLAIN_TENSOR");
+    plan.on = !strict && !(pv && !strcmp(pv, "0"));
+    for (int s = 0; s < d.num_sources; s++) {
+        int c[3], comp;
+        if (source_cell(d, d.sources[s], c, comp)) plan.src.push_back({c[0], c[1], c[2]});
+    }
+    for (const MatD& m : mats) plan.iso.push_back(!strict && is_iso(m));
+    /* the lossy or anisotropic material filling the most tiles */
+    std::vector<size_t> count(mats.size(), 0);
+    if (plan.on && !(tv && !strcmp(tv, "0")))
+        for (int16_t id : uni)
+            if (id >= 0 && mats[id].e_only && !plan.iso[id]) count[id]++;
+    for (size_t id = 0; id < count.size(); id++)
+        if (count[id] && (plan.tns_id < 0 || count[id] > count[plan.tns_id])) plan.tns_id = (int)id;
+}
+
+/* PHP_FUSED at create: the interior launch at any size ("2"), the one-launch
+ * step ("1"), neither (another value); unset: by size and share */
+static bool interior_wanted(const php_desc& d)
+{
+    const char* fv = getenv("PHP_FUSED");
+    return d.precision != PHP_PREC_FP64_STRICT && (fv ? !strcmp(fv, "2") : (int64_t)d.nx * d.ny * d.nz >= kSplitCells);
+}
+
+/* Finds the interior of a whole domain; whether it is worth its launch. */
+static bool plan_interior(const php_desc& d, BlockPlan& plan, int sms)
+{
+    if (!plan.on || !interior_wanted(d)) return false;
+    plan.forced = getenv("PHP_FUSED") != nullptr;
+    const bool f32 = d.precision == PHP_PREC_FP32;
+    plan.find_interior(kBlockY * (f32 ? FusedGeom<float, true>::ROWS : FusedGeom<double, true>::ROWS),
+                       sms * (f32 ? PHP_INNER_MINB32 : PHP_INNER_MINB64), plan.forced ? 2 : 8);
+    return !plan.inner.empty() && (plan.forced || plan.inner_cells >= kSplitShare * (double)d.nx * d.ny * d.nz);
+}
+
+/* Bytes of one field level (E and H), and whether the second one may be had:
+ * it makes a step faster and no domain possible, so half of the device's
+ * memory has to stay free beside it for the contexts that come after. */
+static uint64_t level_bytes(const php_desc& d)
+{
+    return 6 * (uint64_t)((d.nx + 31) / 32 * 32) * d.ny * (d.nz + 2) * rsize(d.precision);
+}
+static bool second_buffers_fit(const php_desc& d, uint64_t free_b, uint64_t total_b)
+{
+    return 2 * level_bytes(d) + total_b / 2 <= free_b;
+}
+constexpr uint64_t kDeviceBytes = (uint64_t)183359 << 20; /* of a B200: the most that cudaMemGetInfo reports */
 
 static int create_impl(const php_desc* desc, php_ctx* ctx)
 {
@@ -1858,12 +1925,9 @@ static int create_impl(const php_desc* desc, php_ctx* ctx)
     ctx->src.assign(d.sources, d.sources + d.num_sources);
     for (int s = 0; s < d.num_sources; s++) {
         const php_source_desc& S = d.sources[s];
-        /* fdtd.c:3375-3393: sources outside the grid or with an unknown
-         * component are skipped (their value still goes to source.txt) */
-        if (S.x < 0 || S.x >= nx || S.y < 0 || S.y >= ny || S.z < 0 || S.z >= nz) continue;
-        int comp = S.component == 'x' ? 0 : S.component == 'y' ? 1 : S.component == 'z' ? 2 : -1;
-        if (comp < 0) continue;
-        ctx->src_cell[ctx->nsrc_active] = ((int64_t)S.z * ny + S.y) * nxp + S.x;
+        int c[3], comp;
+        if (!source_cell(d, S, c, comp)) continue;
+        ctx->src_cell[ctx->nsrc_active] = ((int64_t)c[2] * ny + c[1]) * nxp + c[0];
         ctx->src_comp[ctx->nsrc_active] = comp;
         ctx->src_active_index.push_back(s);
         ctx->nsrc_active++;
@@ -1892,45 +1956,15 @@ static int create_impl(const php_desc* desc, php_ctx* ctx)
                                       v.begin() + ctx->z_off, v.begin() + ctx->z_off + nz); };
         cut(z.slot); cut(z.kappa); cut(z.b); cut(z.c); cut(z.kh); cut(z.kd); cut(z.ch); cut(z.cd);
     }
-    /* block classes of the fast modes (see plan_split and the plain blocks
-     * below) */
+    /* block classes of the fast modes */
     BlockPlan plan;
-    plan.nx = nx, plan.ny = ny, plan.nz = nz, plan.gx = gx, plan.gy = gy;
-    plan.set_axes(axes);
-    plan.uni = uni.data();
-    {
-        const char* pv = getenv("PHP_PLAIN");
-        const char* tv = getenv("PHP_PLAIN_TENSOR");
-        plan.on = !strict && !(pv && !strcmp(pv, "0"));
-        for (int s = 0; s < ctx->nsrc_active; s++) {
-            const int64_t sc = ctx->src_cell[s];
-            plan.src.push_back({(int)(sc % nxp), (int)((sc % ctx->plane) / nxp), (int)(sc / ctx->plane)});
-        }
-        for (const MatD& m : mats) plan.iso.push_back(!strict && is_iso(m));
-        /* the lossy or anisotropic material filling the most tiles */
-        std::vector<size_t> count(mats.size(), 0);
-        if (plan.on && !(tv && !strcmp(tv, "0")))
-            for (int16_t id : uni)
-                if (id >= 0 && mats[id].e_only && !plan.iso[id]) count[id]++;
-        for (size_t id = 0; id < count.size(); id++)
-            if (count[id] && (ctx->tns_id < 0 || count[id] > count[ctx->tns_id])) ctx->tns_id = (int)id;
-        plan.tns_id = ctx->tns_id;
-    }
+    plan_classes(d, mats, axes, uni, plan);
+    ctx->tns_id = plan.tns_id;
     /* the interior in a launch of its own (interior_sweep_tma) */
-    {
-        const char* fv = getenv("PHP_FUSED");
-        const bool whole = !strict && ctx->z_off == 0 && ctx->nz_glob == nz && ctx->allow_split && plan.on;
-        const bool forced = fv && !strcmp(fv, "2");
-        if (whole && (forced || (!fv && split_size(d)))) {
-            const int rows = ctx->prec == PHP_PREC_FP32 ? FusedGeom<float, true>::ROWS : FusedGeom<double, true>::ROWS;
-            plan.find_interior(kBlockY * rows, ctx->num_sms * (ctx->prec == PHP_PREC_FP32 ? PHP_INNER_MINB32 : PHP_INNER_MINB64),
-                               forced ? 2 : 8);
-            size_t free_b = 0, total_b = 0;
-            CK(cudaMemGetInfo(&free_b, &total_b));
-            const uint64_t need = 12 * (uint64_t)ctx->plane * (nz + 2) * rsize(ctx->prec);
-            ctx->split = !plan.inner.empty() &&
-                         (forced || (plan.inner_cells >= kSplitShare * (double)nx * ny * nz && need + total_b / 2 <= free_b));
-        }
+    if (ctx->z_off == 0 && ctx->nz_glob == nz && ctx->allow_split && plan_interior(d, plan, ctx->num_sms)) {
+        size_t free_b = 0, total_b = 0;
+        CK(cudaMemGetInfo(&free_b, &total_b));
+        ctx->split = plan.forced || second_buffers_fit(d, free_b, total_b);
     }
 
     /* 32-bit cell offsets inside the sweeps */
@@ -2169,8 +2203,33 @@ static int create_impl(const php_desc* desc, php_ctx* ctx)
     return PHP_OK;
 }
 
+/* Whether php_create takes the interior launch for a description where memory
+ * allows, as create_impl finds it. */
+static bool interior_expected(const php_desc& d, const std::vector<MatD>& mats)
+{
+    if (!interior_wanted(d)) return false;
+    const int gx = (d.nx + kBlockX - 1) / kBlockX, gy = (d.ny + kBlockY - 1) / kBlockY;
+    std::vector<int16_t> col((size_t)gx * gy * d.nz, -2), uni(col.size()); /* [tile][plane], -2: none seen */
+    for (int i = 0; i < d.nx; i++)
+        for (int j = 0; j < d.ny; j++) {
+            const int32_t* m = d.medium + ((size_t)i * d.ny + j) * d.nz;
+            int16_t* u = &col[((size_t)(j / kBlockY) * gx + i / kBlockX) * d.nz];
+            for (int k = 0; k < d.nz; k++) u[k] = u[k] == -2 || u[k] == m[k] ? (int16_t)m[k] : (int16_t)-1;
+        }
+    for (size_t t = 0; t < (size_t)gx * gy; t++)
+        for (int k = 0; k < d.nz; k++) uni[(size_t)k * gx * gy + t] = col[t * d.nz + k];
+    AxisD axes[3];
+    derive_axis(d, d.nx, d.dx, false, axes[0]);
+    derive_axis(d, d.ny, d.dy, false, axes[1]);
+    derive_axis(d, d.nz, d.dz, true, axes[2]);
+    BlockPlan plan;
+    plan_classes(d, mats, axes, uni, plan);
+    return plan_interior(d, plan, 148) && (plan.forced || second_buffers_fit(d, kDeviceBytes, kDeviceBytes));
+}
+
 /* Device bytes php_create will allocate for a description (the buffers of
- * create_impl, without DFT planes or the probe ring); no device needed. */
+ * create_impl, without DFT planes or the probe ring), and what the interior
+ * launch's second buffers may add; no device needed. */
 static int estimate_bytes(const php_desc& d, uint64_t* out, uint64_t* more)
 {
     if (d.nx < 2 || d.ny < 2 || d.nz < 1 || d.num_materials < 1 || !d.materials || !d.medium || d.pml_thickness < 0 ||
@@ -2181,15 +2240,17 @@ static int estimate_bytes(const php_desc& d, uint64_t* out, uint64_t* more)
     const uint64_t nxp = (uint64_t)(d.nx + 31) / 32 * 32, plane = nxp * d.ny, ncell = plane * d.nz;
     std::vector<int> n3(d.num_materials, 0);
     std::vector<char> slotted(d.num_materials, 0);
-    bool any_ade = false, any_atoms = false;
+    std::vector<MatD> mats(d.num_materials);
+    bool any_ade = false, any_atoms = false, usable = true; /* php_create refuses what is not */
     for (int m = 0; m < d.num_materials; m++) {
         n3[m] = 3 * std::max(0, (int)d.materials[m].natom);
         slotted[m] = d.materials[m].use_ade == 1 || d.materials[m].natom > 0;
-        if (!slotted[m] && !strict) { /* a material that keeps D although it has no ADE and no atoms */
+        if (!strict) {
             php_ctx probe;
-            MatD o;
             probe.d = d;
-            slotted[m] = derive_material(&probe, m, d.materials[m], o) == PHP_OK && o.slotted(false);
+            usable = derive_material(&probe, m, d.materials[m], mats[m]) == PHP_OK && usable;
+            /* a material that keeps D although it has no ADE and no atoms */
+            if (!slotted[m]) slotted[m] = usable && mats[m].slotted(false);
         }
     }
     uint64_t nslot = 0;
@@ -2207,8 +2268,10 @@ static int estimate_bytes(const php_desc& d, uint64_t* out, uint64_t* more)
     }
     const uint64_t L = d.pml_thickness;
     uint64_t b = (strict ? 9 : 6) * plane * (d.nz + 2) * rs;
-    /* second E and H buffers and block lists of the interior launch */
-    *more = !strict && split_size(d) ? 6 * plane * (d.nz + 2) * rs + 48 * ((uint64_t)d.nz * (d.nx / 32 + 1) * (d.ny / 8 + 1) / 2) : 0;
+    const uint64_t tiles = nxp / kBlockX * (((uint64_t)d.ny + kBlockY - 1) / kBlockY);
+    if (!strict) b += 16 * tiles * d.nz; /* class launches: their lists */
+    /* second E and H buffers of the interior launch, its list and the sweeps' */
+    *more = usable && d.num_materials <= 256 && interior_expected(d, mats) ? level_bytes(d) + 32 * tiles * d.nz : 0;
     b += 4 * ((uint64_t)d.nz * d.ny * 2 * L + (uint64_t)d.nz * 2 * L * nxp + 2 * L * d.ny * nxp) * rs;
     const char* fv = getenv("PHP_FUSED");
     if (d.precision != PHP_PREC_FP64_STRICT && fv && !strcmp(fv, "1")) { /* second E, H and H CPML buffers */
