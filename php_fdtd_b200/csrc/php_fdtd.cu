@@ -1734,6 +1734,21 @@ static bool second_buffers_fit(const php_desc& d, uint64_t free_b, uint64_t tota
 {
     return 2 * level_bytes(d) + total_b / 2 <= free_b;
 }
+/* What the device's stream-ordered pool holds and no buffer uses (of contexts
+ * destroyed, where a release threshold keeps it): free for the next context,
+ * though cudaMemGetInfo does not say so. */
+static uint64_t pool_reusable(int device)
+{
+    cudaMemPool_t pool;
+    uint64_t reserved = 0, used = 0;
+    if (cudaDeviceGetMemPool(&pool, device) != cudaSuccess ||
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return reserved > used ? reserved - used : 0;
+}
 constexpr uint64_t kDeviceBytes = (uint64_t)183359 << 20; /* of a B200: the most that cudaMemGetInfo reports */
 
 static int create_impl(const php_desc* desc, php_ctx* ctx)
@@ -1964,6 +1979,7 @@ static int create_impl(const php_desc* desc, php_ctx* ctx)
     if (ctx->z_off == 0 && ctx->nz_glob == nz && ctx->allow_split && plan_interior(d, plan, ctx->num_sms)) {
         size_t free_b = 0, total_b = 0;
         CK(cudaMemGetInfo(&free_b, &total_b));
+        free_b += pool_reusable(d.device);
         ctx->split = plan.forced || second_buffers_fit(d, free_b, total_b);
     }
 
