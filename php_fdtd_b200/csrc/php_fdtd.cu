@@ -114,7 +114,7 @@ struct php_ctx {
     void* f[9] = {};            /* field bases (plane 0) */
     void* psi[12] = {};
     /* one-launch step (he_sweep_tma): the second buffers of E, H (fo[0..2],
-     * fo[6..8]; fo[3..5] = f[3..5]) and of the H CPML state, which the
+     * fo[6..8]) and of the H CPML state, which the
      * launch writes the new level to; swap_levels exchanges them with f and
      * psi after it.  level: how many swaps since php_create, mod 2 */
     bool fused = false;
@@ -2021,16 +2021,6 @@ static int create_impl(const php_desc* desc, php_ctx* ctx)
         ctx->fused = ctx->prec != PHP_PREC_FP64_STRICT && ctx->z_off == 0 && ctx->nz_glob == nz && fv && !strcmp(fv, "1");
         if (ctx->fused) ctx->split = false;
     }
-    if (ctx->split || ctx->fused) {
-        for (int f : {PHP_EX, PHP_HX}) {
-            int rc = alloc_field(&ctx->fo[f]);
-            if (rc) return rc;
-        }
-        for (int q = 0; q < 6 && ctx->fused; q++) {
-            int rc = dalloc(ctx, &ctx->psio[q], psz[q] * rs);
-            if (rc) return rc;
-        }
-    }
     int rc = dalloc(ctx, (void**)&ctx->mat, mat_dev.size());
     if (rc) return rc;
     if ((rc = upload(ctx, ctx->mat, mat_dev.data(), mat_dev.size()))) return rc;
@@ -2070,6 +2060,28 @@ static int create_impl(const php_desc* desc, php_ctx* ctx)
         if ((rc = dalloc(ctx, &ctx->v, (size_t)n3max * ctx->nslot * rs))) return rc;
     }
     if ((rc = setup_ion_pass(ctx, mats, ion_off, d))) return rc;
+    /* the second field level, after everything the domain cannot do without;
+     * the interior launch's is given up where it does not fit after all (the
+     * pools may take more than half of the device, or another context may have
+     * been created meanwhile) */
+    if (ctx->split || ctx->fused) {
+        const size_t held = ctx->allocs.size();
+        for (int f : {PHP_EX, PHP_HX})
+            if (!rc) rc = alloc_field(&ctx->fo[f]);
+        if (!rc && ctx->split && getenv("PHP_TEST_NO_SECOND_LEVEL")) rc = PHP_ERR_OOM; /* failure-path test */
+        for (int q = 0; q < 6 && ctx->fused && !rc; q++) rc = dalloc(ctx, &ctx->psio[q], psz[q] * rs);
+        if (rc == PHP_ERR_OOM && ctx->split) {
+            for (; ctx->allocs.size() > held; ctx->allocs.pop_back()) {
+                cudaFreeAsync(ctx->allocs.back(), ctx->stream);
+                ctx->bytes -= 3 * field_bytes;
+            }
+            for (void*& p : ctx->fo) p = nullptr;
+            ctx->split = false;
+            ctx->err[0] = 0;
+            rc = PHP_OK;
+        }
+        if (rc) return rc;
+    }
     if (ctx->ion_split) { /* the atom material whose blocks read their record from the kernel parameters */
         ctx->atom_id = -1;
         for (int i = 0; i < d.num_materials; i++)

@@ -54,3 +54,19 @@ def test_memory_that_the_pool_keeps_is_free():
         ck(rt.cudaMemPoolSetAttribute(pool, attr, old))
         ck(rt.cudaMemPoolTrimTo(pool, 0))
         ck(rt.cudaStreamDestroy(stream))
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_a_domain_is_created_without_it_where_it_cannot_be_had(precision, monkeypatch):
+    with Simulation(_desc(precision)) as sim:
+        assert _interior_launch(sim)
+        sim.step(20)
+        with_it, vol = sim.memory_bytes, sim.read_volume("Ez")
+    monkeypatch.setenv("PHP_TEST_NO_SECOND_LEVEL", "1")     # its allocation fails, after a part of it
+    with Simulation(_desc(precision)) as sim:
+        assert not _interior_launch(sim)
+        sim.step(20)
+        level = 6 * 224 * 224 * 178 * (4 if precision == "fp32" else 8)
+        assert sim.memory_bytes <= with_it - level
+        assert np.abs(vol).max() > 0
+        np.testing.assert_array_equal(sim.read_volume("Ez"), vol)
