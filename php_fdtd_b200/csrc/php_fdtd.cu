@@ -3161,6 +3161,8 @@ int php_memory_bytes(const php_ctx* ctx, uint64_t* bytes)
     return PHP_OK;
 }
 
+bool php_holds_second_level(const php_ctx* ctx) { return ctx->split; }
+
 int php_estimate_buffers(const php_desc* desc, uint64_t* bytes, uint64_t* more)
 {
     return estimate_bytes(*desc, bytes, more);

@@ -11,6 +11,8 @@ extern "C" {
 __attribute__((visibility("hidden"))) int php_create_buffers(const php_desc* desc, bool split, php_ctx** out);
 /* Device bytes without those buffers, and what they may add. */
 __attribute__((visibility("hidden"))) int php_estimate_buffers(const php_desc* desc, uint64_t* bytes, uint64_t* more);
+/* Whether the context holds them. */
+__attribute__((visibility("hidden"))) bool php_holds_second_level(const php_ctx* ctx);
 }
 
 #endif

@@ -202,6 +202,12 @@ void admission_loop(php_server* s)
         s->building--;
         s->cv_step.notify_one();
         j->info.t_start = now_since(s->t0);
+        if (ok && j->split && !php_holds_second_level(j->ctx)) { /* created without: its bytes are free for other jobs */
+            s->used -= j->more;
+            j->bytes -= j->more;
+            j->info.device_bytes = j->bytes;
+            s->cv_admit.notify_one();
+        }
         if (ok) {
             s->ready.push_back(j);
         } else {

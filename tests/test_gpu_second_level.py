@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 
 from php_fdtd_b200 import Material, Simulation, Source, make_desc
+from php_fdtd_b200.serving import Server, estimate_bytes
 
 pytestmark = pytest.mark.gpu
 
@@ -70,3 +71,27 @@ def test_a_domain_is_created_without_it_where_it_cannot_be_had(precision, monkey
         assert sim.memory_bytes <= with_it - level
         assert np.abs(vol).max() > 0
         np.testing.assert_array_equal(sim.read_volume("Ez"), vol)
+
+
+def test_server_charges_it_to_the_budget_only_where_it_is_held(monkeypatch):
+    """Two such jobs under a budget of one with it and one without: the second
+    runs beside the first only once the first's unused bytes come back."""
+    desc = _desc()
+    full = estimate_bytes(desc)
+    with monkeypatch.context() as m:
+        m.setenv("PHP_FUSED", "0")
+        bare = estimate_bytes(desc)
+
+    def serve():
+        with Server(memory_budget=full + bare - 1) as srv:
+            for _ in range(2):
+                srv.submit(desc, 2000)
+            done = []
+            while len(done) < 2:
+                done += srv.poll(timeout_ms=20000)
+            return [d["device_bytes"] for d in done], srv.stats()
+    got, stats = serve()
+    assert got[0] == full and stats["peak_running"] == 1
+    monkeypatch.setenv("PHP_TEST_NO_SECOND_LEVEL", "1")
+    got, stats = serve()
+    assert got == [bare, bare] and stats["peak_running"] == 2
