@@ -1712,10 +1712,15 @@ static bool interior_wanted(const php_desc& d)
     return d.precision != PHP_PREC_FP64_STRICT && (fv ? !strcmp(fv, "2") : (int64_t)d.nx * d.ny * d.nz >= kSplitCells);
 }
 
+/* A list entry holds the tile's x in 16 bits and its y in 15 (int4::x); longer
+ * domains keep the grid launches, whose z chunks carry no such bound. */
+static bool listable(const BlockPlan& plan) { return plan.gx <= 0xffff && plan.gy <= 0x7fff; }
+
 /* Finds the interior of a whole domain; whether it is worth its launch. */
 static bool plan_interior(const php_desc& d, BlockPlan& plan, int sms)
 {
     if (!plan.on || !interior_wanted(d)) return false;
+    if (!listable(plan)) return false;
     plan.forced = getenv("PHP_FUSED") != nullptr;
     const bool f32 = d.precision == PHP_PREC_FP32;
     plan.find_interior(kBlockY * (f32 ? FusedGeom<float, true>::ROWS : FusedGeom<double, true>::ROWS),
@@ -2154,7 +2159,7 @@ static int create_impl(const php_desc* desc, php_ctx* ctx)
             if ((rc = dalloc(ctx, (void**)&ctx->pcls, pc.size() * sizeof(uint16_t)))) return rc;
             if ((rc = upload(ctx, ctx->pcls, pc.data(), pc.size() * sizeof(uint16_t)))) return rc;
         }
-        ctx->by_class = !ctx->split && !ctx->fused && plan.on && plan.atom_id >= 0 && by_class_size(ctx);
+        ctx->by_class = !ctx->split && !ctx->fused && plan.on && plan.atom_id >= 0 && by_class_size(ctx) && listable(plan);
         if (ctx->split || ctx->by_class) {
             ctx->max_chunk = kListChunk;
             std::vector<int4> hj, ej_all;

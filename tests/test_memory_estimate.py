@@ -63,3 +63,14 @@ def test_estimate_covers_the_context(shape, kw, taken, precision):
         sim.step(2)
         assert (sim.profile_read()["step"]["launches"] > 0) == taken
     assert used <= est <= 1.1 * used + (2 << 20), (used, est)
+
+
+def test_domains_too_long_for_the_block_lists_keep_the_grid_launches(monkeypatch):
+    """A list entry has 15 bits for the tile's y: rows of 262 144 cells and more
+    have tiles beyond them."""
+    for ny, taken in ((262136, True), (262152, False)):
+        desc = _desc((65, ny, 9), "fp32", pml=0)
+        est = estimate_bytes(desc)
+        with monkeypatch.context() as m:
+            m.setenv("PHP_FUSED", "0")
+            assert (est > estimate_bytes(desc)) == taken
