@@ -102,7 +102,8 @@ struct php_ctx {
     void* up_buf[2] = {};
     cudaEvent_t up_ev[2] = {};
     bool up_used[2] = {};
-    int up_next = 0;
+    int up_cur = 0;              /* the buffer being filled, up to up_off */
+    size_t up_off = 0;
     /* last error text: a fixed buffer, so that php_last_error's pointer stays
      * valid while another thread (php_frame_wait) records an error */
     char err[1024] = "";
@@ -288,7 +289,7 @@ static int fail(php_ctx* c, int code, const char* fmt, ...)
  * freed on the context's stream: destroying one context never waits for the
  * work of the others (cudaFree would synchronise the whole device), which
  * the serving loop relies on. */
-static int dalloc(php_ctx* ctx, void** p, size_t bytes)
+static int dalloc(php_ctx* ctx, void** p, size_t bytes, bool clear = true)
 {
     *p = nullptr;
     if (bytes == 0) bytes = 16;
@@ -300,6 +301,7 @@ static int dalloc(php_ctx* ctx, void** p, size_t bytes)
     }
     ctx->allocs.push_back(*p);
     ctx->bytes += bytes;
+    if (!clear) return PHP_OK;
     e = cudaMemsetAsync(*p, 0, bytes, ctx->stream);
     if (e != cudaSuccess) return fail(ctx, PHP_ERR_CUDA, "cudaMemset failed: %s", cudaGetErrorString(e));
     return PHP_OK;
@@ -1219,27 +1221,20 @@ static int upload_tables(php_ctx* ctx, const std::vector<MatD>& mats, const std:
             ctx->pool_mc.assign(p, p + sizeof(MatCoef<R>));
         }
     }
-    int rc = dalloc(ctx, &ctx->mc, mc.size() * sizeof(MatCoef<R>));
+    int rc = dupload(ctx, &ctx->mc, mc.data(), mc.size() * sizeof(MatCoef<R>));
     if (rc) return rc;
-    if ((rc = upload(ctx, ctx->mc, mc.data(), mc.size() * sizeof(MatCoef<R>)))) return rc;
     std::vector<R> ic(ion_coef.size() ? ion_coef.size() : 1);
     for (size_t i = 0; i < ion_coef.size(); i++) ic[i] = (R)ion_coef[i];
-    rc = dalloc(ctx, &ctx->ion_coef, ic.size() * sizeof(R));
-    if (rc) return rc;
-    if ((rc = upload(ctx, ctx->ion_coef, ic.data(), ic.size() * sizeof(R)))) return rc;
+    if ((rc = dupload(ctx, &ctx->ion_coef, ic.data(), ic.size() * sizeof(R)))) return rc;
     for (int ax = 0; ax < 3; ax++) {
         const AxisD& A = axes[ax];
         const std::vector<double>* cols[7] = {&A.kappa, &A.b, &A.c, &A.kh, &A.kd, &A.ch, &A.cd};
         for (int q = 0; q < 7; q++) {
             std::vector<R> h(cols[q]->size());
             for (size_t i = 0; i < h.size(); i++) h[i] = (R)(*cols[q])[i];
-            rc = dalloc(ctx, &ctx->axis_tab[ax][q], h.size() * sizeof(R));
-            if (rc) return rc;
-            if ((rc = upload(ctx, ctx->axis_tab[ax][q], h.data(), h.size() * sizeof(R)))) return rc;
+            if ((rc = dupload(ctx, &ctx->axis_tab[ax][q], h.data(), h.size() * sizeof(R)))) return rc;
         }
     }
-    /* host tables must stay alive until the copies finish */
-    CK(cudaStreamSynchronize(ctx->stream));
     return PHP_OK;
 }
 
@@ -1280,45 +1275,59 @@ static void pinned_put(void* p)
 
 /* Host -> device copy through page-locked staging.  A copy from pageable
  * memory is staged by the driver in small synchronous pieces; while other
- * contexts kept the device busy that took up to seconds per context.  Here
- * chunks of up to kUploadChunk go through two pooled page-locked buffers,
- * one copy in flight while the other buffer fills.  The source may be freed
- * on return. */
+ * contexts kept the device busy that took up to seconds per context.  Here the
+ * pieces are laid one behind the other into two pooled page-locked buffers,
+ * one filled while the other's copies run, and the host waits for the device
+ * only when both are full: in a process of many streams each wait may last as
+ * long as the work that other contexts have queued (16 running jobs, creation
+ * with a wait every second upload and between stages 1.6 s, this way 1.2; 0.03
+ * with CUDA_DEVICE_MAX_CONNECTIONS=32, which gives more streams a hardware
+ * queue of their own).  The source may be freed on return. */
 constexpr size_t kUploadChunk = (size_t)4 << 20;
 static int upload(php_ctx* ctx, void* dst, const void* src, size_t bytes)
 {
-    if (bytes == 0) return PHP_OK;
-    for (int b = 0; b < 2; ++b) {
+    for (size_t off = 0; off < bytes;) {
+        if (ctx->up_off == kUploadChunk) { /* to the other buffer, once its copies have left */
+            CK(cudaEventRecord(ctx->up_ev[ctx->up_cur], ctx->stream));
+            ctx->up_used[ctx->up_cur] = true;
+            ctx->up_cur ^= 1;
+            ctx->up_off = 0;
+            if (ctx->up_used[ctx->up_cur]) CK(cudaEventSynchronize(ctx->up_ev[ctx->up_cur]));
+        }
+        const int b = ctx->up_cur;
         if (!ctx->up_buf[b]) {
             ctx->up_buf[b] = pinned_get(kUploadChunk);
             if (!ctx->up_buf[b]) return fail(ctx, PHP_ERR_OOM, "page-locked host allocation failed");
-            ctx->up_used[b] = false;
         }
         if (!ctx->up_ev[b]) CK(cudaEventCreateWithFlags(&ctx->up_ev[b], cudaEventDisableTiming));
-    }
-    for (size_t off = 0; off < bytes;) {
-        const int b = ctx->up_next & 1;
-        const size_t n = std::min(kUploadChunk, bytes - off);
-        if (ctx->up_used[b]) CK(cudaEventSynchronize(ctx->up_ev[b])); /* its last copy has left */
-        memcpy(ctx->up_buf[b], (const char*)src + off, n);
-        CK(cudaMemcpyAsync((char*)dst + off, ctx->up_buf[b], n, cudaMemcpyHostToDevice, ctx->stream));
-        CK(cudaEventRecord(ctx->up_ev[b], ctx->stream));
-        ctx->up_used[b] = true;
-        ctx->up_next++;
+        const size_t n = std::min(kUploadChunk - ctx->up_off, bytes - off);
+        char* stage = (char*)ctx->up_buf[b] + ctx->up_off;
+        memcpy(stage, (const char*)src + off, n);
+        CK(cudaMemcpyAsync((char*)dst + off, stage, n, cudaMemcpyHostToDevice, ctx->stream));
+        ctx->up_off = std::min(kUploadChunk, (ctx->up_off + n + 255) / 256 * 256);
         off += n;
     }
     return PHP_OK;
 }
 
+/* a buffer and its contents (not cleared first) */
+static int dupload(php_ctx* ctx, void** p, const void* src, size_t bytes)
+{
+    int rc = dalloc(ctx, p, bytes, bytes == 0);
+    return rc ? rc : upload(ctx, *p, src, bytes);
+}
+
 /* returns the staging buffers to the pool once their copies are done */
 static void upload_release(php_ctx* ctx)
 {
+    if (ctx->up_buf[0] && ctx->stream) cudaStreamSynchronize(ctx->stream);
     for (int b = 0; b < 2; ++b) {
-        if (ctx->up_used[b]) cudaEventSynchronize(ctx->up_ev[b]);
         pinned_put(ctx->up_buf[b]);
         ctx->up_buf[b] = nullptr;
         ctx->up_used[b] = false;
     }
+    ctx->up_cur = 0;
+    ctx->up_off = 0;
 }
 
 static void ctx_free(php_ctx* ctx)
@@ -1437,16 +1446,13 @@ static int setup_ion_pass(php_ctx* ctx, const std::vector<MatD>& mats, const std
                 img[off] = hi;
                 img[(size_t)np * np + off] = lo;
             }
-        if ((rc = dalloc(ctx, &ctx->ion_bsplit, img.size() * 2))) return rc;
-        if ((rc = upload(ctx, ctx->ion_bsplit, img.data(), img.size() * 2))) return rc;
-        CK(cudaStreamSynchronize(ctx->stream));
+        if ((rc = dupload(ctx, &ctx->ion_bsplit, img.data(), img.size() * 2))) return rc;
         ctx->ion_tc = true;
     } else {
         std::vector<double> pad((size_t)np * np, 0.0);
         for (int q = 0; q < n3; q++)
             for (int p = 0; p < n3; p++) pad[(size_t)q * np + p] = D[(size_t)q * n3 + p];
-        if ((rc = dalloc(ctx, &ctx->ion_dmm, pad.size() * sizeof(double)))) return rc;
-        if ((rc = upload(ctx, ctx->ion_dmm, pad.data(), pad.size() * sizeof(double)))) return rc;
+        if ((rc = dupload(ctx, &ctx->ion_dmm, pad.data(), pad.size() * sizeof(double)))) return rc;
         /* the same matrix as B fragments of the m8n8k4 FP64 MMA (B[k][n] =
          * DMM[n][k]): lane l of fragment (ks, nt) holds B[4 ks + l % 4][8 nt + l / 4];
          * then the E step, B[t][q] = -QeZM(q, t) (t < 3), and P_ion's B[p][c] =
@@ -1471,9 +1477,7 @@ static int setup_ion_pass(php_ctx* ctx, const std::vector<MatD>& mats, const std
                 const int p = ks * 4 + l % 4, c = l / 4;
                 frag[fp + (size_t)ks * 32 + l] = (c < 3 && p < n3) ? zv[(p / 3) * 9 + c * 3 + p % 3] : 0.0;
             }
-        if ((rc = dalloc(ctx, &ctx->ion_dfrag, frag.size() * sizeof(double)))) return rc;
-        if ((rc = upload(ctx, ctx->ion_dfrag, frag.data(), frag.size() * sizeof(double)))) return rc;
-        CK(cudaStreamSynchronize(ctx->stream));
+        if ((rc = dupload(ctx, &ctx->ion_dfrag, frag.data(), frag.size() * sizeof(double)))) return rc;
     }
     ctx->ion_np = np;
     ctx->ion_split = true;
@@ -2026,35 +2030,24 @@ static int create_impl(const php_desc* desc, php_ctx* ctx)
         ctx->fused = ctx->prec != PHP_PREC_FP64_STRICT && ctx->z_off == 0 && ctx->nz_glob == nz && fv && !strcmp(fv, "1");
         if (ctx->fused) ctx->split = false;
     }
-    int rc = dalloc(ctx, (void**)&ctx->mat, mat_dev.size());
+    int rc = dupload(ctx, (void**)&ctx->mat, mat_dev.data(), mat_dev.size());
     if (rc) return rc;
-    if ((rc = upload(ctx, ctx->mat, mat_dev.data(), mat_dev.size()))) return rc;
     if (ctx->nslot > 0) {
         slot_dev.assign((size_t)ctx->ncell_dev, -1);
         for (int64_t s = 0; s < nreal; s++) slot_dev[slot_cell[s]] = (int32_t)s;
-        rc = dalloc(ctx, (void**)&ctx->slot, slot_dev.size() * sizeof(int32_t));
-        if (rc) return rc;
-        if ((rc = upload(ctx, ctx->slot, slot_dev.data(), slot_dev.size() * sizeof(int32_t)))) return rc;
-        rc = dalloc(ctx, (void**)&ctx->slot_cell, slot_cell.size() * sizeof(int64_t));
-        if (rc) return rc;
-        if ((rc = upload(ctx, ctx->slot_cell, slot_cell.data(), slot_cell.size() * sizeof(int64_t)))) return rc;
-        rc = dalloc(ctx, (void**)&ctx->slot_n3, slot_n3.size() * sizeof(int32_t));
-        if (rc) return rc;
-        if ((rc = upload(ctx, ctx->slot_n3, slot_n3.data(), slot_n3.size() * sizeof(int32_t)))) return rc;
+        if ((rc = dupload(ctx, (void**)&ctx->slot, slot_dev.data(), slot_dev.size() * sizeof(int32_t)))) return rc;
+        if ((rc = dupload(ctx, (void**)&ctx->slot_cell, slot_cell.data(), slot_cell.size() * sizeof(int64_t)))) return rc;
+        if ((rc = dupload(ctx, (void**)&ctx->slot_n3, slot_n3.data(), slot_n3.size() * sizeof(int32_t)))) return rc;
         std::vector<uint8_t> slot_mat(slot_cell.size(), 0);
         for (int64_t s = 0; s < nreal; s++) slot_mat[s] = mat_dev[slot_cell[s]];
-        rc = dalloc(ctx, (void**)&ctx->slot_mat, slot_mat.size());
-        if (rc) return rc;
-        if ((rc = upload(ctx, ctx->slot_mat, slot_mat.data(), slot_mat.size()))) return rc;
-        CK(cudaStreamSynchronize(ctx->stream)); /* the host vectors go out of scope */
+        if ((rc = dupload(ctx, (void**)&ctx->slot_mat, slot_mat.data(), slot_mat.size()))) return rc;
     }
     if (!strict) {
         if (ctx->nslot > 0 && (rc = dalloc(ctx, &ctx->Dp, 3 * (size_t)ctx->nslot * rs))) return rc;
         if (ctx->prec == PHP_PREC_FP32 && ctx->any_atoms && (rc = dalloc(ctx, (void**)&ctx->Dc, (size_t)ctx->nslot * 4))) return rc;
         std::vector<double> dm(9 * mats.size());
         for (size_t i = 0; i < mats.size(); i++) memcpy(&dm[9 * i], mats[i].dm, sizeof(mats[i].dm));
-        if ((rc = dalloc(ctx, (void**)&ctx->dmat, dm.size() * sizeof(double)))) return rc;
-        if ((rc = upload(ctx, ctx->dmat, dm.data(), dm.size() * sizeof(double)))) return rc;
+        if ((rc = dupload(ctx, (void**)&ctx->dmat, dm.data(), dm.size() * sizeof(double)))) return rc;
     }
     if (ctx->any_ade) {
         if ((rc = dalloc(ctx, &ctx->P, 3 * (size_t)ctx->nslot * rs))) return rc;
@@ -2156,8 +2149,7 @@ static int create_impl(const php_desc* desc, php_ctx* ctx)
                         pc[((size_t)k * fy + by) * gx + bx] = (uint16_t)(plan.code(id, inner && zfree) | (ring && zfree ? kHPlain : 0u));
                     }
                 }
-            if ((rc = dalloc(ctx, (void**)&ctx->pcls, pc.size() * sizeof(uint16_t)))) return rc;
-            if ((rc = upload(ctx, ctx->pcls, pc.data(), pc.size() * sizeof(uint16_t)))) return rc;
+            if ((rc = dupload(ctx, (void**)&ctx->pcls, pc.data(), pc.size() * sizeof(uint16_t)))) return rc;
         }
         ctx->by_class = !ctx->split && !ctx->fused && plan.on && plan.atom_id >= 0 && by_class_size(ctx) && listable(plan);
         if (ctx->split || ctx->by_class) {
@@ -2179,8 +2171,7 @@ static int create_impl(const php_desc* desc, php_ctx* ctx)
             for (int q = 0; q < 5; q++) {
                 ctx->nlist[q] = (int)jobs[q]->size();
                 if (jobs[q]->empty()) continue;
-                if ((rc = dalloc(ctx, (void**)&ctx->lists[q], jobs[q]->size() * sizeof(int4)))) return rc;
-                if ((rc = upload(ctx, ctx->lists[q], jobs[q]->data(), jobs[q]->size() * sizeof(int4)))) return rc;
+                if ((rc = dupload(ctx, (void**)&ctx->lists[q], jobs[q]->data(), jobs[q]->size() * sizeof(int4)))) return rc;
             }
         }
         for (size_t b = 0; b < pm.size(); b++) {
@@ -2191,12 +2182,10 @@ static int create_impl(const php_desc* desc, php_ctx* ctx)
         }
         ctx->census[7] = (int64_t)pm.size();
         if (nplain) {
-            if ((rc = dalloc(ctx, (void**)&ctx->plain_blk, pm.size()))) return rc;
-            if ((rc = upload(ctx, ctx->plain_blk, pm.data(), pm.size()))) return rc;
+            if ((rc = dupload(ctx, (void**)&ctx->plain_blk, pm.data(), pm.size()))) return rc;
         }
         if (nplain_h) {
-            if ((rc = dalloc(ctx, (void**)&ctx->plain_h, ph.size()))) return rc;
-            if ((rc = upload(ctx, ctx->plain_h, ph.data(), ph.size()))) return rc;
+            if ((rc = dupload(ctx, (void**)&ctx->plain_h, ph.data(), ph.size()))) return rc;
         }
         ctx->khp[0] = d.dt / (d.mu0 * d.dx * 1.0);
         ctx->khp[1] = d.dt / (d.mu0 * d.dy * 1.0);
