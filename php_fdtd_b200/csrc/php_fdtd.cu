@@ -1510,9 +1510,17 @@ static bool is_iso(const MatD& s)
            e[6] == 0.0 && e[7] == 0.0 && e[0] == e[4] && e[0] == e[8];
 }
 
-/* Sizes from which the interior runs in a launch of its own, and the share
- * of the cells it has to hold: below, its blocks do not fill the GPU, or the
- * third launch costs what the interior saves. */
+/* Sizes from which the interior runs in a launch of its own, and the share of
+ * the cells it has to hold.  Gain of a step over the two sweeps, FP64 and FP32,
+ * vacuum / two-atom slab / metal tip over a tensor slab, CPML of 8 cells:
+ *   96^3  0.86 0.88 0.98, 0.79 0.60 0.82     128^3 1.05 0.98 1.22, 0.96 0.91 0.99
+ *   160^3 1.09 1.03 1.18, 1.07 1.09 1.20     192^3 1.11 1.04 1.17, 1.07 1.02 1.14
+ *   256 x 256 x 128 1.14 1.05 1.21, 1.07 1.04 1.16
+ *   256^3 1.15 1.05 1.19, 1.04 1.04 1.11; with a CPML of 56 cells (a quarter of
+ *   the domain inside) 1.11 and 1.06 in vacuum
+ * It pays from some 4 M cells on and down to small interiors.  Both lines are
+ * well inside: a second field level is memory that the domain could be stepped
+ * without, taken where a step gains several per cent by it. */
 constexpr int64_t kSplitCells = 8 << 20;
 constexpr double kSplitShare = 0.4;
 
@@ -1957,17 +1965,23 @@ static int create_impl(const php_desc* desc, php_ctx* ctx)
         ctx->nsrc_active++;
     }
 
-    /* z chunking: short marches while keeping at least ~2 waves of blocks on
-     * 148 SMs.  Measured on 256^3 (the tip workload): FP64 fastest with 4
-     * planes per block (E sweep 0.331 ms, H 0.210 ms; 8 planes 0.339 and
-     * 0.214; 16 planes 0.364 and 0.225), FP32 with 8 (E 0.204 ms; 4 planes
-     * 0.210, 16 planes 0.219); on the 96^3 two-atom slab with 2 (1728 blocks;
-     * FP64 step 56.3 us, 1 plane 61.0, 4 planes 62.5; FP32 36.6, 39.1, 39.7),
-     * on 101 x 67 x 53 with 1 (1908 blocks; strict step 51 us, 2 planes 56) */
+    /* z chunking: long marches while they leave at least 2 waves of 4 blocks on
+     * 148 SMs, in the strict mode 4 (its marches are bound by the divisions of
+     * a cell, so a longer one saves nothing), and for 8 planes 4.  Step in us
+     * with 1, 2, 4, 8 planes per block:
+     *   vacuum 80^3    FP64 24.4 22.8 25.7 36.3  FP32 19.8 17.9 20.3 25.4  strict 56.5 61.7 77.5 124
+     *   vacuum 128^3   FP64 87.2 73.2 70.6 75.5  FP32 55.8 44.6 41.9 44.7  strict 169 165 177 201
+     *   two-atom 128^3 FP64 113 98.2 95.6 97.8   FP32 76.7 66.4 67.1 75.7  strict 254 253 268 306
+     *   two-atom 160^3 FP64 209 177 167 171      FP32 143 118 115 124      strict 467 453 462 496
+     *   vacuum 192^3   FP64 268 216 195 200      FP32 195 141 124 121      strict 508 472 465 482
+     * (within 3 % of the best of the four on cubes of 80 to 192 of vacuum, a
+     * two-atom slab or a metal tip, 48^3 and 64^3 within 6 %, 101 x 67 x 53
+     * FP32 13 %; with 2 waves throughout the strict mode was up to 10 % off, FP32
+     * at 160^3 8 %; with 4 FP64 and FP32 up to 11 % at 80^3) */
     {
         const int tiles = ((nx + kBlockX - 1) / kBlockX) * ((ny + kBlockY - 1) / kBlockY);
         int zc = std::min(ctx->prec == PHP_PREC_FP32 ? 8 : 4, nz);
-        while (zc > 1 && (int64_t)tiles * ((nz + zc - 1) / zc) < 148 * 4 * 2) zc /= 2;
+        while (zc > 1 && (int64_t)tiles * ((nz + zc - 1) / zc) < 148 * 4 * (strict || zc == 8 ? 4 : 2)) zc /= 2;
         ctx->zchunk = d.z_chunk > 0 ? d.z_chunk : zc;
     }
     AxisD axes[3];
