@@ -940,11 +940,12 @@ static void launch_e_lists(php_ctx* ctx, int s_local, StepArgs<R>& a, const TmaM
         launch_chained(ctx, e_sweep_tma<R, false, NA, kEGeneral>, dim3(ctx->nlist[4]), smem, a, maps, beside);
         beside = true;
     }
-    if (ctx->nlist[3]) {
-        a.list = ctx->lists[3];
-        launch_chained(ctx, e_sweep_tma<R, false, NA, kEAtoms>, dim3(ctx->nlist[3]), smem, a, maps, beside);
-        beside = true;
-    }
+    if constexpr (NA <= 4) /* more atoms in the sweep: no atom blocks */
+        if (ctx->nlist[3]) {
+            a.list = ctx->lists[3];
+            launch_chained(ctx, e_sweep_tma<R, false, NA, kEAtoms>, dim3(ctx->nlist[3]), smem, a, maps, beside);
+            beside = true;
+        }
     if (ctx->nlist[2]) {
         a.list = ctx->lists[2];
         launch_chained(ctx, e_sweep_tma<R, false, 0, kEPlain>, dim3(ctx->nlist[2]), smem, a, maps, beside);
@@ -1085,7 +1086,8 @@ static int prepare_t(php_ctx* ctx)
         if (e == cudaSuccess && (ctx->split || ctx->by_class)) {
             const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
             e = cudaFuncSetAttribute(e_sweep_tma<R, STRICT, 0, kEPlain>, at, (int)TmaGeom<R>::E_SMEM);
-            if (e == cudaSuccess) e = cudaFuncSetAttribute(e_sweep_tma<R, STRICT, NA, kEAtoms>, at, (int)TmaGeom<R>::E_SMEM);
+            if constexpr (NA <= 4)
+                if (e == cudaSuccess) e = cudaFuncSetAttribute(e_sweep_tma<R, STRICT, NA, kEAtoms>, at, (int)TmaGeom<R>::E_SMEM);
             if (e == cudaSuccess) e = cudaFuncSetAttribute(e_sweep_tma<R, STRICT, NA, kEGeneral>, at, (int)TmaGeom<R>::E_SMEM);
         }
     if constexpr (!STRICT)

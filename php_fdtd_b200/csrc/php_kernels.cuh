@@ -268,12 +268,6 @@ __device__ __forceinline__ float ldg_nh(const float* p)
     asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
     return v;
 }
-__device__ __forceinline__ int32_t ldg_nh(const int32_t* p)
-{
-    int32_t v;
-    asm volatile("ld.global.nc.s32 %0, [%1];" : "=r"(v) : "l"(p));
-    return v;
-}
 
 /* The launches of recorded steps form a chain of programmatic launches: a
  * launch may start once every block of the one before it has passed

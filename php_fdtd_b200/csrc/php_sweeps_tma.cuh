@@ -2,7 +2,7 @@
  * php_sweeps_tma.cuh -- the two sweeps with a TMA plane pipeline (sm_100a).
  *
  * A block owns a 32 x 8 (x, y) tile of a z chunk.  One thread streams whole
- * planes of the tile into a ring of kTmaStages shared-memory stages with
+ * planes of the tile into a ring of shared-memory stages with
  * cp.async.bulk.tensor (tile mode, no multicast: every byte comes from this
  * GPU's own memory), each stage completed on its own mbarrier; all 256
  * threads compute from shared memory.  The bytes in flight are set by the
@@ -31,7 +31,6 @@
 
 namespace phpdev {
 
-constexpr int kTmaStages = 4;
 constexpr uint32_t kWaitLimit = 1u << 24;
 
 /* Ring depths.  A plane's load takes about 1.8 us from its issue to the
