@@ -44,7 +44,14 @@ constexpr int kMaxChunk = 256;      /* steps per recorded graph */
  * 512 steps are enqueued ahead */
 constexpr int kListChunk = 64;
 constexpr int kProfKinds = PHP_PROFILE_KINDS; /* H sweep, E sweep, probe, DFT, ion pass, one-launch step */
-constexpr size_t kDirectSlice = 256 << 10; /* bytes of a slice that its gather writes to host memory itself */
+/* Bytes of a slice that its gather writes to page-locked host memory itself,
+ * and of monitor rows that frame_gather does; more go by a copy.  Frame with a
+ * slice, by copy and direct: 16 KB 34 and 29 us, 64 KB 37 and 34, 256 KB 49
+ * and 46, 512 KB 61 and 55, 1 MB 110 and 108, 4 MB 378 and 415.  Frame with
+ * rows (one block writes them): 1 KB 27 and 26, 16 KB 29 and 28, 64 KB 40 and
+ * 39, 131 KB 45 and 48, 262 KB 50 and 73. */
+constexpr size_t kDirectSlice = 256 << 10;
+constexpr int64_t kDirectRows = 64 << 10;
 constexpr int kProbeCap = 8192;     /* probe rows held on the device */
 constexpr double kEpsInf = 20.0;    /* EPS_INF, fdtd.c:202 */
 /* The FP32 path keeps the lattice state as 2^48 r and 2^48 v: early in a
@@ -665,8 +672,9 @@ static bool dft_folded(const php_ctx* ctx, size_t q)
 
 /* Whether the sweeps record the monitor row themselves (StepArgs::probe_*):
  * the field cell is a plane of the grid (not a halo plane) and a sweep
- * updates the atom cell's r and v (no ion pass apart).  Where the caller set
- * the z chunks, only for field and atom cells of one chunk. */
+ * updates the atom cell's r and v (no ion pass apart).  A caller that sets the
+ * z chunks keeps the launches it had with them: the row is folded where field
+ * and atom cell lie in one chunk. */
 static bool probe_folded(const php_ctx* ctx)
 {
     if (!ctx->probe || !ctx->probe_fold || ctx->ion_split) return false;
@@ -3043,7 +3051,7 @@ int php_frame_begin(php_ctx* ctx, const php_frame_req* req, int32_t* ticket)
     /* many rows (a long interval, a large lattice) by a copy, ahead of the
      * gather that resets their counter */
     const double* rows_dev = req->probe ? ctx->probe_rows : nullptr;
-    const bool copy_rows = rows * row_len * (int64_t)sizeof(double) > 65536;
+    const bool copy_rows = rows * row_len * (int64_t)sizeof(double) > kDirectRows;
     if (req->probe && copy_rows)
         CK(cudaMemcpyAsync(F.rows, rows_dev, (size_t)rows * row_len * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
     double* rows_out = req->probe && !copy_rows ? F.rows : nullptr;

@@ -17,13 +17,13 @@
  *   pools         SoA: P[3][nslot], Po[3][nslot], r[3*natom_max][nslot], v[...]
  *   D             strict mode: field arrays like E and H.  Fast modes: only
  *                 where E is not a fixed linear map of D (ADE and atom
- *                 cells): Dp[3][nslot] beside the other state of those
- *                 cells.  Every other cell keeps E alone and advances it by
- *                 M (D^{n+1} - D^n), M the material's 3 x 3 map from D to E
- *                 (e_only_add): a step then neither reads nor writes D
- *                 there, 6 of the 21 field words per cell of the two sweeps
- *                 (256^3 tip workload: see php_sweeps_tma.cuh).  Read-outs
- *                 of D form M^-1 E (d_at).
+ *                 cells) or the map would lose digits: Dp[3][nslot] beside
+ *                 the other state of those cells.  Every other cell keeps E
+ *                 alone and advances it by M (D^{n+1} - D^n), M the material's
+ *                 3 x 3 map from D to E (e_only_add): the two sweeps move 18
+ *                 field words per cell instead of 21 (E is read in place of
+ *                 D and D not written; 24 where a lossy cell read both).
+ *                 Read-outs of D form M^-1 E (d_at).
  *
  * Arithmetic modes:
  *   Strict (double): every operation of the reference in its order, with
@@ -139,7 +139,7 @@ struct StepArgs {
     const R* ion_coef;
     R *P, *Po, *r, *v;         /* pools */
     R* Dp;                     /* D of the cells with a slot [3][nslot] (fast modes) */
-    uint32_t* Dc;              /* FP32 without ADE: what Dp's sums rounded off (pool_add) [nslot], else null */
+    uint32_t* Dc;              /* FP32 with atoms: what Dp's sums rounded off (pool_add) [nslot], else null */
     DView<R> dv;
     const R* pr;               /* QeZV . r [3][nslot] when the ion pass runs apart (php_ions.cuh), else null */
     int32_t ion_k_off;         /* ion_coef offset of the material copied in ion_k, -1 for none */

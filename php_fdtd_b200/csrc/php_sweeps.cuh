@@ -294,7 +294,8 @@ __device__ __forceinline__ void e_only_add(const R* m, R ux, R uy, R uz, R& ex, 
 /* D of a pool cell: D += u.  FP32 carries what the sum rounds off to the next
  * step: the lattice integrates E = M (D - P) twice, so the slow drift of a
  * plain sum's rounding (a static charge) is the largest error of r and v,
- * several times that of the fields.  w holds the three components' remainders
+ * several times that of the fields.  The remainder is that of an error-free
+ * sum (Knuth's two-sum, The Art of Computer Programming 2, 4.2.2).  w holds the three components' remainders
  * in 10 bits each, in units of 2^-10 ulp of the D they belong to: one word per
  * cell read and written. */
 template <typename R, bool CG = false>

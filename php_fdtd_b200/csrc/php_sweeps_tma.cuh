@@ -510,10 +510,10 @@ __global__ void __launch_bounds__(kBlockX * kBlockY, sizeof(R) == 4 ? PHP_H_MINB
 
 /* ================================================================ E sweep */
 
-/* fdtd.c:3238-3528 fused, with H, the old E (strict mode: D) and the
- * material ids streamed through the stage ring.  Bound by HBM: 9 words per
- * cell (read H, E; write E) plus the CPML and pool state; with D kept for
- * every cell it was 12, and 15 in lossy cells. */
+/* fdtd.c:3238-3528 fused, with H and the old E (strict mode: D) streamed
+ * through the stage ring; material ids and pool slots are read a plane ahead.
+ * Bound by HBM: 9 words per cell (read H, E; write E) plus the CPML and pool
+ * state; with D kept for every cell it was 12, and 15 in lossy cells. */
 /* The classes of blocks an instantiation holds: a launch over a list of
  * blocks of one kind gets the registers that kind needs. */
 enum : int { kEAll = 0, kEPlain = 1, kEAtoms = 2, kEGeneral = 3 };
