@@ -924,9 +924,9 @@ def run_serving(args, ws, rank, local):
                 "d2h_bytes_per_step": round(d2h / steps.sum(), 3),
                 "path": "php_batch_submit host descriptions -> php_batch_poll/fetch_dft, whole stream timed"},
         "clocks": clocks.summary(),
-        # per job step: the two sweeps at least (the E sweep of a larger lattice domain is one launch
-        # per kind of block, not counted; the one-launch step with PHP_FUSED=1), which also sample
-        # the running DFT (a launch of its own with PHP_DFT_FOLD=0)
+        # a lower bound: per job step the two sweeps (the one-launch step with PHP_FUSED=1), which also
+        # sample the running DFT (a launch of its own with PHP_DFT_FOLD=0); the server does not say how
+        # many of its jobs take the E sweep as one launch per kind of block
         "gpu_launches": int(steps.sum()) * ((1 if os.environ.get("PHP_FUSED") == "1" else 2) +
                                             (1 if os.environ.get("PHP_DFT_FOLD") == "0" else 0)),
     }

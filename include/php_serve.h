@@ -6,9 +6,10 @@
  * counterpart; a sweep over wavenumbers or tip heights is a shell loop of
  * separate runs.  Here a server (one per GPU) has admission threads that
  *  - admit submitted simulations in arrival order while the sum of their
- *    device footprints (php_estimate_bytes + DFT planes) stays within the
- *    memory budget and the number of running simulations within max_active,
- *    and build their contexts in parallel;
+ *    device footprints (php_estimate_bytes, the second field level of a large
+ *    domain only where the budget has room for it, + DFT planes) stays within
+ *    the memory budget and the number of running simulations within
+ *    max_active, and build their contexts in parallel;
  * and a stepping thread that
  *  - keeps every admitted simulation's fields on the device and keeps up to
  *    two chunks of its time steps (CUDA graphs, php_step) queued on its own
@@ -23,6 +24,11 @@
  * Threading: every call may come from any host thread; the server
  * serialises them internally.  Times are seconds on the server's monotonic
  * clock (php_server_clock).
+ *
+ * A process of many streams shares few hardware queues, and building a context
+ * waits behind what others have queued there: CUDA_DEVICE_MAX_CONNECTIONS=32 in
+ * the environment before the first CUDA call takes the build beside 16 running
+ * simulations from 1.2 s to 0.03 s (p50).  The library does not set it.
  */
 #ifndef PHP_SERVE_H
 #define PHP_SERVE_H

@@ -63,8 +63,9 @@ def test_fp32_d_is_as_accurate_as_h(c, axis, angle):
 @pytest.mark.parametrize("precision,rtol", [("fp64", 1e-12), ("fp32", 1e-5)])   # as between the block paths elsewhere
 @pytest.mark.parametrize("shape", [(41, 33, 29), (97, 65, 64)])                 # one E sweep; a launch per kind of block
 def test_blocks_of_a_material_that_keeps_d(shape, precision, rtol, monkeypatch):
-    """The blocks of that material alone against the general path, with the
-    material lossy, and a metal (ADE) of fewer cells beside it."""
+    """The blocks of that material alone against the general path, in the two
+    sweeps and in the one-launch step, with the material lossy, and a metal (ADE)
+    of fewer cells beside it."""
     nx, ny, nz = shape
     med = np.zeros(shape, np.int32)
     med[:, :, nz // 4:nz // 2] = 1
@@ -74,13 +75,15 @@ def test_blocks_of_a_material_that_keeps_d(shape, precision, rtol, monkeypatch):
     src = [Source(type=1, x=nx // 3, y=ny // 3, z=nz // 2 + 1, component="z", frequency=1.5e15)]
     desc = make_desc(med, mats, src, dx=DL, dy=DL, dz=DL, dt=DT, pml_thickness=4, precision=precision, source_frequency=3e13)
     out = []
-    for plain in ("1", "0"):
+    for plain, fused in (("0", "0"), ("1", "0"), ("1", "1")):
         monkeypatch.setenv("PHP_PLAIN_ATOMS", plain)
+        monkeypatch.setenv("PHP_FUSED", fused)
         with Simulation(desc) as sim:
             pid = sim.dft_add("Dx", nz // 3, [1.5e15])
             sim.step(150)
             out.append([sim.read_volume(c) for c in range(9)] + [sim.dft_read(pid)[0]])
             assert (sim.block_census()["e_atoms"] > 0) == (plain == "1")
-    for q, (x, y) in enumerate(zip(*out)):
+    for q, (y, *others) in enumerate(zip(*out)):
         assert np.abs(y).max() > 0
-        np.testing.assert_allclose(x, y, rtol=0, atol=rtol * np.abs(y).max(), err_msg=f"output {q}")
+        for x in others:
+            np.testing.assert_allclose(x, y, rtol=0, atol=rtol * np.abs(y).max(), err_msg=f"output {q}")
